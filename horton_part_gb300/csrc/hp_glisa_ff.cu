@@ -357,7 +357,7 @@ constexpr int kRingSlots = 6;
 
 // Shared memory of a fused pass for S shells without its staging ring (bytes).
 __host__ __device__ constexpr size_t fuse_fixed_bytes(int S) {
-  return 8 * (size_t)S                     // per active row: x as a float pair
+  return 8 * (size_t)((S + 1) / 2 * 2)      // per active row: x as a float pair (16-byte units)
          + 8 * (size_t)kFuseWarps * kFuseSP  // partial sums
          + 32 * (size_t)kFuseSP              // per point: (v, s)
          + 8 * (size_t)(kFuseMaxShells - kFuseRegRowsTotal)  // gradient sums of the rows past them
@@ -465,7 +465,9 @@ __global__ void __launch_bounds__(kFuseThreads, 2) k_glisa_fused_ff(Batch bt, in
   uint32_t* xt = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(fsm) + xoff);
   float* ring = hess ? reinterpret_cast<float*>(xt + 32 * xrows) : reinterpret_cast<float*>(fsm);
   float2* xa = reinterpret_cast<float2*>(ring + ring_floats);  // x of active row i
-  Dot2* part = reinterpret_cast<Dot2*>(xa + S);
+  // an even number of pairs, so that the float4 array behind the partial sums
+  // starts on a 16-byte boundary for an odd number of shells too
+  Dot2* part = reinterpret_cast<Dot2*>(xa + (S + 1) / 2 * 2);
   float4* pvs = reinterpret_cast<float4*>(part + kFuseWarps * kFuseSP);  // (v hi, v lo, s, -)
   Dot2* ovf = reinterpret_cast<Dot2*>(pvs + 2 * kFuseSP);  // rows i >= kFuseRegRowsTotal
   double* red = reinterpret_cast<double*>(ovf + (kFuseMaxShells - kFuseRegRowsTotal));
