@@ -1,0 +1,112 @@
+// FP64 building blocks of the per-point loops.
+//
+// GB300 issues FP64 at 2 lanes per clock and SM (1/64 of the FP32 rate), so
+// a warp-wide FP64 instruction of any kind (FMA, add, compare, conversion)
+// holds the pipe for 16 clocks and the FP64 kernels cost their instruction
+// count; integer, FP32, shared-memory and HBM work beside it is nearly free
+// (a stored FP64 value costs 1.2 ps of copy bandwidth, one FP64 instruction
+// 1.6 ps). Hence: table lookups for polynomial terms, stored distances and
+// pro-atoms instead of their recomputation, and sums that cross warps in
+// shared memory before they cross lanes.
+#pragma once
+
+#include "hp_internal.cuh"
+
+namespace hp {
+namespace f64 {
+
+// exp(x) by Tang's table-driven method (ACM TOMS 15(2), 1989): x = n ln2/512
+// + f, |f| <= ln2/1024; exp(x) = 2^(n >> 9) T[n & 511] (1 + (e^f - 1)) with
+// T[j] = 2^(j/512) and e^f - 1 by its Taylor polynomial of degree 4
+// (truncation below 2e-18). Nine FP64 instructions; error below 1.1 ulp plus
+// the rounding of x. tab: the table in shared memory (random 8-byte reads,
+// which the FP64 pipe hides). |x| >= 708, infinities and NaN go to exp.
+constexpr int kExpTab = 512;
+
+static __device__ __noinline__ double exp_rare(double x) { return exp(x); }
+
+__device__ __forceinline__ double exp64(double x, const double* tab) {
+  const unsigned hx = (unsigned)__double2hiint(x);
+  if ((hx & 0x7fffffffu) >= 0x40862000u) {  // |x| >= 708
+    if (hx >= 0xc0875000u && hx < 0xfff00000u) return 0.0;  // x <= -746: below the subnormals
+    return exp_rare(x);
+  }
+  const double kL = 0x1.71547652b82fep+9;                            // 512 / ln2
+  const double kC1 = 0x1.62e42fefa39efp-10, kC2 = 0x1.abc9e3b39803fp-65;  // ln2 / 512
+  const double kMagic = 6755399441055744.0;  // 1.5 * 2^52: round to nearest integer
+  const double t = __fma_rn(x, kL, kMagic);
+  const int n = __double2loint(t);
+  const double nd = t - kMagic;
+  double f = __fma_rn(nd, -kC1, x);
+  f = __fma_rn(nd, -kC2, f);
+  const double T = tab[n & (kExpTab - 1)];
+  const double ts = __hiloint2double(__double2hiint(T) + ((n >> 9) << 20), __double2loint(T));
+  double q = __fma_rn(f, 1.0 / 24.0, 1.0 / 6.0);
+  q = __fma_rn(q, f, 0.5);
+  q = __fma_rn(q, f * f, f);
+  return __fma_rn(ts, q, ts);
+}
+
+// Block-local copy of the table; the caller synchronises before its use.
+__device__ __forceinline__ void load_exp64(double* tab, const double* src) {
+  for (int i = threadIdx.x; i < kExpTab; i += blockDim.x) tab[i] = src[i];
+}
+
+// a / d with the reciprocal from the hardware's approximation and one step
+// of the third-order iteration y (1 + e + e^2), e = 1 - d y: five FP64
+// instructions, within 2 ulp. Divisors outside 2^-959 .. 2^960 (and zero,
+// negative, infinite or NaN ones) are divided plainly.
+__device__ __forceinline__ double div64(double a, double d) {
+  if ((unsigned)(__double2hiint(d) - 0x04000000) >= 0x78000000u) return a / d;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = __fma_rn(-d, y, 1.0);
+  y = __fma_rn(y, __fma_rn(e, e, e), y);
+  return a * y;
+}
+
+// Distance from grid point p to atom a, in one fixed sequence of roundings:
+// the stored value (JobDev::rd) and a recomputed one are the same bits.
+__device__ __forceinline__ double dist64(const JobDev& J, int p, int a) {
+  const double dx = J.px[p] - J.ax[a], dy = J.py[p] - J.ay[a], dz = J.pz[p] - J.az[a];
+  return sqrt(__fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx)));
+}
+
+__device__ __forceinline__ double dist_of(const JobDev& J, const double* rd, int p, int a) {
+  return rd ? rd[p] : dist64(J, p, a);
+}
+
+// Amplitude N S^3 / (8 pi) of an MBIS shell.
+__device__ __forceinline__ double mbis_amp(double n, double s) { return n * (s * s * s) * kInv8PiD; }
+
+// Pro-atom of n MBIS shells at distance r from amplitudes and exponents.
+__device__ __forceinline__ double mbis_pro(const double* amp, const double* s, int stride, int n,
+                                           double r, const double* tab) {
+  double y = 0.0;
+  for (int k = 0; k < n; ++k) y = __fma_rn(amp[k * stride], exp64(-s[k * stride] * r, tab), y);
+  return y;
+}
+
+// Block sums of nq <= Q per-thread values: the warps' values of a lane are
+// added first (from shared memory, warp q for quantity q), then the lanes,
+// which takes 12 warp-wide additions a quantity instead of 48. put(q, sum)
+// is called by lane 0 of a warp. red: Q * kThreads doubles.
+template <int Q, typename Put>
+__device__ __forceinline__ void block_sums(const double (&acc)[Q], int nq, double* red, Put put) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if (q < nq) red[q * kThreads + threadIdx.x] = acc[q];
+  __syncthreads();
+  for (int q = warp; q < nq; q += kWarps) {
+    double v = red[q * kThreads + lane];
+#pragma unroll
+    for (int w = 1; w < kWarps; ++w) v += red[q * kThreads + 32 * w + lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) put(q, v);
+  }
+}
+
+}  // namespace f64
+}  // namespace hp

@@ -27,6 +27,7 @@ namespace hp {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxShells = 16;  // per atom
+constexpr int kMbisMaxShell = 7;  // MBIS / NLIS shells per atom: get_nshell() <= 7 (mbis.py:36-46)
 // A point tile is kThreads * ppt consecutive points; ppt is fixed per job
 // (it depends only on that job's npoint, so a job's reductions are the same
 // alone and inside a batch).
@@ -207,6 +208,11 @@ struct JobDev {
   const double* rad_r;    // nrad: radial nodes
   const double* rad_w;    // nrad: radial weights
   double* radrho;         // nrad: spherical average of w_a rho
+  // FP64 kernels (hp_fp64.cuh)
+  const double* etab;     // 2^(j/512), j < 512
+  double* rd;             // MBIS: distances [natom][npoint], or null (recomputed)
+  double* oldpro;         // MBIS: pro-atoms of the last inner iteration [natom][npoint], or null;
+  int* oldok;             // valid where oldok[natom][ntile] is set
   double* hist_propars;   // [maxiter][nparam]
   double* hist_charges;   // [maxiter][natom]
   double* hist_ent;       // [maxiter]
@@ -633,6 +639,13 @@ void launch_change_radial(const HostBatch& hb, cudaStream_t st);
 void launch_gisa_local(const HostBatch& hb, cudaStream_t st);     // spherical averages + radial moments
 void launch_lisa_sc_local(const HostBatch& hb, cudaStream_t st);  // spherical averages + radial sc solve
 void launch_gisa_qp(const HostBatch& hb, cudaStream_t st);        // k_gisa_qp alone
+
+// FP64 MBIS (hp_mbis.cu)
+void launch_rdist64(const HostBatch& hb, cudaStream_t st);  // rd of the batch's jobs
+void launch_promol64(const HostBatch& hb, cudaStream_t st);
+void launch_mbis_inner64(const HostBatch& hb, cudaStream_t st);
+void launch_change64(const HostBatch& hb, cudaStream_t st);
+void launch_final_atweights64(const HostBatch& hb, cudaStream_t st, int use_old);
 
 // float-float MBIS (hp_ff.cu)
 void launch_promol_ff(const HostBatch& hb, cudaStream_t st);

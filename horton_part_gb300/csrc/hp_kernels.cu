@@ -2,7 +2,7 @@
 //
 // One kernel family per hot-path step of horton-part's stockholder loop
 // (file:line are in the reference package src/horton_part):
-//   k_promol          pro-atoms on the molecular grid + promolecule
+//   k_promol          pro-atoms on the molecular grid + promolecule (MBIS: hp_mbis.cu)
 //                     (core/stockholder.py:153-175, 352-367; mbis.py:263-289;
 //                      gisa.py:202-220)
 //   k_atweights       at_weights = clip(pro_a / promol, 0, 1), rho_a = w_a rho,
@@ -10,7 +10,8 @@
 //                     (core/stockholder.py:369-377, 145-151; mbis.py:200-203)
 //   k_change          sum_a int (rho_a0(new) - rho_a0(old))^2
 //                     (core/iterstock.py:32-45)
-//   k_mbis_*          MBIS inner fixed point (mbis.py:81-163)
+//   k_mbis_update     MBIS parameter update (mbis.py:81-163; the passes over
+//                     the grid are in hp_mbis.cu)
 //   k_basis_qvec, k_gisa_qp   GISA quadratic program (gisa.py:348-421)
 //   k_lisa_sc_*       aLISA self-consistent solver (alisa.py:193-291)
 //   k_lisa_newton_*   aLISA (modified) Newton solver (alisa.py:753-938)
@@ -18,7 +19,7 @@
 // Every kernel runs over a batch of jobs (see hp_internal.cuh).
 #include <math.h>
 
-#include "hp_internal.cuh"
+#include "hp_fp64.cuh"
 
 namespace hp {
 
@@ -105,9 +106,7 @@ __device__ __forceinline__ T proatom(const JobDev& J, int a, const double* par, 
   const int s0 = J.shell_off[a], s1 = J.shell_off[a + 1];
   const double* pa = par + J.par_off[a];
   T y = (T)0;
-  if (MODEL == MODEL_MBIS) {
-    for (int k = 0; k < s1 - s0; ++k) y += slater_shell<T>((T)pa[2 * k], (T)pa[2 * k + 1], r);
-  } else if (MODEL == MODEL_NLIS) {
+  if (MODEL == MODEL_NLIS) {
     for (int k = 0; k < s1 - s0; ++k)
       y += (T)nlis_shell(pa[3 * k], pa[3 * k + 1], pa[3 * k + 2], (double)r);
   } else {
@@ -226,6 +225,9 @@ __global__ void k_copy_old(Batch bt) {
   const JobDev& J = decode_local(bt, local);
   if (glisa_idle(J)) return;
   for (int i = threadIdx.x; i < J.nparam; i += blockDim.x) J.propars_old[i] = J.propars[i];
+  if (J.scheme == SCHEME_MBIS && !J.mixed)  // the amplitudes of the step's start (hp_mbis.cu)
+    for (int k = threadIdx.x; k < J.nshell; k += blockDim.x)
+      J.keep[2 * k] = f64::mbis_amp(J.propars[2 * k], J.propars[2 * k + 1]);
   if (J.fuse)  // entropy and negativity partials of the parameters the step starts from
     for (int t = threadIdx.x; t < J.ntile; t += blockDim.x) {
       J.jpart[(size_t)QJ_ENT_PREV * J.ntile + t] = J.jpart[(size_t)QJ_ENTROPY * J.ntile + t];
@@ -324,8 +326,7 @@ __global__ void __launch_bounds__(kThreads) k_change(Batch bt) {
     const int s0 = J.shell_off[at.atom], nsh = J.shell_off[at.atom + 1] - s0;
     const double* pn = J.propars + J.par_off[at.atom];
     const double* po = J.propars_old + J.par_off[at.atom];
-    const double b = MODEL == MODEL_MBIS ? mbis_bound(pn, nsh, r) + mbis_bound(po, nsh, r)
-                                         : basis_bound(J, s0, nsh, pn, po, r);
+    const double b = basis_bound(J, s0, nsh, pn, po, r);
     if (tile_weight(J, at.tile) * b * b < kSkipRel * J.threshold * J.threshold) {
       if (threadIdx.x == 0) {
         apart_ptr(J, at.atom, QA_CHANGE)[at.tile] = 0.0;
@@ -495,82 +496,8 @@ __global__ void k_inner_init(Batch bt) {
 // MBIS inner fixed point (mbis.py:81-163)
 // ---------------------------------------------------------------------------
 
-constexpr int kMbisMaxShell = 7;            // get_nshell() <= 7 (mbis.py:36-46)
-constexpr int kMbisQ = 2 * kMbisMaxShell + 1;
+constexpr int kMbisQ = 2 * kMbisMaxShell + 1;  // moments (2 per shell), inner change
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_mbis_inner(Batch bt) {
-  __shared__ double red[kWarps * kMbisQ];
-  __shared__ double out[kMbisQ];
-  const JobDev* Jp;
-  const AtomTile at = decode_atom_tile(bt, Jp);
-  const JobDev& J = *Jp;
-  if (!J.active[at.atom]) return;
-  const int nsh = J.shell_off[at.atom + 1] - J.shell_off[at.atom];
-  const double* pc = J.cur + J.par_off[at.atom];
-  const double* pp = J.prev + J.par_off[at.atom];
-  const bool first = J.inner_it[at.atom] == 0;
-  if (J.tgeo && J.amax[(size_t)at.atom * J.ntile + at.tile] < (float)J.density_cutoff) {
-    // per-atom cutoff: rho_a below the cutoff on the whole tile (the moments
-    // are exact zeros); skip if the change term is negligible too
-    const double r = tile_rmin(J, at.atom, at.tile);
-    const double b = mbis_bound(pc, nsh, r) + (first ? 0.0 : mbis_bound(pp, nsh, r));
-    if (tile_weight(J, at.tile) * b * b < kSkipRel * J.inner_threshold * J.inner_threshold) {
-      if (threadIdx.x < 2 * nsh) apart_ptr(J, at.atom, QA_INNER + threadIdx.x)[at.tile] = 0.0;
-      if (threadIdx.x == 0) {
-        apart_ptr(J, at.atom, QA_INNER + kMbisQ - 1)[at.tile] = 0.0;
-        count_skipped(J, at.tile, 1.0);
-      }
-      return;
-    }
-  }
-  T cn[kMbisMaxShell], cs[kMbisMaxShell], pn[kMbisMaxShell], ps[kMbisMaxShell];
-#pragma unroll
-  for (int k = 0; k < kMbisMaxShell; ++k) {
-    const bool on = k < nsh;
-    cn[k] = on ? (T)pc[2 * k] : (T)0;
-    cs[k] = on ? (T)pc[2 * k + 1] : (T)0;
-    pn[k] = on ? (T)pp[2 * k] : (T)0;
-    ps[k] = on ? (T)pp[2 * k + 1] : (T)0;
-  }
-  double acc[kMbisQ];
-#pragma unroll
-  for (int q = 0; q < kMbisQ; ++q) acc[q] = 0.0;
-  const double* ra = J.rhoa + (size_t)at.atom * J.npoint;
-  for (int i = 0; i < J.ppt; ++i) {
-    const int p = point_of(J, at.tile, i);
-    if (p >= J.npoint) continue;
-    const T r = Dist<T>::r(J, p, at.atom);
-    T t[kMbisMaxShell];
-    T pro = (T)0, oldpro = (T)0;
-#pragma unroll
-    for (int k = 0; k < kMbisMaxShell; ++k) {
-      t[k] = (T)0;
-      if (k < nsh) {
-        t[k] = slater_shell<T>(cn[k], cs[k], r);
-        pro += t[k];
-        if (!first) oldpro += slater_shell<T>(pn[k], ps[k], r);
-      }
-    }
-    const double rho = ra[p];
-    const double w = J.w[p];
-    const bool sick = (rho < J.density_cutoff) || ((double)pro < J.density_cutoff);
-    const double ratio = sick ? 0.0 : rho / (double)pro;
-#pragma unroll
-    for (int k = 0; k < kMbisMaxShell; ++k) {
-      const double m0 = w * ((double)t[k] * ratio);
-      acc[2 * k] += m0;
-      acc[2 * k + 1] += m0 * (double)r;
-    }
-    const double e = (double)oldpro - (double)pro;
-    acc[kMbisQ - 1] += w * e * e;
-  }
-  block_sum<kMbisQ>(acc, red, out);
-  if (threadIdx.x < 2 * nsh) apart_ptr(J, at.atom, QA_INNER + threadIdx.x)[at.tile] = out[threadIdx.x];
-  if (threadIdx.x == 0) apart_ptr(J, at.atom, QA_INNER + kMbisQ - 1)[at.tile] = out[kMbisQ - 1];
-}
-
-// One warp per atom: N_k <- m0_k, S_k <- 3 m0_k / m1_k, convergence test.
 // NLIS / GMBIS inner iteration (nlis.py:99-195), per (atom, tile): with the
 // unit shells u_k = n S^(3/n) exp(-S r^n) / (4 pi Gamma(3/n)) (prefactors
 // formed once per block) and t_k = N_k u_k: m0_k = int w t_k rho_a / pro,
@@ -677,6 +604,9 @@ __global__ void k_nlis_update(Batch bt) {
   }
 }
 
+// One warp per atom: N_k <- m0_k, S_k <- 3 m0_k / m1_k, convergence test. The
+// moments of FP64 jobs (k_mbis_inner64) are those of the bare exponentials:
+// the amplitudes (keep) enter here, and those of the new parameters go there.
 __global__ void k_mbis_update(Batch bt) {
   int a;
   const JobDev& J = decode_local(bt, a);
@@ -693,8 +623,9 @@ __global__ void k_mbis_update(Batch bt) {
   double* pp = J.prev + J.par_off[a];
   double* pr = J.propars + J.par_off[a];
   double nw[2 * kMbisMaxShell];
+  double* amp = J.keep + J.par_off[a];
   for (int k = 0; k < nsh; ++k) {
-    nw[2 * k] = m[2 * k];
+    nw[2 * k] = J.mixed ? m[2 * k] : amp[2 * k] * m[2 * k];
     nw[2 * k + 1] = 3.0 * m[2 * k] / m[2 * k + 1];
   }
   const bool conv = change < J.inner_threshold || mixed_stalled(J, a, change);
@@ -709,6 +640,8 @@ __global__ void k_mbis_update(Batch bt) {
       pp[q] = pc[q];
       pc[q] = nw[q];
     }
+    if (!J.mixed)
+      for (int k = 0; k < nsh; ++k) amp[2 * k] = f64::mbis_amp(nw[2 * k], nw[2 * k + 1]);
     J.inner_it[a] = it + 1;
     J.atom_out[a * AO_COUNT + AO_INNER_CHANGE] = change;
     if (J.mixed)
@@ -2874,8 +2807,8 @@ void launch_copy_old(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_copy_ol
 void launch_promol(const HostBatch& hb, cudaStream_t st, int mixed, int model) {
   if (mixed == PH_FF && model == MODEL_MBIS) return launch_promol_ff(hb, st);
   if (mixed) return launch_promol_mx(hb, st, model);
-  if (model == MODEL_MBIS) HP_LAUNCH((k_promol<double, MODEL_MBIS>), K_POINT1, kThreads);
-  else if (model == MODEL_NLIS) HP_LAUNCH((k_promol<double, MODEL_NLIS>), K_POINT1, kThreads);
+  if (model == MODEL_MBIS) return launch_promol64(hb, st);
+  if (model == MODEL_NLIS) HP_LAUNCH((k_promol<double, MODEL_NLIS>), K_POINT1, kThreads);
   else HP_LAUNCH((k_promol<double, MODEL_BASIS>), K_POINT1, kThreads);
   HP_LAUNCH(k_atweights, K_ATOM_TILE, kThreads);
 }
@@ -2890,16 +2823,16 @@ void launch_final_atweights(const HostBatch& hb, cudaStream_t st, int mixed, int
                             int use_old) {
   if (mixed == PH_FF && model == MODEL_MBIS) return launch_final_atweights_ff(hb, st, use_old);
   if (mixed) return launch_final_atweights_mx(hb, st, model, use_old);
-  if (model == MODEL_MBIS) HP_LAUNCH((k_final_atweights<double, MODEL_MBIS>), K_ATOM_TILE, kThreads, use_old);
-  else if (model == MODEL_NLIS)
+  if (model == MODEL_MBIS) return launch_final_atweights64(hb, st, use_old);
+  if (model == MODEL_NLIS)
     HP_LAUNCH((k_final_atweights<double, MODEL_NLIS>), K_ATOM_TILE, kThreads, use_old);
   else HP_LAUNCH((k_final_atweights<double, MODEL_BASIS>), K_ATOM_TILE, kThreads, use_old);
 }
 
 void launch_change(const HostBatch& hb, cudaStream_t st, int mixed, int model) {
   if (mixed) return launch_change_mx(hb, st, model);
-  if (model == MODEL_MBIS) HP_LAUNCH((k_change<double, MODEL_MBIS>), K_ATOM_TILE, kThreads);
-  else if (model == MODEL_NLIS) HP_LAUNCH((k_change<double, MODEL_NLIS>), K_ATOM_TILE, kThreads);
+  if (model == MODEL_MBIS) return launch_change64(hb, st);
+  if (model == MODEL_NLIS) HP_LAUNCH((k_change<double, MODEL_NLIS>), K_ATOM_TILE, kThreads);
   else HP_LAUNCH((k_change<double, MODEL_BASIS>), K_ATOM_TILE, kThreads);
 }
 
@@ -2918,7 +2851,7 @@ void launch_count_active(const HostBatch& hb, cudaStream_t st) {
 void launch_mbis_inner(const HostBatch& hb, cudaStream_t st, int mixed) {
   if (mixed == PH_FF) launch_mbis_inner_ff(hb, st);
   else if (mixed) launch_mbis_inner_mx(hb, st);
-  else HP_LAUNCH(k_mbis_inner<double>, K_ATOM_TILE, kThreads);
+  else launch_mbis_inner64(hb, st);
   HP_LAUNCH(k_mbis_update, K_ATOM, 32);
 }
 

@@ -1,0 +1,285 @@
+// MBIS kernels in FP64 (the default precision), mbis.py:81-163 and
+// core/stockholder.py:153-175 of the reference. All are bound by the FP64
+// pipe (2 lanes per clock and SM), so they are written for few FP64
+// instructions per (point, atom) pair: see hp_fp64.cuh. Shells enter as
+// amplitude A = N S^3 / (8 pi) and exponent S; JobDev::keep holds the
+// amplitudes of the parameters a pass evaluates (k_copy_old, the inner
+// update), at the slot of N.
+//
+// Per job, where they take at most half of the remaining budget, the
+// distances of all pairs (rd) and the pro-atoms of the last inner iteration
+// (oldpro, valid on the (atom, tile) pairs flagged in oldok) are kept; jobs
+// without them recompute the same bits.
+#include <math.h>
+
+#include "hp_fp64.cuh"
+
+namespace hp {
+
+namespace {
+
+constexpr int kQ = 2 * kMbisMaxShell + 1;
+
+__device__ __forceinline__ const JobDev& decode_local_mb(const Batch& bt, int& local) {
+  const int j = find_job(bt, blockIdx.x);
+  local = blockIdx.x - bt.prefix[j];
+  return bt.jobs[j];
+}
+
+__device__ __forceinline__ const JobDev& decode_at_mb(const Batch& bt, int& atom, int& tile) {
+  int local;
+  const JobDev& J = decode_local_mb(bt, local);
+  atom = local / J.ntile;
+  tile = local - atom * J.ntile;
+  return J;
+}
+
+__device__ __forceinline__ const double* rd_row(const JobDev& J, int a) {
+  return J.rd ? J.rd + (size_t)a * J.npoint : nullptr;
+}
+
+}  // namespace
+
+// Distances of every (atom, point) pair, once per job initialisation.
+__global__ void __launch_bounds__(kThreads) k_rdist64(Batch bt) {
+  int blk;
+  const JobDev& J = decode_local_mb(bt, blk);
+  if (!J.rd) return;
+  const int p = blk * kThreads + threadIdx.x;
+  if (p >= J.npoint) return;
+  for (int a = 0; a < J.natom; ++a) J.rd[(size_t)a * J.npoint + p] = f64::dist64(J, p, a);
+}
+
+// Pro-atoms and promolecule, one thread per point.
+__global__ void __launch_bounds__(kThreads) k_promol64(Batch bt) {
+  __shared__ double tab[f64::kExpTab];
+  int blk;
+  const JobDev& J = decode_local_mb(bt, blk);
+  f64::load_exp64(tab, J.etab);
+  __syncthreads();
+  const int p = blk * kThreads + threadIdx.x;
+  if (p >= J.npoint) return;
+  double promol = 0.0;
+  for (int a = 0; a < J.natom; ++a) {
+    const int s0 = J.shell_off[a], n = J.shell_off[a + 1] - s0;
+    const double r = f64::dist_of(J, rd_row(J, a), p, a);
+    const double pro = f64::mbis_pro(J.keep + 2 * s0, J.propars + 2 * s0 + 1, 2, n, r, tab);
+    J.rhoa[(size_t)a * J.npoint + p] = pro;
+    promol += pro;
+    promol += 1e-100;
+  }
+  J.promol[p] = promol;
+  J.invpro[p] = 1.0 / promol;
+}
+
+// One (atom, tile) of an inner iteration with NSH shells: the moments
+// sum w e_k rho_a / pro and sum w e_k r rho_a / pro of the bare exponentials
+// e_k (the update multiplies by A_k) and the change sum w (oldpro - pro)^2.
+// Per pair 12 FP64 instructions a shell (9 of the exponential) and 13 more.
+template <int NSH>
+__device__ __forceinline__ void mbis_tile(const JobDev& J, int a, int tile, bool first,
+                                          const double* tab, double* red) {
+  constexpr int NQ = 2 * NSH + 1;
+  const int s0 = J.shell_off[a];
+  double A[NSH], S[NSH], acc[NQ];
+#pragma unroll
+  for (int k = 0; k < NSH; ++k) {
+    A[k] = J.keep[2 * (s0 + k)];
+    S[k] = -J.cur[2 * (s0 + k) + 1];
+  }
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) acc[q] = 0.0;
+  const size_t row = (size_t)a * J.npoint;
+  const double* __restrict__ ra = J.rhoa + row;
+  const double* __restrict__ wv = J.w;
+  const double* rd = rd_row(J, a);
+  double* old = J.oldpro ? J.oldpro + row : nullptr;
+  const bool stored = old && J.oldok[a * J.ntile + tile] != 0;
+  const double cut = J.density_cutoff;
+  const int p0 = tile * J.tile_points + threadIdx.x;
+  const int p1 = min((tile + 1) * J.tile_points, J.npoint);
+  // the next point's values are loaded while the current one is worked on
+  double rn = 0.0, rhon = 0.0, wn = 0.0, on = 0.0;
+  auto load = [&](int p) {
+    if (p < p1) {
+      rhon = ra[p];
+      wn = wv[p];
+      if (rd) rn = rd[p];
+      if (stored && !first) on = old[p];
+    }
+  };
+  load(p0);
+  for (int p = p0; p < p1; p += kThreads) {
+    const double r = rd ? rn : f64::dist64(J, p, a);
+    const double rho = rhon, w = wn, oldv = on;
+    load(p + kThreads);
+    double e[NSH], pro = 0.0;
+#pragma unroll
+    for (int k = 0; k < NSH; ++k) {
+      e[k] = f64::exp64(S[k] * r, tab);
+      pro = __fma_rn(A[k], e[k], pro);
+    }
+    const bool sick = (rho < cut) || (pro < cut);
+    const double wr = sick ? 0.0 : w * f64::div64(rho, pro);
+    const double wrr = wr * r;
+#pragma unroll
+    for (int k = 0; k < NSH; ++k) {
+      acc[2 * k] = __fma_rn(e[k], wr, acc[2 * k]);
+      acc[2 * k + 1] = __fma_rn(e[k], wrr, acc[2 * k + 1]);
+    }
+    if (old) old[p] = pro;
+    if (first) continue;  // no change in the first iteration (the update takes 1e100)
+    double op = oldv;
+    if (!stored) {
+      op = 0.0;
+      for (int k = 0; k < NSH; ++k) {
+        const double n = J.prev[2 * (s0 + k)], s = J.prev[2 * (s0 + k) + 1];
+        op = __fma_rn(f64::mbis_amp(n, s), f64::exp64(-s * r, tab), op);
+      }
+    }
+    const double d = op - pro;
+    acc[NQ - 1] = __fma_rn(w * d, d, acc[NQ - 1]);
+  }
+  double* out = J.apart + ((size_t)a * J.qa + QA_INNER) * J.ntile + tile;
+  const int nt = J.ntile;
+  f64::block_sums<NQ>(acc, NQ, red, [&](int q, double v) {
+    out[(size_t)(q == NQ - 1 ? kQ - 1 : q) * nt] = v;
+  });
+  if (old && threadIdx.x == 0) J.oldok[a * J.ntile + tile] = 1;
+}
+
+// MBIS inner iteration, one block per (atom, tile). Bound by the FP64 pipe:
+// about 30 FP64 instructions a pair at 1.5 shells, against ~150 when the
+// distance, the old pro-atom's exponentials, CUDA's exp and divide and the
+// sums of seven shells were all formed per pair. Two outer iterations of a
+// 22-atom chain of 320k points: 116.7 -> 34.5 ms.
+__global__ void __launch_bounds__(kThreads) k_mbis_inner64(Batch bt) {
+  __shared__ double tab[f64::kExpTab];
+  __shared__ double red[kQ * kThreads];
+  int a, tile;
+  const JobDev& J = decode_at_mb(bt, a, tile);
+  if (!J.active[a]) return;
+  const int s0 = J.shell_off[a], nsh = J.shell_off[a + 1] - s0;
+  const bool first = J.inner_it[a] == 0;
+  if (J.tgeo && J.amax[(size_t)a * J.ntile + tile] < (float)J.density_cutoff) {
+    // per-atom cutoff: rho_a below the cutoff on the whole tile (the moments
+    // are exact zeros); skip if the change term is negligible too
+    const double r = tile_rmin(J, a, tile);
+    const double b = mbis_bound(J.cur + 2 * s0, nsh, r) + (first ? 0.0 : mbis_bound(J.prev + 2 * s0, nsh, r));
+    if (tile_weight(J, tile) * b * b < kSkipRel * J.inner_threshold * J.inner_threshold) {
+      double* out = J.apart + ((size_t)a * J.qa + QA_INNER) * J.ntile + tile;
+      if (threadIdx.x < 2 * nsh) out[(size_t)threadIdx.x * J.ntile] = 0.0;
+      if (threadIdx.x == 0) {
+        out[(size_t)(kQ - 1) * J.ntile] = 0.0;
+        if (J.oldok) J.oldok[a * J.ntile + tile] = 0;
+        count_skipped(J, tile, 1.0);
+      }
+      return;
+    }
+  }
+  f64::load_exp64(tab, J.etab);
+  __syncthreads();
+  switch (nsh) {
+    case 1: mbis_tile<1>(J, a, tile, first, tab, red); break;
+    case 2: mbis_tile<2>(J, a, tile, first, tab, red); break;
+    case 3: mbis_tile<3>(J, a, tile, first, tab, red); break;
+    case 4: mbis_tile<4>(J, a, tile, first, tab, red); break;
+    case 5: mbis_tile<5>(J, a, tile, first, tab, red); break;
+    case 6: mbis_tile<6>(J, a, tile, first, tab, red); break;
+    default: mbis_tile<7>(J, a, tile, first, tab, red); break;
+  }
+}
+
+// Outer change sum w (pro(new) - pro(old))^2 (core/iterstock.py:32-45).
+__global__ void __launch_bounds__(kThreads) k_change64(Batch bt) {
+  __shared__ double tab[f64::kExpTab];
+  __shared__ double red[kThreads];
+  __shared__ double co[4 * kMbisMaxShell];  // per shell: A, S of new and old
+  int a, tile;
+  const JobDev& J = decode_at_mb(bt, a, tile);
+  const int s0 = J.shell_off[a], nsh = J.shell_off[a + 1] - s0;
+  const double* pn = J.propars + 2 * s0;
+  const double* po = J.propars_old + 2 * s0;
+  if (J.tgeo) {  // per-atom cutoff: bound of the pair's change term
+    const double r = tile_rmin(J, a, tile);
+    const double b = mbis_bound(pn, nsh, r) + mbis_bound(po, nsh, r);
+    if (tile_weight(J, tile) * b * b < kSkipRel * J.threshold * J.threshold) {
+      if (threadIdx.x == 0) {
+        J.apart[((size_t)a * J.qa + QA_CHANGE) * J.ntile + tile] = 0.0;
+        count_skipped(J, tile, 2.0);
+      }
+      return;
+    }
+  }
+  f64::load_exp64(tab, J.etab);
+  if (threadIdx.x < 2 * nsh) {
+    const int k = threadIdx.x >> 1;
+    const double* q = (threadIdx.x & 1) ? po : pn;
+    co[4 * k + 2 * (threadIdx.x & 1)] = f64::mbis_amp(q[2 * k], q[2 * k + 1]);
+    co[4 * k + 2 * (threadIdx.x & 1) + 1] = q[2 * k + 1];
+  }
+  __syncthreads();
+  const double* rd = rd_row(J, a);
+  double acc[1] = {0.0};
+  const int p1 = min((tile + 1) * J.tile_points, J.npoint);
+  for (int p = tile * J.tile_points + threadIdx.x; p < p1; p += kThreads) {
+    const double r = f64::dist_of(J, rd, p, a);
+    const double d = f64::mbis_pro(co, co + 1, 4, nsh, r, tab) - f64::mbis_pro(co + 2, co + 3, 4, nsh, r, tab);
+    acc[0] = __fma_rn(J.w[p] * d, d, acc[0]);
+  }
+  f64::block_sums<1>(acc, 1, red, [&](int, double v) {
+    J.apart[((size_t)a * J.qa + QA_CHANGE) * J.ntile + tile] = v;
+  });
+}
+
+// at_weights output: clip(pro_a / promol, 0, 1) into rhoa (use_old: the
+// parameters at the start of the last outer iteration).
+__global__ void __launch_bounds__(kThreads) k_final_atweights64(Batch bt, int use_old) {
+  __shared__ double tab[f64::kExpTab];
+  __shared__ double co[2 * kMbisMaxShell];
+  int a, tile;
+  const JobDev& J = decode_at_mb(bt, a, tile);
+  const int s0 = J.shell_off[a], nsh = J.shell_off[a + 1] - s0;
+  const double* par = (use_old ? J.propars_old : J.propars) + 2 * s0;
+  f64::load_exp64(tab, J.etab);
+  if (threadIdx.x < nsh) {
+    co[2 * threadIdx.x] = f64::mbis_amp(par[2 * threadIdx.x], par[2 * threadIdx.x + 1]);
+    co[2 * threadIdx.x + 1] = par[2 * threadIdx.x + 1];
+  }
+  __syncthreads();
+  const double* rd = rd_row(J, a);
+  const int p1 = min((tile + 1) * J.tile_points, J.npoint);
+  for (int p = tile * J.tile_points + threadIdx.x; p < p1; p += kThreads) {
+    const double pro = f64::mbis_pro(co, co + 1, 2, nsh, f64::dist_of(J, rd, p, a), tab);
+    J.rhoa[(size_t)a * J.npoint + p] = fmin(fmax(pro / J.promol[p], 0.0), 1.0);
+  }
+}
+
+#define HP_LAUNCH_MB(kernel, kind, threads, ...)                                       \
+  do {                                                                                 \
+    if (hb.blocks[kind] > 0) {                                                         \
+      kernel<<<hb.blocks[kind], threads, 0, st>>>(hb.b[kind], ##__VA_ARGS__);          \
+      ++g_launch_count;                                                                \
+    }                                                                                  \
+  } while (0)
+
+void launch_rdist64(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH_MB(k_rdist64, K_POINT1, kThreads); }
+
+void launch_promol64(const HostBatch& hb, cudaStream_t st) {
+  HP_LAUNCH_MB(k_promol64, K_POINT1, kThreads);
+  launch_atweights(hb, st);
+}
+
+void launch_mbis_inner64(const HostBatch& hb, cudaStream_t st) {
+  HP_LAUNCH_MB(k_mbis_inner64, K_ATOM_TILE, kThreads);
+}
+
+void launch_change64(const HostBatch& hb, cudaStream_t st) {
+  HP_LAUNCH_MB(k_change64, K_ATOM_TILE, kThreads);
+}
+
+void launch_final_atweights64(const HostBatch& hb, cudaStream_t st, int use_old) {
+  HP_LAUNCH_MB(k_final_atweights64, K_ATOM_TILE, kThreads, use_old);
+}
+
+}  // namespace hp

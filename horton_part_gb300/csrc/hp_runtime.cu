@@ -52,11 +52,13 @@ struct hp_ctx {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   size_t budget = 0, used = 0;
+  size_t kept = 0;  // part of `used` that jobs give back on demand (hp_job::keep_mem)
   Mailbox* mail_dev = nullptr;
   Mailbox* mail_host = nullptr;
   std::vector<hp_job*> slots;
   JobDev* batch_dev = nullptr;     // JobDev array of the current batch
   JobDev* batch_host = nullptr;    // pinned staging
+  double* exp_tab = nullptr;       // 2^(j/512), j < 512 (JobDev::etab)
   int* prefix_dev = nullptr;       // [K_NKIND][kMaxSlots + 1]
   int* prefix_host = nullptr;      // pinned staging
   // kernel timing (hp_ctx_profile)
@@ -121,12 +123,75 @@ struct hp_job {
   int64_t g_active = -1; // fused gLISA: G values in the tiles' active rows (-1: not read yet)
   double skipped = 0.0;  // point-atom evaluations skipped by the per-atom cutoff
   bool host_driven = false;  // finished by hp_glisa_finish (histories kept by the host)
+  // FP64 MBIS: the stored distances and pro-atoms (JobDev::rd, oldpro,
+  // oldok), given back when another allocation needs the room (make_room)
+  void* keep_mem = nullptr;
+  size_t keep_bytes = 0;
   void* pack_mem = nullptr;  // fused gLISA: packed G (dev.gpack, dev.gtile_off)
   size_t pack_bytes = 0;
   std::vector<double> changes;  // outer changes of this run
 };
 
 namespace {
+
+void drop_kept(hp_job* j) {
+  if (!j->keep_mem) return;
+  job_free(j->ctx, j->keep_mem);  // in stream order, after the kernels that read it
+  j->ctx->used -= j->keep_bytes;
+  j->ctx->kept -= j->keep_bytes;
+  j->bytes -= j->keep_bytes;
+  j->keep_mem = nullptr;
+  j->keep_bytes = 0;
+  j->dev.rd = nullptr;
+  j->dev.oldpro = nullptr;
+  j->dev.oldok = nullptr;
+}
+
+// Whether the budget has room for `bytes`: jobs give back what they only
+// keep to save recomputation (their results do not depend on it) before an
+// allocation is refused.
+bool make_room(hp_ctx* ctx, size_t bytes) {
+  for (size_t k = 0; k < ctx->slots.size() && ctx->used + bytes > ctx->budget; ++k)
+    if (ctx->slots[k]) drop_kept(ctx->slots[k]);
+  return ctx->used + bytes <= ctx->budget;
+}
+
+// The same for device memory itself: one retry after giving everything back.
+cudaError_t job_alloc_retry(hp_ctx* ctx, void** p, size_t bytes) {
+  cudaError_t e = job_alloc(ctx, p, bytes);
+  if (e == cudaSuccess) return e;
+  cudaGetLastError();
+  for (hp_job* j : ctx->slots)
+    if (j) drop_kept(j);
+  return job_alloc(ctx, p, bytes);
+}
+
+// FP64 MBIS: storage for the pair distances and, on the molecular grid, the
+// pro-atoms of the last inner iteration, where it takes at most half of what
+// is left of the budget.
+void alloc_kept(hp_ctx* ctx, hp_job* j) {
+  JobDev& J = j->dev;
+  if (J.scheme != SCHEME_MBIS || J.mixed) return;
+  const size_t pair = align_up(8 * (size_t)J.natom * (size_t)J.npoint);
+  const size_t bytes = J.local ? pair : 2 * pair + align_up(4 * (size_t)J.natom * J.ntile);
+  const size_t room = ctx->budget > ctx->used ? ctx->budget - ctx->used : 0;
+  if (bytes > room / 2) return;
+  void* mem = nullptr;
+  if (job_alloc(ctx, &mem, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  j->keep_mem = mem;
+  j->keep_bytes = bytes;
+  j->bytes += bytes;
+  ctx->used += bytes;
+  ctx->kept += bytes;
+  J.rd = reinterpret_cast<double*>(mem);
+  if (!J.local) {
+    J.oldpro = reinterpret_cast<double*>((char*)mem + pair);
+    J.oldok = reinterpret_cast<int*>((char*)mem + 2 * pair);
+  }
+}
 
 // State of a mixed-precision job after an outer iteration:
 //   MIXED_FLOOR: the outer change has stopped decreasing (the best change of
@@ -382,9 +447,9 @@ int pack_layout(hp_ctx* ctx, const std::vector<hp_job*>& jobs) {
     const std::vector<int> sched = tile_schedule(work, nb);
     const size_t gbytes = 2 * 4 * (size_t)std::max<int64_t>(total, 1);
     const size_t bytes = gbytes + 8 * (size_t)J.ntile + 4 * sched.size();
-    if (ctx->used + bytes > ctx->budget) return fail(HP_ERR_NO_MEMORY, "HBM budget exceeded (packed G)");
+    if (!make_room(ctx, bytes)) return fail(HP_ERR_NO_MEMORY, "HBM budget exceeded (packed G)");
     void* mem = nullptr;
-    if (job_alloc(ctx, &mem, bytes) != cudaSuccess) {
+    if (job_alloc_retry(ctx, &mem, bytes) != cudaSuccess) {
       cudaGetLastError();
       return fail(HP_ERR_NO_MEMORY, "device allocation failed");
     }
@@ -407,12 +472,14 @@ int pack_layout(hp_ctx* ctx, const std::vector<hp_job*>& jobs) {
 
 int job_init(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatch& hb) {
   launch_nelec(hb, ctx->stream);
-  bool any_basis = false, any_basis_ff = false, any_rdist = false;
+  bool any_basis = false, any_basis_ff = false, any_rdist = false, any_rd = false;
   for (hp_job* j : jobs) {
     any_basis |= j->dev.gmat != nullptr;
     any_basis_ff |= j->dev.gmat_lo != nullptr;
     any_rdist |= j->dev.rdist != nullptr;
+    any_rd |= j->dev.rd != nullptr;
   }
+  if (any_rd) launch_rdist64(hb, ctx->stream);
   if (any_rdist) launch_rdist_ff(hb, ctx->stream);
   if (any_basis) launch_glisa_basis(hb, ctx->stream);
   if (any_basis_ff) launch_glisa_basis_ff(hb, ctx->stream);
@@ -964,6 +1031,15 @@ int32_t hp_ctx_create(int32_t device, size_t hbm_budget, void* stream, hp_ctx** 
     hp_ctx_destroy(c);
     return fail(HP_ERR_NO_MEMORY, "context allocation failed");
   }
+  {
+    double tab[512];
+    for (int j = 0; j < 512; ++j) tab[j] = (double)exp2l((long double)j / 512.0L);
+    if (cudaMalloc(&c->exp_tab, sizeof(tab)) != cudaSuccess ||
+        cudaMemcpy(c->exp_tab, tab, sizeof(tab), cudaMemcpyHostToDevice) != cudaSuccess) {
+      hp_ctx_destroy(c);
+      return fail(HP_ERR_NO_MEMORY, "context allocation failed");
+    }
+  }
   cudaMemsetAsync(c->mail_dev, 0, sizeof(Mailbox) * kMaxSlots, c->stream);
   memset(c->mail_host, 0, sizeof(Mailbox) * kMaxSlots);
   *out = c;
@@ -979,6 +1055,7 @@ int32_t hp_ctx_destroy(hp_ctx* c) {
   if (c->mail_dev) cudaFree(c->mail_dev);
   if (c->mail_host) cudaFreeHost(c->mail_host);
   if (c->batch_dev) cudaFree(c->batch_dev);
+  if (c->exp_tab) cudaFree(c->exp_tab);
   if (c->batch_host) cudaFreeHost(c->batch_host);
   if (c->prefix_dev) cudaFree(c->prefix_dev);
   if (c->prefix_host) cudaFreeHost(c->prefix_host);
@@ -1136,7 +1213,8 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   // when the matrix takes at most half of the remaining budget: every pass
   // then reads G instead of recomputing exponentials (gLISA always does).
   const size_t gbytes = 8 * (size_t)S * N;
-  const size_t room = ctx->budget > ctx->used ? ctx->budget - ctx->used : 0;
+  const size_t firm = ctx->used - ctx->kept;
+  const size_t room = ctx->budget > firm ? ctx->budget - firm : 0;
   if (!glisa && !mbis && !nlis && !mixed && gbytes <= room / 2) add(&J.gmat, gbytes);
   if (glisa) {
     if (!gff) add(&J.gmat, 8 * (size_t)S * N);
@@ -1208,10 +1286,10 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   add(&J.charges, 8 * (size_t)A);
   size_t total = 0;
   for (auto& p : parts) total += align_up(p.bytes);
-  if (ctx->used + total > ctx->budget)
+  if (!make_room(ctx, total))
     return fail(HP_ERR_NO_MEMORY, "job needs " + std::to_string(total) + " bytes; HBM budget exceeded");
   void* mem = nullptr;
-  if (job_alloc(ctx, &mem, total) != cudaSuccess) {
+  if (job_alloc_retry(ctx, &mem, total) != cudaSuccess) {
     cudaGetLastError();
     return fail(HP_ERR_NO_MEMORY, "device allocation of " + std::to_string(total) + " bytes failed");
   }
@@ -1221,6 +1299,7 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
     cur += align_up(p.bytes);
   }
   J.mail = ctx->mail_dev + slot;
+  J.etab = ctx->exp_tab;
   J.natom = A; J.npoint = N; J.ntile = ntile; J.nparam = P; J.nshell = S; J.qa = qa;
   J.scheme = d->scheme; J.solver = solver; J.maxiter = maxiter;
   J.mixed = !mixed ? PH_FP64 : d->precision == HP_PRECISION_FF ? PH_FF : PH_FP32;
@@ -1260,13 +1339,14 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   bool ok = true;
   {
     std::vector<std::pair<char*, char*>> skip;
-    auto plane = [&](const float* q) {
-      if (q) skip.push_back({(char*)q, (char*)q + align_up(4 * (size_t)S * N)});
+    auto plane = [&](const void* q, size_t bytes) {
+      if (q) skip.push_back({(char*)q, (char*)q + align_up(bytes)});
     };
     if (J.gmat_lo) {  // the float-float planes exist only together
-      plane(J.gmat32);
-      plane(J.gmat_lo);
+      plane(J.gmat32, 4 * (size_t)S * N);
+      plane(J.gmat_lo, 4 * (size_t)S * N);
     }
+
     std::sort(skip.begin(), skip.end());
     char* at = (char*)mem;
     for (const auto& r : skip) {
@@ -1437,6 +1517,7 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   ctx->slots[slot] = job;
   ctx->slots_hi = std::max(ctx->slots_hi, slot + 1);
   ctx->used += total;
+  alloc_kept(ctx, job);
   *out = job;
   return HP_OK;
 }
@@ -1448,7 +1529,9 @@ int32_t hp_job_destroy(hp_job* job) {
   cudaStreamSynchronize(ctx->stream);
   job_free(ctx, job->mem);  // back to the context's pool, in stream order
   job_free(ctx, job->pack_mem);
+  job_free(ctx, job->keep_mem);
   ctx->used -= job->bytes;
+  ctx->kept -= job->keep_bytes;
   ctx->slots[job->slot] = nullptr;
   delete job;
   return HP_OK;
@@ -1853,7 +1936,7 @@ int32_t hp_density_plan_create(hp_ctx* ctx, const hp_density_desc* d, hp_density
   HP_CK(cudaSetDevice(ctx->device));
   const size_t ndbl = 3 * (size_t)ns + ns + 2 * (size_t)d->nprim + (size_t)d->nmat * nb * nb;
   const size_t bytes = 8 * ndbl + 4 * 5 * (size_t)ns + 8 * 3;
-  if (ctx->used + bytes > ctx->budget) return fail(HP_ERR_NO_MEMORY, "HBM budget exceeded");
+  if (!make_room(ctx, bytes)) return fail(HP_ERR_NO_MEMORY, "HBM budget exceeded");
   hp_density_plan* p = new hp_density_plan();
   p->ctx = ctx;
   if (cudaMalloc(&p->dev, 8 * std::max<size_t>(ndbl, 1)) != cudaSuccess ||
@@ -1929,7 +2012,7 @@ int32_t hp_density_plan_eval(hp_density_plan* p, int64_t npoint, const double* p
       p->scratch = nullptr;
       p->scratch_points = 0;
     }
-    if (ctx->used + 8 * need > ctx->budget) return fail(HP_ERR_NO_MEMORY, "HBM budget exceeded");
+    if (!make_room(ctx, 8 * need)) return fail(HP_ERR_NO_MEMORY, "HBM budget exceeded");
     if (cudaMalloc(&p->scratch, 8 * need) != cudaSuccess) return fail(HP_ERR_NO_MEMORY, "device allocation failed");
     p->scratch_points = need;
     ctx->used += 8 * need;
