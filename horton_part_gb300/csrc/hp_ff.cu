@@ -15,7 +15,7 @@
 #include <math.h>
 
 #include "hp_ff.cuh"
-#include "hp_internal.cuh"
+#include "hp_inner.cuh"
 
 namespace hp {
 
@@ -91,11 +91,14 @@ __device__ __forceinline__ float shell_delta_f(float t_new, const float* c, floa
 }
 
 // Deterministic block sum of Q FF accumulators; out[q] valid for all threads.
+// Only the first n and the last one are summed (the rest belong to shells the
+// atom does not have).
 template <int Q>
-__device__ __forceinline__ void block_sum_f2(f2 (&acc)[Q], float2* red, float2* out) {
+__device__ __forceinline__ void block_sum_f2(f2 (&acc)[Q], float2* red, float2* out, int n = Q) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
+    if (q >= n && q != Q - 1) continue;
     f2 v = acc[q];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -215,6 +218,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_mbis_inner_ff(Batch bt) {
   __shared__ float2 red[kWarps * kFfMbisQ];
   __shared__ float2 out[kFfMbisQ];
   ffa::load_exp_table(tab);
+  inner_begin();
   int a, tile;
   const JobDev& J = decode_at_ff(bt, a, tile);
   if (!J.active[a]) return;
@@ -231,6 +235,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_mbis_inner_ff(Batch bt) {
         put_partial_ff(J, a, QA_INNER + kFfMbisQ - 1, tile, make_float2(0.f, 0.f));
         count_skipped(J, tile, 1.0);
       }
+      if (last_block_of(J, a)) mbis_update(J, a);
       return;
     }
   }
@@ -270,9 +275,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_mbis_inner_ff(Batch bt) {
     }
     acc[kFfMbisQ - 1] = ffa::add(acc[kFfMbisQ - 1], w.hi * delta * delta);
   }
-  block_sum_f2<kFfMbisQ>(acc, red, out);
+  block_sum_f2<kFfMbisQ>(acc, red, out, 2 * n);
   if (threadIdx.x < 2 * n) put_partial_ff(J, a, QA_INNER + threadIdx.x, tile, out[threadIdx.x]);
   if (threadIdx.x == 0) put_partial_ff(J, a, QA_INNER + kFfMbisQ - 1, tile, out[kFfMbisQ - 1]);
+  if (last_block_of(J, a)) mbis_update(J, a);
 }
 
 // at_weights output (FP64 values written over the rho_a buffer; once per job).
@@ -412,7 +418,7 @@ void launch_promol_ff(const HostBatch& hb, cudaStream_t st) {
 
 void launch_mbis_inner_ff(const HostBatch& hb, cudaStream_t st) {
   ensure_exp_table();
-  HP_LAUNCH_FF(k_mbis_inner_ff, K_ATOM_TILE, kThreads);
+  launch_inner_kernel(k_mbis_inner_ff, hb, K_ATOM_TILE, st);
 }
 
 void launch_rdist_ff(const HostBatch& hb, cudaStream_t st) {

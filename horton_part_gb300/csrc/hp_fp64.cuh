@@ -87,6 +87,21 @@ __device__ __forceinline__ double mbis_pro(const double* amp, const double* s, i
   return y;
 }
 
+// The bound sum |N_k| S_k^3 / (8 pi) exp(-S_k r) of an MBIS pro-atom
+// (N_k >= 0) at distance r >= 0, for the new and (po non-null) the old parameters together:
+// one warp, a shell a lane. tab as exp64.
+__device__ __forceinline__ double mbis_bound_warp(const double* pn, const double* po, int nsh,
+                                                  double r, const double* tab) {
+  const int lane = threadIdx.x & 31;
+  const double* q = lane < 16 ? pn : po;
+  const int k = lane & 15;
+  double b = 0.0;
+  if (k < nsh && q) b = mbis_amp(fabs(q[2 * k]), q[2 * k + 1]) * exp64(-q[2 * k + 1] * r, tab);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+  return b;
+}
+
 // Block sums of nq <= Q per-thread values: the warps' values of a lane are
 // added first (from shared memory, warp q for quantity q), then the lanes,
 // which takes 12 warp-wide additions a quantity instead of 48. put(q, sum)

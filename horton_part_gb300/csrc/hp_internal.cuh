@@ -73,7 +73,8 @@ enum MailI {
   MI_DONE = 6,        // gLISA: finished (converged, failed or out of iterations)
   MI_R0T = 7,         // fused gLISA: 1 + the accepted trial whose densities (r0t) are the next
                       // pass's rho0, 0 when that pass forms rho0 = G^T c itself
-  MI_COUNT = 8
+  MI_INNER_MAX = 8,   // most inner iterations of an atom in the current outer iteration
+  MI_COUNT = 10       // (even: the next mailbox stays 8-byte aligned)
 };
 struct Mailbox {
   double d[MD_COUNT];
@@ -155,6 +156,7 @@ struct JobDev {
   double* atom_out;       // [natom][AO_COUNT]
   int* active;            // natom
   int* inner_it;          // natom
+  int* arrive;            // natom: blocks of the atom that have finished the current inner iteration
   int* ls_fail;           // per (atom, tile) line-search failure bitmask
   double* gmat;           // gLISA: basis values [nshell][npoint]
   double* gpart;          // gLISA: gradient partials [nshell][ntile]
@@ -224,6 +226,7 @@ struct JobDev {
   // pass [natom][ntile]; null when the job has no cutoff
   const double* tgeo;
   float* amax;
+  double* rmin;           // [natom][ntile] distance from the atom to the tile's bounding sphere
   Mailbox* mail;
   int natom, npoint, ntile, nparam, nshell, qa;
   int scheme, solver, mixed, maxiter;
@@ -276,7 +279,14 @@ __device__ __forceinline__ float block_max_f(float v, float* red) {
   return m;
 }
 
+// Distance from atom a to tile t's bounding sphere: formed once per job
+// (k_tile_rmin), read by every test of the cutoff; a square root in every
+// thread of a skipped block costs more of the FP64 pipe than it saves.
 __device__ __forceinline__ double tile_rmin(const JobDev& J, int a, int t) {
+  return J.rmin[(size_t)a * J.ntile + t];
+}
+
+__device__ __forceinline__ double tile_rmin_form(const JobDev& J, int a, int t) {
   const double* g = J.tgeo + 5 * (size_t)t;
   const double dx = J.ax[a] - g[0], dy = J.ay[a] - g[1], dz = J.az[a] - g[2];
   return fmax(0.0, sqrt(dx * dx + dy * dy + dz * dz) - g[3]);
@@ -284,17 +294,6 @@ __device__ __forceinline__ double tile_rmin(const JobDev& J, int a, int t) {
 
 __device__ __forceinline__ double tile_weight(const JobDev& J, int t) {
   return J.tgeo[5 * (size_t)t + 4];
-}
-
-// Upper bound of an MBIS pro-atom (pairs (N_k, S_k), N_k >= 0) at distance
-// r >= 0 from its atom: sum |N_k| S_k^3 / (8 pi) exp(-S_k r).
-__device__ __forceinline__ double mbis_bound(const double* par, int nsh, double r) {
-  double b = 0.0;
-  for (int k = 0; k < nsh; ++k) {
-    const double n = fabs(par[2 * k]), x = par[2 * k + 1];
-    b += n * x * x * x * (0.125 / M_PI) * exp(-x * r);
-  }
-  return b;
 }
 
 // Upper bound of sum_k |a_k - b_k| g_k(r) for an atom's basis shells s0 ..
@@ -311,8 +310,10 @@ __device__ __forceinline__ double basis_bound(const JobDev& J, int s0, int nsh, 
   return s;
 }
 
-// The same bound from the FP32 shell coefficient table of the mixed and
-// float-float kernels (fco: per shell 8 floats; A = N S^3 / (8 pi) at column
+// Upper bound of an MBIS pro-atom (pairs (N_k, S_k), N_k >= 0) at distance
+// r >= 0 from its atom, sum |N_k| S_k^3 / (8 pi) exp(-S_k r) (FP64:
+// f64::mbis_bound_warp), from the FP32 shell coefficient table of the mixed
+// and float-float kernels (fco: per shell 8 floats; A = N S^3 / (8 pi) at column
 // ca, S at column ca + 1).
 __device__ __forceinline__ float mbis_bound_f(const float* co, int nsh, int ca, float r) {
   float b = 0.0f;
@@ -539,6 +540,7 @@ struct HostBatch {
 };
 
 void launch_nelec(const HostBatch& hb, cudaStream_t st);
+void launch_tile_rmin(const HostBatch& hb, cudaStream_t st);
 void launch_copy_old(const HostBatch& hb, cudaStream_t st);
 void launch_promol(const HostBatch& hb, cudaStream_t st, int mixed, int model);
 void launch_final_atweights(const HostBatch& hb, cudaStream_t st, int mixed, int model, int use_old);
@@ -547,6 +549,7 @@ void launch_outer_finish(const HostBatch& hb, cudaStream_t st, int with_charges)
 void launch_charges(const HostBatch& hb, cudaStream_t st);
 void launch_inner_init(const HostBatch& hb, cudaStream_t st);
 void launch_count_active(const HostBatch& hb, cudaStream_t st);
+// one launch per inner iteration, parameter update included (hp_inner.cuh)
 void launch_mbis_inner(const HostBatch& hb, cudaStream_t st, int mixed);
 void launch_nlis_inner(const HostBatch& hb, cudaStream_t st);  // NLIS / GMBIS, FP64
 void launch_nlis_local(const HostBatch& hb, cudaStream_t st);  // spherical averages + radial solve

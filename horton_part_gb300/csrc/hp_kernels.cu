@@ -10,8 +10,7 @@
 //                     (core/stockholder.py:369-377, 145-151; mbis.py:200-203)
 //   k_change          sum_a int (rho_a0(new) - rho_a0(old))^2
 //                     (core/iterstock.py:32-45)
-//   k_mbis_update     MBIS parameter update (mbis.py:81-163; the passes over
-//                     the grid are in hp_mbis.cu)
+//   (MBIS: hp_mbis.cu; the parameter updates of the inner solvers: hp_inner.cuh)
 //   k_basis_qvec, k_gisa_qp   GISA quadratic program (gisa.py:348-421)
 //   k_lisa_sc_*       aLISA self-consistent solver (alisa.py:193-291)
 //   k_lisa_newton_*   aLISA (modified) Newton solver (alisa.py:753-938)
@@ -19,7 +18,7 @@
 // Every kernel runs over a batch of jobs (see hp_internal.cuh).
 #include <math.h>
 
-#include "hp_fp64.cuh"
+#include "hp_inner.cuh"
 
 namespace hp {
 
@@ -201,6 +200,14 @@ __global__ void __launch_bounds__(kThreads) k_nelec(Batch bt) {
   }
   const double s = block_sum1(acc, red);
   if (threadIdx.x == 0) store_partial(J, J.jpart + (size_t)QJ_NELEC * J.ntile + tile, s);
+}
+
+// Once per job initialisation: the cutoff's distances (see tile_rmin).
+__global__ void __launch_bounds__(kThreads) k_tile_rmin(Batch bt) {
+  int a;
+  const JobDev& J = decode_local(bt, a);
+  if (!J.tgeo) return;
+  for (int t = threadIdx.x; t < J.ntile; t += kThreads) J.rmin[(size_t)a * J.ntile + t] = tile_rmin_form(J, a, t);
 }
 
 // Integrated density; basis schemes rescale the initial populations to it
@@ -452,15 +459,8 @@ __global__ void __launch_bounds__(kChargesThreads) k_charges(Batch bt) {
   }
 }
 
-// Mixed precision only: the inner change of FP32-evaluated pro-atoms has a
-// noise floor (about 1e-9 of the pro-atom's L2 norm), so the FP32 inner solve
-// stops at 1000 x the inner threshold; the exact convergence to the
-// threshold happens in the FP64 outer iterations that finish a mixed job.
-__device__ __forceinline__ bool mixed_stalled(const JobDev& J, int a, double change) {
-  (void)a;
-  return J.mixed == PH_FP32 && change < 1e3 * J.inner_threshold;
-}
-
+// Atoms still active, for the solvers whose update kernels do not count them
+// (aLISA Newton and quasi-Newton).
 __global__ void k_count_active(Batch bt) {
   int local;
   const JobDev& J = decode_local(bt, local);
@@ -482,12 +482,14 @@ __global__ void k_inner_init(Batch bt) {
   for (int a = threadIdx.x; a < J.natom; a += blockDim.x) {
     J.active[a] = 1;
     J.inner_it[a] = 0;
+    J.arrive[a] = 0;
     J.atom_out[a * AO_COUNT + AO_INNER_CHANGE] = 1e300;
   }
   if (J.mixed)
     for (int s = threadIdx.x; s < J.nshell; s += blockDim.x) fill_fco(J, s, J.propars, J.propars);
   if (threadIdx.x == 0) {
     J.mail->i[MI_NACTIVE] = J.natom;
+    J.mail->i[MI_INNER_MAX] = 0;
     J.mail->d[MD_INNER_TOTAL] = 0.0;
   }
 }
@@ -503,10 +505,11 @@ constexpr int kMbisQ = 2 * kMbisMaxShell + 1;  // moments (2 per shell), inner c
 // formed once per block) and t_k = N_k u_k: m0_k = int w t_k rho_a / pro,
 // m1_k = int w u_k (rho_a / pro) r^n_k (the reference's m1, without N_k), and
 // int w (oldpro - pro)^2 for the inner change. FP64.
-__global__ void __launch_bounds__(kThreads) k_nlis_inner(Batch bt) {
+__global__ void __launch_bounds__(kThreads, 2) k_nlis_inner(Batch bt) {
   __shared__ double red[kWarps * kMbisQ];
   __shared__ double out[kMbisQ];
   __shared__ double pu[2][kMbisMaxShell];  // unit-shell prefactors of cur, prev
+  inner_begin();
   const JobDev* Jp;
   const AtomTile at = decode_atom_tile(bt, Jp);
   const JobDev& J = *Jp;
@@ -561,92 +564,7 @@ __global__ void __launch_bounds__(kThreads) k_nlis_inner(Batch bt) {
   block_sum<kMbisQ>(acc, red, out);
   if (threadIdx.x < 2 * nsh) apart_ptr(J, at.atom, QA_INNER + threadIdx.x)[at.tile] = out[threadIdx.x];
   if (threadIdx.x == 0) apart_ptr(J, at.atom, QA_INNER + kMbisQ - 1)[at.tile] = out[kMbisQ - 1];
-}
-
-// NLIS update per atom: N_k <- m0_k, S_k <- 3 / (n_k m1_k) (1e-5 where m1_k is
-// within 1e-8 of zero, numpy.isclose), n_k fixed; convergence as MBIS.
-__global__ void k_nlis_update(Batch bt) {
-  int a;
-  const JobDev& J = decode_local(bt, a);
-  if (!J.active[a]) return;
-  const int lane = threadIdx.x & 31;
-  const int nsh = J.shell_off[a + 1] - J.shell_off[a];
-  double m[2 * kMbisMaxShell];
-  for (int q = 0; q < 2 * nsh; ++q) m[q] = warp_tile_sum(J, apart_ptr(J, a, QA_INNER + q), J.ntile);
-  const double chg2 = warp_tile_sum(J, apart_ptr(J, a, QA_INNER + kMbisQ - 1), J.ntile);
-  if (lane != 0) return;
-  const int it = J.inner_it[a];
-  const double change = (it == 0) ? 1e100 : sqrt(chg2);
-  double* pc = J.cur + J.par_off[a];
-  double* pp = J.prev + J.par_off[a];
-  double* pr = J.propars + J.par_off[a];
-  double nw[3 * kMbisMaxShell];
-  for (int k = 0; k < nsh; ++k) {
-    const double n = pc[3 * k + 2], m1 = m[2 * k + 1];
-    nw[3 * k] = m[2 * k];
-    nw[3 * k + 1] = fabs(m1) <= 1e-8 ? 1e-5 : 3.0 / (m1 * n);
-    nw[3 * k + 2] = n;
-  }
-  const bool conv = change < J.inner_threshold;
-  if (conv || it + 1 >= J.inner_maxiter) {
-    for (int q = 0; q < 3 * nsh; ++q) pr[q] = nw[q];
-    J.active[a] = 0;
-    J.atom_out[a * AO_COUNT + AO_INNER_CHANGE] = change;
-    atomicAdd(&J.mail->d[MD_INNER_TOTAL], (double)(it + 1));
-    if (!conv) atomicOr(&J.mail->i[MI_WARN], W_INNER);
-  } else {
-    for (int q = 0; q < 3 * nsh; ++q) {
-      pp[q] = pc[q];
-      pc[q] = nw[q];
-    }
-    J.inner_it[a] = it + 1;
-    J.atom_out[a * AO_COUNT + AO_INNER_CHANGE] = change;
-  }
-}
-
-// One warp per atom: N_k <- m0_k, S_k <- 3 m0_k / m1_k, convergence test. The
-// moments of FP64 jobs (k_mbis_inner64) are those of the bare exponentials:
-// the amplitudes (keep) enter here, and those of the new parameters go there.
-__global__ void k_mbis_update(Batch bt) {
-  int a;
-  const JobDev& J = decode_local(bt, a);
-  if (!J.active[a]) return;
-  const int lane = threadIdx.x & 31;
-  const int nsh = J.shell_off[a + 1] - J.shell_off[a];
-  double m[2 * kMbisMaxShell];
-  for (int q = 0; q < 2 * nsh; ++q) m[q] = warp_tile_sum(J, apart_ptr(J, a, QA_INNER + q), J.ntile);
-  const double chg2 = warp_tile_sum(J, apart_ptr(J, a, QA_INNER + kMbisQ - 1), J.ntile);
-  if (lane != 0) return;
-  const int it = J.inner_it[a];
-  const double change = (it == 0) ? 1e100 : sqrt(chg2);
-  double* pc = J.cur + J.par_off[a];
-  double* pp = J.prev + J.par_off[a];
-  double* pr = J.propars + J.par_off[a];
-  double nw[2 * kMbisMaxShell];
-  double* amp = J.keep + J.par_off[a];
-  for (int k = 0; k < nsh; ++k) {
-    nw[2 * k] = J.mixed ? m[2 * k] : amp[2 * k] * m[2 * k];
-    nw[2 * k + 1] = 3.0 * m[2 * k] / m[2 * k + 1];
-  }
-  const bool conv = change < J.inner_threshold || mixed_stalled(J, a, change);
-  if (conv || it + 1 >= J.inner_maxiter) {
-    for (int q = 0; q < 2 * nsh; ++q) pr[q] = nw[q];
-    J.active[a] = 0;
-    J.atom_out[a * AO_COUNT + AO_INNER_CHANGE] = change;
-    atomicAdd(&J.mail->d[MD_INNER_TOTAL], (double)(it + 1));
-    if (!conv) atomicOr(&J.mail->i[MI_WARN], W_INNER);
-  } else {
-    for (int q = 0; q < 2 * nsh; ++q) {
-      pp[q] = pc[q];
-      pc[q] = nw[q];
-    }
-    if (!J.mixed)
-      for (int k = 0; k < nsh; ++k) amp[2 * k] = f64::mbis_amp(nw[2 * k], nw[2 * k + 1]);
-    J.inner_it[a] = it + 1;
-    J.atom_out[a * AO_COUNT + AO_INNER_CHANGE] = change;
-    if (J.mixed)
-      for (int s = J.shell_off[a]; s < J.shell_off[a + 1]; ++s) fill_fco(J, s, J.cur, J.prev);
-  }
+  if (last_block_of(J, at.atom)) nlis_update(J, at.atom);
 }
 
 // ---------------------------------------------------------------------------
@@ -861,10 +779,11 @@ __global__ void k_gisa_qp(Batch bt) {
 // ---------------------------------------------------------------------------
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_lisa_sc_inner(Batch bt) {
+__global__ void __launch_bounds__(kThreads, 2) k_lisa_sc_inner(Batch bt) {
   constexpr int Q = kMaxShells + 1;
   __shared__ double red[kWarps * Q];
   __shared__ double out[Q];
+  inner_begin();
   const JobDev* Jp;
   const AtomTile at = decode_atom_tile(bt, Jp);
   const JobDev& J = *Jp;
@@ -883,6 +802,7 @@ __global__ void __launch_bounds__(kThreads) k_lisa_sc_inner(Batch bt) {
         apart_ptr(J, at.atom, QA_INNER + Q - 1)[at.tile] = 0.0;
         count_skipped(J, at.tile, 1.0);
       }
+      if (last_block_of(J, at.atom)) lisa_sc_update(J, at.atom);
       return;
     }
   }
@@ -918,47 +838,7 @@ __global__ void __launch_bounds__(kThreads) k_lisa_sc_inner(Batch bt) {
   block_sum<Q>(acc, red, out);
   if (threadIdx.x < nsh) apart_ptr(J, at.atom, QA_INNER + threadIdx.x)[at.tile] = out[threadIdx.x];
   if (threadIdx.x == 0) apart_ptr(J, at.atom, QA_INNER + Q - 1)[at.tile] = out[Q - 1];
-}
-
-__global__ void k_lisa_sc_update(Batch bt) {
-  constexpr int Q = kMaxShells + 1;
-  int a;
-  const JobDev& J = decode_local(bt, a);
-  if (!J.active[a]) return;
-  const int lane = threadIdx.x & 31;
-  const int nsh = J.shell_off[a + 1] - J.shell_off[a];
-  double m[kMaxShells];
-  for (int k = 0; k < nsh; ++k) m[k] = warp_tile_sum(J, apart_ptr(J, a, QA_INNER + k), J.ntile);
-  const double chg2 = warp_tile_sum(J, apart_ptr(J, a, QA_INNER + Q - 1), J.ntile);
-  const double pop = warp_tile_sum(J, apart_ptr(J, a, QA_POP), J.ntile);
-  if (lane != 0) return;
-  const int it = J.inner_it[a];
-  const double change = (it == 0) ? 1e100 : sqrt(chg2);
-  double* pc = J.cur + J.par_off[a];
-  double* pp = J.prev + J.par_off[a];
-  double* pr = J.propars + J.par_off[a];
-  const bool conv = change < J.inner_threshold || mixed_stalled(J, a, change);
-  if (conv || it + 1 >= J.inner_maxiter) {
-    double s = 0.0;
-    for (int k = 0; k < nsh; ++k) {
-      pr[k] = m[k];
-      s += m[k];
-    }
-    J.active[a] = 0;
-    J.atom_out[a * AO_COUNT + AO_INNER_CHANGE] = change;
-    atomicAdd(&J.mail->d[MD_INNER_TOTAL], (double)(it + 1));
-    if (!conv) atomicOr(&J.mail->i[MI_WARN], W_INNER);
-    else if (fabs(s - pop) > J.population_cutoff) atomicOr(&J.mail->i[MI_WARN], W_POPULATION);
-  } else {
-    for (int k = 0; k < nsh; ++k) {
-      pp[k] = pc[k];
-      pc[k] = m[k];
-    }
-    J.inner_it[a] = it + 1;
-    J.atom_out[a * AO_COUNT + AO_INNER_CHANGE] = change;
-    if (J.mixed)
-      for (int s = J.shell_off[a]; s < J.shell_off[a + 1]; ++s) fill_fco(J, s, J.cur, J.prev);
-  }
+  if (last_block_of(J, at.atom)) lisa_sc_update(J, at.atom);
 }
 
 // ---------------------------------------------------------------------------
@@ -2800,6 +2680,8 @@ void launch_nelec(const HostBatch& hb, cudaStream_t st) {
   HP_LAUNCH(k_init_params, K_JOB, 32);
 }
 
+void launch_tile_rmin(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_tile_rmin, K_ATOM, kThreads); }
+
 void launch_copy_old(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_copy_old, K_JOB, 128); }
 
 // FP32 variants live in hp_mixed.cu, float-float (MBIS) in hp_ff.cu; `mixed`
@@ -2852,12 +2734,10 @@ void launch_mbis_inner(const HostBatch& hb, cudaStream_t st, int mixed) {
   if (mixed == PH_FF) launch_mbis_inner_ff(hb, st);
   else if (mixed) launch_mbis_inner_mx(hb, st);
   else launch_mbis_inner64(hb, st);
-  HP_LAUNCH(k_mbis_update, K_ATOM, 32);
 }
 
 void launch_nlis_inner(const HostBatch& hb, cudaStream_t st) {
-  HP_LAUNCH(k_nlis_inner, K_ATOM_TILE, kThreads);
-  HP_LAUNCH(k_nlis_update, K_ATOM, 32);
+  launch_inner_kernel(k_nlis_inner, hb, K_ATOM_TILE, st);
 }
 
 void launch_gisa(const HostBatch& hb, cudaStream_t st, int mixed) {
@@ -2868,8 +2748,7 @@ void launch_gisa(const HostBatch& hb, cudaStream_t st, int mixed) {
 
 void launch_lisa_sc_inner(const HostBatch& hb, cudaStream_t st, int mixed) {
   if (mixed) launch_lisa_sc_inner_mx(hb, st);
-  else HP_LAUNCH(k_lisa_sc_inner<double>, K_ATOM_TILE, kThreads);
-  HP_LAUNCH(k_lisa_sc_update, K_ATOM, 32);
+  else launch_inner_kernel(k_lisa_sc_inner<double>, hb, K_ATOM_TILE, st);
 }
 
 // Newton keeps FP64 evaluation (its Hessian needs it); mixed jobs are

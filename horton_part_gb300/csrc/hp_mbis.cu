@@ -12,7 +12,7 @@
 // without them recompute the same bits.
 #include <math.h>
 
-#include "hp_fp64.cuh"
+#include "hp_inner.cuh"
 
 namespace hp {
 
@@ -120,7 +120,9 @@ __device__ __forceinline__ void mbis_tile(const JobDev& J, int a, int tile, bool
       pro = __fma_rn(A[k], e[k], pro);
     }
     const bool sick = (rho < cut) || (pro < cut);
-    const double wr = sick ? 0.0 : w * f64::div64(rho, pro);
+    // (no quotient where sick: far from the atom pro underflows, and a zero
+    // divisor takes the divide's slow path)
+    const double wr = sick ? 0.0 : w * f64::div64(rho, sick ? 1.0 : pro);
     const double wrr = wr * r;
 #pragma unroll
     for (int k = 0; k < NSH; ++k) {
@@ -156,17 +158,27 @@ __device__ __forceinline__ void mbis_tile(const JobDev& J, int a, int tile, bool
 __global__ void __launch_bounds__(kThreads) k_mbis_inner64(Batch bt) {
   __shared__ double tab[f64::kExpTab];
   __shared__ double red[kQ * kThreads];
+  __shared__ int skip_s;
   int a, tile;
   const JobDev& J = decode_at_mb(bt, a, tile);
+  f64::load_exp64(tab, J.etab);
+  inner_begin();
   if (!J.active[a]) return;
+  __syncthreads();  // the table
   const int s0 = J.shell_off[a], nsh = J.shell_off[a + 1] - s0;
   const bool first = J.inner_it[a] == 0;
   if (J.tgeo && J.amax[(size_t)a * J.ntile + tile] < (float)J.density_cutoff) {
     // per-atom cutoff: rho_a below the cutoff on the whole tile (the moments
-    // are exact zeros); skip if the change term is negligible too
-    const double r = tile_rmin(J, a, tile);
-    const double b = mbis_bound(J.cur + 2 * s0, nsh, r) + (first ? 0.0 : mbis_bound(J.prev + 2 * s0, nsh, r));
-    if (tile_weight(J, tile) * b * b < kSkipRel * J.inner_threshold * J.inner_threshold) {
+    // are exact zeros); skip if the change term is negligible too. One warp
+    // forms the bound: in every thread it costs as much of the FP64 pipe as
+    // the tile itself
+    if (threadIdx.x < 32) {
+      const double b = f64::mbis_bound_warp(J.cur + 2 * s0, first ? nullptr : J.prev + 2 * s0, nsh,
+                                            tile_rmin(J, a, tile), tab);
+      skip_s = tile_weight(J, tile) * b * b < kSkipRel * J.inner_threshold * J.inner_threshold;
+    }
+    __syncthreads();
+    if (skip_s) {
       double* out = J.apart + ((size_t)a * J.qa + QA_INNER) * J.ntile + tile;
       if (threadIdx.x < 2 * nsh) out[(size_t)threadIdx.x * J.ntile] = 0.0;
       if (threadIdx.x == 0) {
@@ -174,11 +186,10 @@ __global__ void __launch_bounds__(kThreads) k_mbis_inner64(Batch bt) {
         if (J.oldok) J.oldok[a * J.ntile + tile] = 0;
         count_skipped(J, tile, 1.0);
       }
+      if (last_block_of(J, a)) mbis_update(J, a);
       return;
     }
   }
-  f64::load_exp64(tab, J.etab);
-  __syncthreads();
   switch (nsh) {
     case 1: mbis_tile<1>(J, a, tile, first, tab, red); break;
     case 2: mbis_tile<2>(J, a, tile, first, tab, red); break;
@@ -188,6 +199,7 @@ __global__ void __launch_bounds__(kThreads) k_mbis_inner64(Batch bt) {
     case 6: mbis_tile<6>(J, a, tile, first, tab, red); break;
     default: mbis_tile<7>(J, a, tile, first, tab, red); break;
   }
+  if (last_block_of(J, a)) mbis_update(J, a);
 }
 
 // Outer change sum w (pro(new) - pro(old))^2 (core/iterstock.py:32-45).
@@ -195,15 +207,21 @@ __global__ void __launch_bounds__(kThreads) k_change64(Batch bt) {
   __shared__ double tab[f64::kExpTab];
   __shared__ double red[kThreads];
   __shared__ double co[4 * kMbisMaxShell];  // per shell: A, S of new and old
+  __shared__ int skip_s;
   int a, tile;
   const JobDev& J = decode_at_mb(bt, a, tile);
   const int s0 = J.shell_off[a], nsh = J.shell_off[a + 1] - s0;
   const double* pn = J.propars + 2 * s0;
   const double* po = J.propars_old + 2 * s0;
+  f64::load_exp64(tab, J.etab);
+  __syncthreads();
   if (J.tgeo) {  // per-atom cutoff: bound of the pair's change term
-    const double r = tile_rmin(J, a, tile);
-    const double b = mbis_bound(pn, nsh, r) + mbis_bound(po, nsh, r);
-    if (tile_weight(J, tile) * b * b < kSkipRel * J.threshold * J.threshold) {
+    if (threadIdx.x < 32) {
+      const double b = f64::mbis_bound_warp(pn, po, nsh, tile_rmin(J, a, tile), tab);
+      skip_s = tile_weight(J, tile) * b * b < kSkipRel * J.threshold * J.threshold;
+    }
+    __syncthreads();
+    if (skip_s) {
       if (threadIdx.x == 0) {
         J.apart[((size_t)a * J.qa + QA_CHANGE) * J.ntile + tile] = 0.0;
         count_skipped(J, tile, 2.0);
@@ -211,7 +229,6 @@ __global__ void __launch_bounds__(kThreads) k_change64(Batch bt) {
       return;
     }
   }
-  f64::load_exp64(tab, J.etab);
   if (threadIdx.x < 2 * nsh) {
     const int k = threadIdx.x >> 1;
     const double* q = (threadIdx.x & 1) ? po : pn;
@@ -271,7 +288,7 @@ void launch_promol64(const HostBatch& hb, cudaStream_t st) {
 }
 
 void launch_mbis_inner64(const HostBatch& hb, cudaStream_t st) {
-  HP_LAUNCH_MB(k_mbis_inner64, K_ATOM_TILE, kThreads);
+  launch_inner_kernel(k_mbis_inner64, hb, K_ATOM_TILE, st);
 }
 
 void launch_change64(const HostBatch& hb, cudaStream_t st) {

@@ -21,7 +21,7 @@
 // Same steps and reference citations as hp_kernels.cu.
 #include <math.h>
 
-#include "hp_internal.cuh"
+#include "hp_inner.cuh"
 
 namespace hp {
 
@@ -48,12 +48,15 @@ __device__ __forceinline__ ff ff_add(ff a, ff b) {
 }
 
 // Block sum of Q float-float accumulators (fixed order); out[q] valid for all
-// threads afterwards.
+// threads afterwards. Only the first n and the last one are summed (the rest
+// belong to shells the atom does not have): with 4 points a thread the sums
+// of all 15 quantities cost more than the points.
 template <int Q>
-__device__ __forceinline__ void block_sum_ff(ff (&acc)[Q], float2* red, float2* out) {
+__device__ __forceinline__ void block_sum_ff(ff (&acc)[Q], float2* red, float2* out, int n = Q) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
+    if (q >= n && q != Q - 1) continue;
     ff v = acc[q];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -250,7 +253,7 @@ __global__ void __launch_bounds__(kThreads) k_change_mx(Batch bt) {
 
 // ---------------------------------------------------------------------------
 // MBIS inner fixed point (mbis.py:81-163); coefficients of (cur, prev) in fco,
-// written by k_inner_init / k_mbis_update
+// written by k_inner_init / mbis_update
 // ---------------------------------------------------------------------------
 
 constexpr int kMxMbisQ = 2 * 7 + 1;
@@ -260,6 +263,7 @@ constexpr int kMxMbisQ = 2 * 7 + 1;
 __global__ void __launch_bounds__(kThreads, 4) k_mbis_inner_mx(Batch bt) {
   __shared__ float2 red[kWarps * kMxMbisQ];
   __shared__ float2 out[kMxMbisQ];
+  inner_begin();
   int a, tile;
   const JobDev& J = decode_at_mx(bt, a, tile);
   if (!J.active[a]) return;
@@ -276,6 +280,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_mbis_inner_mx(Batch bt) {
         put_partial(J, a, QA_INNER + kMxMbisQ - 1, tile, make_float2(0.f, 0.f));
         count_skipped(J, tile, 1.0);
       }
+      if (last_block_of(J, a)) mbis_update(J, a);
       return;
     }
   }
@@ -314,9 +319,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_mbis_inner_mx(Batch bt) {
     }
     acc[kMxMbisQ - 1] = ff_add(acc[kMxMbisQ - 1], w * delta * delta);
   }
-  block_sum_ff<kMxMbisQ>(acc, red, out);
+  block_sum_ff<kMxMbisQ>(acc, red, out, 2 * n);
   if (threadIdx.x < 2 * n) put_partial(J, a, QA_INNER + threadIdx.x, tile, out[threadIdx.x]);
   if (threadIdx.x == 0) put_partial(J, a, QA_INNER + kMxMbisQ - 1, tile, out[kMxMbisQ - 1]);
+  if (last_block_of(J, a)) mbis_update(J, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -342,7 +348,7 @@ __global__ void __launch_bounds__(kThreads) k_basis_qvec_mx(Batch bt) {
     for (int k = 0; k < kMaxShells; ++k)
       if (k < n) acc[k] = ff_add(acc[k], wr * shell_value_f(J, s0 + k, r));
   }
-  block_sum_ff<kMaxShells>(acc, red, out);
+  block_sum_ff<kMaxShells>(acc, red, out, n);
   if (threadIdx.x < n) put_partial(J, a, QA_INNER + threadIdx.x, tile, out[threadIdx.x]);
 }
 
@@ -350,6 +356,7 @@ __global__ void __launch_bounds__(kThreads) k_lisa_sc_inner_mx(Batch bt) {
   constexpr int Q = kMaxShells + 1;
   __shared__ float2 red[kWarps * Q];
   __shared__ float2 out[Q];
+  inner_begin();
   int a, tile;
   const JobDev& J = decode_at_mx(bt, a, tile);
   if (!J.active[a]) return;
@@ -369,6 +376,7 @@ __global__ void __launch_bounds__(kThreads) k_lisa_sc_inner_mx(Batch bt) {
         put_partial(J, a, QA_INNER + Q - 1, tile, make_float2(0.f, 0.f));
         count_skipped(J, tile, 1.0);
       }
+      if (last_block_of(J, a)) lisa_sc_update(J, a);
       return;
     }
   }
@@ -402,9 +410,10 @@ __global__ void __launch_bounds__(kThreads) k_lisa_sc_inner_mx(Batch bt) {
       if (k < n) acc[k] = ff_add(acc[k], wr * (co[8 * k] * g[k]));
     acc[Q - 1] = ff_add(acc[Q - 1], w * delta * delta);
   }
-  block_sum_ff<Q>(acc, red, out);
+  block_sum_ff<Q>(acc, red, out, n);
   if (threadIdx.x < n) put_partial(J, a, QA_INNER + threadIdx.x, tile, out[threadIdx.x]);
   if (threadIdx.x == 0) put_partial(J, a, QA_INNER + Q - 1, tile, out[Q - 1]);
+  if (last_block_of(J, a)) lisa_sc_update(J, a);
 }
 
 // at_weights output (FP64 values written over the float rho_a buffer; runs
@@ -461,7 +470,7 @@ void launch_change_mx(const HostBatch& hb, cudaStream_t st, int model) {
 }
 
 void launch_mbis_inner_mx(const HostBatch& hb, cudaStream_t st) {
-  HP_LAUNCH_MX(k_mbis_inner_mx, K_ATOM_TILE, kThreads);
+  launch_inner_kernel(k_mbis_inner_mx, hb, K_ATOM_TILE, st);
 }
 
 void launch_basis_qvec_mx(const HostBatch& hb, cudaStream_t st) {
@@ -469,7 +478,7 @@ void launch_basis_qvec_mx(const HostBatch& hb, cudaStream_t st) {
 }
 
 void launch_lisa_sc_inner_mx(const HostBatch& hb, cudaStream_t st) {
-  HP_LAUNCH_MX(k_lisa_sc_inner_mx, K_ATOM_TILE, kThreads);
+  launch_inner_kernel(k_lisa_sc_inner_mx, hb, K_ATOM_TILE, st);
 }
 
 void launch_final_atweights_mx(const HostBatch& hb, cudaStream_t st, int model, int use_old) {

@@ -345,17 +345,20 @@ const char* err_text(int err) {
 }
 
 // Inner-solver loop for a batch: launch chunks of inner iterations until no
-// atom of any job is active.
+// atom of any job is active. The first chunk is what the slowest atom took in
+// the last outer iteration (a launch with no active atom costs ~2 us, a host
+// wait ~10); each further one is a quarter of those launched. counted: the
+// update kernels do not keep MI_NACTIVE themselves (aLISA Newton).
 template <typename F>
 int run_inner(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatch& hb, F launch_one,
-              int max_launch) {
+              int max_launch, bool counted = false) {
   launch_inner_init(hb, ctx->stream);
   int chunk = 1;
   for (hp_job* j : jobs) chunk = std::max(chunk, j->last_inner);
   int launched = 0;
   while (true) {
     for (int c = 0; c < chunk && launched < max_launch; ++c, ++launched) launch_one();
-    launch_count_active(hb, ctx->stream);
+    if (counted) launch_count_active(hb, ctx->stream);
     int rc = check_launch();
     if (rc) return rc;
     rc = read_mail(ctx);
@@ -364,9 +367,11 @@ int run_inner(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatch& hb
     for (hp_job* j : jobs) nact += ctx->mail_host[j->slot].i[MI_NACTIVE];
     if (nact == 0) break;
     if (launched >= max_launch) break;
-    chunk = 2;
+    chunk = counted ? 2 : std::max(2, launched / 4);
   }
-  for (hp_job* j : jobs) j->last_inner = std::max(1, std::min(launched, 64));
+  for (hp_job* j : jobs)
+    j->last_inner = counted ? std::max(1, std::min(launched, 64))
+                            : std::max(1, std::min(ctx->mail_host[j->slot].i[MI_INNER_MAX], 512));
   return HP_OK;
 }
 
@@ -473,12 +478,15 @@ int pack_layout(hp_ctx* ctx, const std::vector<hp_job*>& jobs) {
 int job_init(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatch& hb) {
   launch_nelec(hb, ctx->stream);
   bool any_basis = false, any_basis_ff = false, any_rdist = false, any_rd = false;
+  bool any_geo = false;
   for (hp_job* j : jobs) {
     any_basis |= j->dev.gmat != nullptr;
     any_basis_ff |= j->dev.gmat_lo != nullptr;
     any_rdist |= j->dev.rdist != nullptr;
     any_rd |= j->dev.rd != nullptr;
+    any_geo |= j->dev.tgeo != nullptr;
   }
+  if (any_geo) launch_tile_rmin(hb, ctx->stream);
   if (any_rd) launch_rdist64(hb, ctx->stream);
   if (any_rdist) launch_rdist_ff(hb, ctx->stream);
   if (any_basis) launch_glisa_basis(hb, ctx->stream);
@@ -573,7 +581,7 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
           ProfScope ps(ctx, HP_KERNEL_INNER);
           launch_lisa_newton_inner(hb, st, mixed,
                                    j0->dev.solver == SOLVER_M_NEWTON || j0->dev.solver == SOLVER_BFGS);
-        }, j0->dev.inner_maxiter + 1);
+        }, j0->dev.inner_maxiter + 1, true);
       break;
   }
   if (rc) return rc;
@@ -1208,6 +1216,7 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   add(&J.jpart, 8 * (size_t)QJ_COUNT * ntile);
   add(&J.atom_out, 8 * (size_t)A * AO_COUNT);
   add(&J.active, 4 * (size_t)A); add(&J.inner_it, 4 * (size_t)A);
+  add(&J.arrive, 4 * (size_t)A);
   add(&J.ls_fail, 8 * (size_t)A * ntile);
   // GISA / aLISA in FP64 keep the (fixed) unit-population shells on the device
   // when the matrix takes at most half of the remaining budget: every pass
@@ -1279,6 +1288,7 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   if (cutoff) {
     add(&J.tgeo, 8 * 5 * (size_t)ntile);
     add(&J.amax, 4 * (size_t)A * ntile);
+    add(&J.rmin, 8 * (size_t)A * ntile);
   }
   add(&J.hist_propars, 8 * (size_t)maxiter * P);
   add(&J.hist_charges, 8 * (size_t)maxiter * A);
