@@ -525,7 +525,8 @@ enum Kind {
   K_HESS = 4,       // gLISA Hessian: (tile pair, point split)
   K_SQUARE = 5,     // gLISA reduce: ceil(nshell^2 / kThreads)
   K_FUSE = 7,       // fused gLISA pass: min(ntile, kFuseCtas) persistent blocks per job
-  K_NKIND = 8
+  K_SOLVE = 8,      // whole inner solve: natom * ceil(ntile / solve_tiles), all resident
+  K_NKIND = 9
 };
 
 // Persistent blocks of the fused gLISA pass per job (two per SM): each
@@ -536,6 +537,7 @@ constexpr int kFuseCtas = 2 * 152;
 struct HostBatch {
   Batch b[K_NKIND];
   int blocks[K_NKIND];
+  int solve_tiles = 0;  // K_SOLVE: tiles per block, 0 when the batch does not take it
   int nact_max = 0;  // fused gLISA: most active rows of a tile over the batch's jobs
 };
 
@@ -647,6 +649,8 @@ void launch_gisa_qp(const HostBatch& hb, cudaStream_t st);        // k_gisa_qp a
 void launch_rdist64(const HostBatch& hb, cudaStream_t st);  // rd of the batch's jobs
 void launch_promol64(const HostBatch& hb, cudaStream_t st);
 void launch_mbis_inner64(const HostBatch& hb, cudaStream_t st);
+int mbis_solve_capacity();
+void launch_mbis_solve64(const HostBatch& hb, cudaStream_t st);  // every inner iteration (K_SOLVE)
 void launch_change64(const HostBatch& hb, cudaStream_t st);
 void launch_final_atweights64(const HostBatch& hb, cudaStream_t st, int use_old);
 

@@ -76,16 +76,18 @@ __global__ void __launch_bounds__(kThreads) k_promol64(Batch bt) {
 // sum w e_k rho_a / pro and sum w e_k r rho_a / pro of the bare exponentials
 // e_k (the update multiplies by A_k) and the change sum w (oldpro - pro)^2.
 // Per pair 12 FP64 instructions a shell (9 of the exponential) and 13 more.
+// amp[2 k], cur[2 k + 1], prev[2 k], prev[2 k + 1]: the atom's amplitudes,
+// exponents and previous parameters; out: the tile's partials, stride ntile.
 template <int NSH>
 __device__ __forceinline__ void mbis_tile(const JobDev& J, int a, int tile, bool first,
-                                          const double* tab, double* red) {
+                                          const double* amp, const double* cur, const double* prev,
+                                          const double* tab, double* red, double* out) {
   constexpr int NQ = 2 * NSH + 1;
-  const int s0 = J.shell_off[a];
   double A[NSH], S[NSH], acc[NQ];
 #pragma unroll
   for (int k = 0; k < NSH; ++k) {
-    A[k] = J.keep[2 * (s0 + k)];
-    S[k] = -J.cur[2 * (s0 + k) + 1];
+    A[k] = amp[2 * k];
+    S[k] = -cur[2 * k + 1];
   }
 #pragma unroll
   for (int q = 0; q < NQ; ++q) acc[q] = 0.0;
@@ -135,14 +137,13 @@ __device__ __forceinline__ void mbis_tile(const JobDev& J, int a, int tile, bool
     if (!stored) {
       op = 0.0;
       for (int k = 0; k < NSH; ++k) {
-        const double n = J.prev[2 * (s0 + k)], s = J.prev[2 * (s0 + k) + 1];
+        const double n = prev[2 * k], s = prev[2 * k + 1];
         op = __fma_rn(f64::mbis_amp(n, s), f64::exp64(-s * r, tab), op);
       }
     }
     const double d = op - pro;
     acc[NQ - 1] = __fma_rn(w * d, d, acc[NQ - 1]);
   }
-  double* out = J.apart + ((size_t)a * J.qa + QA_INNER) * J.ntile + tile;
   const int nt = J.ntile;
   f64::block_sums<NQ>(acc, NQ, red, [&](int q, double v) {
     out[(size_t)(q == NQ - 1 ? kQ - 1 : q) * nt] = v;
@@ -150,11 +151,55 @@ __device__ __forceinline__ void mbis_tile(const JobDev& J, int a, int tile, bool
   if (old && threadIdx.x == 0) J.oldok[a * J.ntile + tile] = 1;
 }
 
+__device__ __forceinline__ void mbis_tile_n(int nsh, const JobDev& J, int a, int tile, bool first,
+                                            const double* amp, const double* cur, const double* prev,
+                                            const double* tab, double* red, double* out) {
+  switch (nsh) {
+    case 1: mbis_tile<1>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
+    case 2: mbis_tile<2>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
+    case 3: mbis_tile<3>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
+    case 4: mbis_tile<4>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
+    case 5: mbis_tile<5>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
+    case 6: mbis_tile<6>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
+    default: mbis_tile<7>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
+  }
+}
+
+// The per-atom cutoff of an inner iteration: rho_a below the cutoff on the
+// whole tile (the moments are exact zeros) and a negligible change term. The
+// tile's partials are zeroed and it is counted. One warp forms the bound: in
+// every thread it costs as much of the FP64 pipe as the tile itself. Uniform
+// over the block; skip_s: one int of shared memory.
+__device__ __forceinline__ bool mbis_skip(const JobDev& J, int a, int tile, int nsh, bool first,
+                                          const double* cur, const double* prev, const double* tab,
+                                          double* out, int* skip_s) {
+  if (!J.tgeo || !(J.amax[(size_t)a * J.ntile + tile] < (float)J.density_cutoff)) return false;
+  if (threadIdx.x < 32) {
+    const double b = f64::mbis_bound_warp(cur, first ? nullptr : prev, nsh, tile_rmin(J, a, tile), tab);
+    *skip_s = tile_weight(J, tile) * b * b < kSkipRel * J.inner_threshold * J.inner_threshold;
+  }
+  __syncthreads();
+  const bool skip = *skip_s != 0;
+  __syncthreads();
+  if (!skip) return false;
+  if (threadIdx.x < 2 * nsh) out[(size_t)threadIdx.x * J.ntile] = 0.0;
+  if (threadIdx.x == 0) {
+    out[(size_t)(kQ - 1) * J.ntile] = 0.0;
+    if (J.oldok) J.oldok[a * J.ntile + tile] = 0;
+    count_skipped(J, tile, 1.0);
+  }
+  return true;
+}
+
+__device__ __forceinline__ double* inner_partials(const JobDev& J, int a, int parity) {
+  return J.apart + ((size_t)a * J.qa + QA_INNER + parity * kQ) * J.ntile;
+}
+
 // MBIS inner iteration, one block per (atom, tile). Bound by the FP64 pipe:
 // about 30 FP64 instructions a pair at 1.5 shells, against ~150 when the
 // distance, the old pro-atom's exponentials, CUDA's exp and divide and the
 // sums of seven shells were all formed per pair. Two outer iterations of a
-// 22-atom chain of 320k points: 116.7 -> 34.5 ms.
+// 22-atom chain of 320k points: 116.7 -> 32.6 ms.
 __global__ void __launch_bounds__(kThreads) k_mbis_inner64(Batch bt) {
   __shared__ double tab[f64::kExpTab];
   __shared__ double red[kQ * kThreads];
@@ -167,39 +212,102 @@ __global__ void __launch_bounds__(kThreads) k_mbis_inner64(Batch bt) {
   __syncthreads();  // the table
   const int s0 = J.shell_off[a], nsh = J.shell_off[a + 1] - s0;
   const bool first = J.inner_it[a] == 0;
-  if (J.tgeo && J.amax[(size_t)a * J.ntile + tile] < (float)J.density_cutoff) {
-    // per-atom cutoff: rho_a below the cutoff on the whole tile (the moments
-    // are exact zeros); skip if the change term is negligible too. One warp
-    // forms the bound: in every thread it costs as much of the FP64 pipe as
-    // the tile itself
-    if (threadIdx.x < 32) {
-      const double b = f64::mbis_bound_warp(J.cur + 2 * s0, first ? nullptr : J.prev + 2 * s0, nsh,
-                                            tile_rmin(J, a, tile), tab);
-      skip_s = tile_weight(J, tile) * b * b < kSkipRel * J.inner_threshold * J.inner_threshold;
+  const double *amp = J.keep + 2 * s0, *cur = J.cur + 2 * s0, *prev = J.prev + 2 * s0;
+  double* out = inner_partials(J, a, 0) + tile;
+  if (!mbis_skip(J, a, tile, nsh, first, cur, prev, tab, out, &skip_s))
+    mbis_tile_n(nsh, J, a, tile, first, amp, cur, prev, tab, red, out);
+  if (last_block_of(J, a)) mbis_update(J, a);
+}
+
+// The whole inner solve of every atom in one launch, for batches small enough
+// that all blocks are resident (a cooperative launch): atom a's blocks (T
+// consecutive tiles each) go through its iterations together, meeting at a
+// counter per atom; each of them then sums the atom's partials in the order
+// of warp_tile_sum and forms the same new parameters, so nothing is handed
+// back. The partials alternate between two buffers: a block that is one
+// iteration ahead does not write what a slower one still reads. Bits as
+// k_mbis_inner64.
+// Water (3 atoms, 147 blocks) through the class: 21.1 -> 14.1 ms.
+// An iteration costs two L2 round trips beside the tiles' work instead of a
+// launch, cold instruction and data caches and an update at its end.
+// The wait is bounded: a block that runs out of polls sets E_TIMEOUT and
+// ends, and so do the others, each by its own bound.
+constexpr int kSolvePolls = 1 << 20;
+
+__global__ void __launch_bounds__(kThreads, 2) k_mbis_solve64(Batch bt, int T) {
+  __shared__ double tab[f64::kExpTab];
+  __shared__ double red[kQ * kThreads];
+  __shared__ double amp[2 * kMbisMaxShell], cur[2 * kMbisMaxShell], prev[2 * kMbisMaxShell];
+  __shared__ double m[kQ];
+  __shared__ int skip_s, late_s, state_s;
+  int local;
+  const JobDev& J = decode_local_mb(bt, local);
+  f64::load_exp64(tab, J.etab);
+  const int nb = (J.ntile + T - 1) / T;  // blocks of an atom
+  const int a = local / nb, b = local - a * nb;
+  const int s0 = J.shell_off[a], nsh = J.shell_off[a + 1] - s0;
+  const int t0 = b * T, t1 = min(t0 + T, J.ntile);
+  if (threadIdx.x < 2 * nsh) {
+    amp[threadIdx.x] = J.keep[2 * s0 + threadIdx.x];
+    cur[threadIdx.x] = prev[threadIdx.x] = J.cur[2 * s0 + threadIdx.x];
+  }
+  if (threadIdx.x == 0) late_s = 0;
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int it = 0;; ++it) {
+    double* part = inner_partials(J, a, it & 1);
+    for (int tile = t0; tile < t1; ++tile) {
+      if (!mbis_skip(J, a, tile, nsh, it == 0, cur, prev, tab, part + tile, &skip_s))
+        mbis_tile_n(nsh, J, a, tile, it == 0, amp, cur, prev, tab, red, part + tile);
+      __syncthreads();  // red, and this block's partials are written
+    }
+    if (threadIdx.x == 0) {
+      __threadfence();
+      atomicAdd(&J.arrive[a], 1);
+      const int target = (it + 1) * nb;
+      int polls = 0, seen;
+      do {
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(J.arrive + a) : "memory");
+      } while (seen < target && ++polls < kSolvePolls);
+      if (seen < target) late_s = 1;
     }
     __syncthreads();
-    if (skip_s) {
-      double* out = J.apart + ((size_t)a * J.qa + QA_INNER) * J.ntile + tile;
-      if (threadIdx.x < 2 * nsh) out[(size_t)threadIdx.x * J.ntile] = 0.0;
-      if (threadIdx.x == 0) {
-        out[(size_t)(kQ - 1) * J.ntile] = 0.0;
-        if (J.oldok) J.oldok[a * J.ntile + tile] = 0;
-        count_skipped(J, tile, 1.0);
-      }
-      if (last_block_of(J, a)) mbis_update(J, a);
+    if (late_s) {
+      if (threadIdx.x == 0) atomicOr(&J.mail->i[MI_ERR], E_TIMEOUT);
       return;
     }
+    for (int q = warp; q < 2 * nsh + 1; q += kWarps) {
+      const double v = warp_tile_sum_cg(J, part + (size_t)(q == 2 * nsh ? kQ - 1 : q) * J.ntile, J.ntile);
+      if (lane == 0) m[q] = v;
+    }
+    __syncthreads();
+    // the update (mbis_update): the parameters on warp 0, the test on warp 1
+    double n = 0.0, s = 0.0;
+    if (threadIdx.x < nsh) {
+      n = amp[2 * threadIdx.x] * m[2 * threadIdx.x];
+      s = 3.0 * m[2 * threadIdx.x] / m[2 * threadIdx.x + 1];
+      prev[2 * threadIdx.x] = cur[2 * threadIdx.x];
+      prev[2 * threadIdx.x + 1] = cur[2 * threadIdx.x + 1];
+      cur[2 * threadIdx.x] = n;
+      cur[2 * threadIdx.x + 1] = s;
+      amp[2 * threadIdx.x] = f64::mbis_amp(n, s);
+    } else if (threadIdx.x == 32) {
+      const double change = it == 0 ? 1e100 : sqrt(m[2 * nsh]);
+      state_s = change < J.inner_threshold ? 1 : it + 1 >= J.inner_maxiter ? 2 : 0;
+      if (b == 0) J.atom_out[a * AO_COUNT + AO_INNER_CHANGE] = change;
+    }
+    __syncthreads();
+    const int state = state_s;
+    if (state == 0) continue;
+    if (b == 0) {
+      if (threadIdx.x < 2 * nsh) J.propars[2 * s0 + threadIdx.x] = cur[threadIdx.x];
+      if (threadIdx.x == 0) {
+        inner_done(J, a, it + 1);
+        if (state == 2) atomicOr(&J.mail->i[MI_WARN], W_INNER);
+      }
+    }
+    return;
   }
-  switch (nsh) {
-    case 1: mbis_tile<1>(J, a, tile, first, tab, red); break;
-    case 2: mbis_tile<2>(J, a, tile, first, tab, red); break;
-    case 3: mbis_tile<3>(J, a, tile, first, tab, red); break;
-    case 4: mbis_tile<4>(J, a, tile, first, tab, red); break;
-    case 5: mbis_tile<5>(J, a, tile, first, tab, red); break;
-    case 6: mbis_tile<6>(J, a, tile, first, tab, red); break;
-    default: mbis_tile<7>(J, a, tile, first, tab, red); break;
-  }
-  if (last_block_of(J, a)) mbis_update(J, a);
 }
 
 // Outer change sum w (pro(new) - pro(old))^2 (core/iterstock.py:32-45).
@@ -289,6 +397,30 @@ void launch_promol64(const HostBatch& hb, cudaStream_t st) {
 
 void launch_mbis_inner64(const HostBatch& hb, cudaStream_t st) {
   launch_inner_kernel(k_mbis_inner64, hb, K_ATOM_TILE, st);
+}
+
+// Blocks of k_mbis_solve64 that are resident together on this device.
+int mbis_solve_capacity() {
+  static int dev_of = -1, cap = 0;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev_of != dev) {
+    int per_sm = 0, sms = 0, coop = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mbis_solve64, kThreads, 0);
+    cap = coop ? per_sm * sms : 0;
+    dev_of = dev;
+  }
+  return cap;
+}
+
+void launch_mbis_solve64(const HostBatch& hb, cudaStream_t st) {
+  Batch bt = hb.b[K_SOLVE];
+  int T = hb.solve_tiles;
+  void* args[] = {&bt, &T};
+  cudaLaunchCooperativeKernel((void*)k_mbis_solve64, dim3((unsigned)hb.blocks[K_SOLVE]), dim3(kThreads), args, 0, st);
+  ++g_launch_count;
 }
 
 void launch_change64(const HostBatch& hb, cudaStream_t st) {

@@ -280,10 +280,33 @@ int blocks_for(const JobDev& J, int kind) {
   return 0;
 }
 
+// FP64 MBIS on the molecular grid: tiles per block of k_mbis_solve64, the
+// fewest with which a batch's blocks are all resident, at most kSolveTiles
+// (0: one launch per inner iteration). With more tiles a block the launches
+// it saves count for little, and atoms that are done leave their blocks idle.
+constexpr int kSolveTiles = 4;
+
+int solve_blocks(const JobDev& J, int tiles) {
+  return tiles > 0 ? J.natom * ((J.ntile + tiles - 1) / tiles) : 0;
+}
+
+int solve_tiles(const std::vector<hp_job*>& jobs) {
+  const JobDev& J0 = jobs[0]->dev;
+  if (J0.scheme != SCHEME_MBIS || J0.mixed || J0.local) return 0;
+  const int cap = mbis_solve_capacity();
+  for (int t = 1; t <= kSolveTiles; ++t) {
+    int64_t blocks = 0;
+    for (const hp_job* j : jobs) blocks += solve_blocks(j->dev, t);
+    if (blocks <= cap) return t;
+  }
+  return 0;
+}
+
 // Upload the batch description (JobDev copies and per-kind block prefixes).
 int build_batch(hp_ctx* ctx, const std::vector<hp_job*>& jobs, HostBatch& hb) {
   const int n = (int)jobs.size();
   hb.nact_max = 0;
+  hb.solve_tiles = solve_tiles(jobs);
   for (int j = 0; j < n; ++j) {
     ctx->batch_host[j] = jobs[j]->dev;
     hb.nact_max = std::max(hb.nact_max, jobs[j]->dev.nact_max);
@@ -293,7 +316,8 @@ int build_batch(hp_ctx* ctx, const std::vector<hp_job*>& jobs, HostBatch& hb) {
   for (int k = 0; k < K_NKIND; ++k) {
     int* pre = ctx->prefix_host + (size_t)k * (kMaxSlots + 1);
     pre[0] = 0;
-    for (int j = 0; j < n; ++j) pre[j + 1] = pre[j] + blocks_for(jobs[j]->dev, k);
+    for (int j = 0; j < n; ++j)
+      pre[j + 1] = pre[j] + (k == K_SOLVE ? solve_blocks(jobs[j]->dev, hb.solve_tiles) : blocks_for(jobs[j]->dev, k));
     hb.blocks[k] = pre[n];
     hb.b[k].jobs = ctx->batch_dev;
     hb.b[k].prefix = ctx->prefix_dev + (size_t)k * (kMaxSlots + 1);
@@ -335,7 +359,7 @@ int status_of(int err) {
 }
 
 const char* err_text(int err) {
-  if (err & E_TIMEOUT) return "tensor-core Hessian: a bounded device wait ran out; MMAs issued before it may not have retired, so treat this context as suspect and recreate it";
+  if (err & E_TIMEOUT) return "a bounded device wait ran out (tensor-core Hessian: MMAs issued before it may not have retired; MBIS inner solve: a block of the atom did not arrive), so treat this context as suspect and recreate it";
   if (err & E_NEG_DENSITY) return "Negative pro-atom density found!";
   if (err & E_SINGULAR) return "Hessian is not positive definite (singular Newton system)";
   if (err & E_LINESEARCH) return "Line search failed!";
@@ -537,6 +561,10 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
         ProfScope ps(ctx, HP_KERNEL_INNER);
         launch_inner_init(hb, st);
         launch_mbis_local(hb, st);
+      } else if (!mixed && hb.solve_tiles > 0) {  // the same in one cooperative launch
+        ProfScope ps(ctx, HP_KERNEL_INNER);
+        launch_inner_init(hb, st);
+        launch_mbis_solve64(hb, st);
       } else {
         rc = run_inner(ctx, jobs, hb, [&] {
           ProfScope ps(ctx, HP_KERNEL_INNER);
@@ -1137,6 +1165,7 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   const int tile_points = kThreads * ppt;
   const int ntile = (N + tile_points - 1) / tile_points;
   int qa = 2 + std::max(2 * 7 + 1, kMaxShells + 1);
+  if (mbis && d->precision == HP_PRECISION_FP64) qa = 2 + 2 * (2 * kMbisMaxShell + 1);  // k_mbis_solve64
   if (d->scheme == HP_SCHEME_LISA && solver != HP_SOLVER_SC) qa = 2 + kNewtonQ(kmax);
   const int maxiter = d->maxiter;
   // gLISA keeps FP64 evaluation; its mixed mode is the tensor-core Hessian

@@ -74,3 +74,23 @@ def test_stored_pairs_are_given_back_and_change_no_bits():
     assert used < kept
     for key in stored:
         np.testing.assert_array_equal(stored[key], recomputed[key])
+
+
+@pytest.mark.parametrize("npoint", [513, 2400])
+def test_one_launch_solve_has_the_bits_of_the_stepwise_one(npoint, gpu_context):
+    """A small job alone takes the cooperative inner solve; beside a large one, a launch per inner iteration."""
+    small = _pair(8, npoint)
+    mol = synthetic.chain_molecule({6: 6, 1: 8}, 40, 110, seed=9)
+    results = []
+    for others in (False, True):
+        jobs = [_job(gpu_context, *small, maxiter=3, threshold=1e-14)]
+        if others:
+            jobs.append(_job(gpu_context, mol.coordinates, mol.numbers, mol.grid, mol.density, maxiter=3))
+        for _ in range(3):
+            gpu_context.step(jobs)
+        results.append((jobs[0].results(at_weights=True), jobs[0].info().inner_iterations))
+        for j in jobs:
+            j.close()
+    assert results[0][1] == results[1][1]
+    for key in results[0][0]:
+        np.testing.assert_array_equal(results[0][0][key], results[1][0][key])
