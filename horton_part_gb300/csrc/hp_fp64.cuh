@@ -105,18 +105,23 @@ __device__ __forceinline__ double mbis_bound_warp(const double* pn, const double
 // Block sums of nq <= Q per-thread values: the warps' values of a lane are
 // added first (from shared memory, warp q for quantity q), then the lanes,
 // which takes 12 warp-wide additions a quantity instead of 48. put(q, sum)
-// is called by lane 0 of a warp. red: Q * kThreads doubles.
+// is called by lane 0 of a warp. red: Q * kThreads doubles. nw: warps that
+// have values (the others' are left out).
 template <int Q, typename Put>
-__device__ __forceinline__ void block_sums(const double (&acc)[Q], int nq, double* red, Put put) {
+__device__ __forceinline__ void block_sums(const double (&acc)[Q], int nq, double* red, Put put,
+                                           int nw = kWarps) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < nw) {
 #pragma unroll
-  for (int q = 0; q < Q; ++q)
-    if (q < nq) red[q * kThreads + threadIdx.x] = acc[q];
+    for (int q = 0; q < Q; ++q)
+      if (q < nq) red[q * kThreads + threadIdx.x] = acc[q];
+  }
   __syncthreads();
   for (int q = warp; q < nq; q += kWarps) {
     double v = red[q * kThreads + lane];
 #pragma unroll
-    for (int w = 1; w < kWarps; ++w) v += red[q * kThreads + 32 * w + lane];
+    for (int w = 1; w < kWarps; ++w)
+      if (w < nw) v += red[q * kThreads + 32 * w + lane];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (lane == 0) put(q, v);

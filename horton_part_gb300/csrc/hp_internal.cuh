@@ -544,7 +544,7 @@ struct HostBatch {
 void launch_nelec(const HostBatch& hb, cudaStream_t st);
 void launch_tile_rmin(const HostBatch& hb, cudaStream_t st);
 void launch_copy_old(const HostBatch& hb, cudaStream_t st);
-void launch_promol(const HostBatch& hb, cudaStream_t st, int mixed, int model);
+void launch_promol(const HostBatch& hb, cudaStream_t st, int mixed, int model, bool weights = true);
 void launch_final_atweights(const HostBatch& hb, cudaStream_t st, int mixed, int model, int use_old);
 void launch_change(const HostBatch& hb, cudaStream_t st, int mixed, int model);
 void launch_outer_finish(const HostBatch& hb, cudaStream_t st, int with_charges);
@@ -639,7 +639,8 @@ void launch_lisa_sc_inner_mx(const HostBatch& hb, cudaStream_t st);
 void launch_final_atweights_mx(const HostBatch& hb, cudaStream_t st, int model, int use_old);
 
 // MBIS on atom grids (hp_local.cu)
-void launch_mbis_local(const HostBatch& hb, cudaStream_t st);  // spherical averages + radial inner solve
+// spherical averages + radial inner solve + change (FP64: and the at_weights)
+void launch_mbis_local(const HostBatch& hb, cudaStream_t st, int mixed);
 void launch_change_radial(const HostBatch& hb, cudaStream_t st);
 void launch_gisa_local(const HostBatch& hb, cudaStream_t st);     // spherical averages + radial moments
 void launch_lisa_sc_local(const HostBatch& hb, cudaStream_t st);  // spherical averages + radial sc solve
@@ -647,7 +648,7 @@ void launch_gisa_qp(const HostBatch& hb, cudaStream_t st);        // k_gisa_qp a
 
 // FP64 MBIS (hp_mbis.cu)
 void launch_rdist64(const HostBatch& hb, cudaStream_t st);  // rd of the batch's jobs
-void launch_promol64(const HostBatch& hb, cudaStream_t st);
+void launch_promol64(const HostBatch& hb, cudaStream_t st, bool weights);  // weights: k_atweights too
 void launch_mbis_inner64(const HostBatch& hb, cudaStream_t st);
 int mbis_solve_capacity();
 void launch_mbis_solve64(const HostBatch& hb, cudaStream_t st);  // every inner iteration (K_SOLVE)

@@ -2686,10 +2686,11 @@ void launch_copy_old(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_copy_ol
 
 // FP32 variants live in hp_mixed.cu, float-float (MBIS) in hp_ff.cu; `mixed`
 // is the job group's evaluation phase (Phase).
-void launch_promol(const HostBatch& hb, cudaStream_t st, int mixed, int model) {
+// weights false: without the at_weights pass (FP64 MBIS on atom grids).
+void launch_promol(const HostBatch& hb, cudaStream_t st, int mixed, int model, bool weights) {
   if (mixed == PH_FF && model == MODEL_MBIS) return launch_promol_ff(hb, st);
   if (mixed) return launch_promol_mx(hb, st, model);
-  if (model == MODEL_MBIS) return launch_promol64(hb, st);
+  if (model == MODEL_MBIS) return launch_promol64(hb, st, weights);
   if (model == MODEL_NLIS) HP_LAUNCH((k_promol<double, MODEL_NLIS>), K_POINT1, kThreads);
   else HP_LAUNCH((k_promol<double, MODEL_BASIS>), K_POINT1, kThreads);
   HP_LAUNCH(k_atweights, K_ATOM_TILE, kThreads);

@@ -19,7 +19,7 @@
 // weights wsph (Lebedev weight / 4 pi, summing to 1 over a shell).
 #include <math.h>
 
-#include "hp_internal.cuh"
+#include "hp_fp64.cuh"
 
 namespace hp {
 
@@ -75,24 +75,75 @@ __global__ void __launch_bounds__(kThreads) k_sph_avg(Batch bt) {
   }
 }
 
+// FP64 jobs: the spherical averages straight from the pro-atoms k_promol64
+// left in rhoa, at_weights formed on the atom's own points only (no other
+// point of its row is used here); kAvgSplit blocks per atom, warps over its
+// radial shells.
+constexpr int kAvgSplit = 8;
+
+__global__ void __launch_bounds__(kThreads) k_sph_avg64(Batch bt) {
+  const int blk = blockIdx.x / kAvgSplit, part = blockIdx.x - blk * kAvgSplit;
+  const int j = find_job(bt, blk);
+  const JobDev& J = bt.jobs[j];
+  const int a = blk - bt.prefix[j];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double* pro = J.rhoa + (size_t)a * J.npoint;
+  for (int s = J.rad_off[a] + part * kWarps + warp; s < J.rad_off[a + 1]; s += kAvgSplit * kWarps) {
+    double v = 0.0;
+    for (long long p = J.shell_pt[s] + lane; p < J.shell_pt[s + 1]; p += 32) {
+      const double aw = fmin(fmax(pro[p] * J.invpro[p], 0.0), 1.0);
+      v += J.wsph[p] * (aw * J.rho[p]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) J.radrho[s] = v;
+  }
+}
+
+// The entropy partials of k_atweights, one block per point tile.
+__global__ void __launch_bounds__(kThreads) k_entropy64(Batch bt) {
+  __shared__ double red[kThreads];
+  int tile;
+  const JobDev& J = decode_atom_lc(bt, tile);  // (the block's index within its job)
+  double acc[1] = {0.0};
+  const int p1 = min((tile + 1) * J.tile_points, J.npoint);
+  for (int p = tile * J.tile_points + threadIdx.x; p < p1; p += kThreads) {
+    const double promol = J.promol[p], rho = J.rho[p];
+    if (!((promol < J.density_cutoff) || (rho < J.density_cutoff)))
+      acc[0] += J.w[p] * rho * log(rho / promol);
+  }
+  f64::block_sums<1>(acc, 1, red, [&](int, double v) {
+    J.jpart[(size_t)QJ_ENTROPY * J.ntile + tile] = v;
+  });
+}
+
 // Inner MBIS fixed point of every atom on its radial grid (one block per
-// atom, every inner iteration in this launch), population and charge input.
-__global__ void __launch_bounds__(kThreads) k_mbis_radial(Batch bt) {
-  __shared__ double red[kWarps * kLocalQ];
-  __shared__ double out[kLocalQ];
-  __shared__ double par[14];
-  __shared__ int done_s;
-  int a;
-  const JobDev& J = decode_atom_lc(bt, a);
-  const int r0 = J.rad_off[a], nrad = J.rad_off[a + 1] - r0;
-  const int nsh = J.shell_off[a + 1] - J.shell_off[a];
-  double* pa = J.propars + J.par_off[a];
-  if (threadIdx.x < 2 * nsh) par[threadIdx.x] = pa[threadIdx.x];
-  if (threadIdx.x == 0) done_s = 0;
-  // this thread's radial nodes (nrad <= kLocalMaxRad = 4 x kThreads)
+// atom, every inner iteration in this launch), population and charge input,
+// and the outer change sum_i 4 pi r_i^2 w_i (pro_new - pro_old)^2.
+// Bound by latency: an iteration is a chain of ~45 dependent FP64
+// instructions on one SM, ~40 of them issued per node and shell pair; only
+// the warps that hold nodes issue any (75 nodes: 3 of the 32 slots that 1024
+// nodes fill). See hp_fp64.cuh for the arithmetic. 9 atoms x 75 nodes: 1344
+// us a launch when every slot was evaluated.
+template <int NSH>
+__device__ __forceinline__ void mbis_radial(const JobDev& J, int a, const double* tab, double* red) {
   constexpr int kPer = kLocalMaxRad / kThreads;
+  constexpr int NQ = 2 * NSH + 1;
+  __shared__ double amp[NSH], sx[NSH], m[NQ];
+  __shared__ int state_s;
+  const int r0 = J.rad_off[a], nrad = J.rad_off[a + 1] - r0;
+  double* pa = J.propars + J.par_off[a];
+  const double* po = J.propars_old + J.par_off[a];
+  if (threadIdx.x < NSH) {
+    amp[threadIdx.x] = f64::mbis_amp(pa[2 * threadIdx.x], pa[2 * threadIdx.x + 1]);
+    sx[threadIdx.x] = pa[2 * threadIdx.x + 1];
+  }
+  // this thread's radial nodes threadIdx.x + q kThreads; slots whose whole
+  // warp is past the last node are skipped
+  const int base = threadIdx.x & ~31;
+  const int nw = min(kWarps, (nrad + 31) / 32);
   double rr[kPer], ww[kPer], rh[kPer], oldpro[kPer];
-  double pop = 0.0;
+  double pop[1] = {0.0};
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
     const int i = threadIdx.x + q * kThreads;
@@ -101,64 +152,96 @@ __global__ void __launch_bounds__(kThreads) k_mbis_radial(Batch bt) {
     ww[q] = in ? 4.0 * M_PI * rr[q] * rr[q] * J.rad_w[r0 + i] : 0.0;
     rh[q] = in ? J.radrho[r0 + i] : 0.0;
     oldpro[q] = 0.0;
-    pop += ww[q] * rh[q];
+    pop[0] += ww[q] * rh[q];
   }
-  {
-    double acc1[1] = {pop};
-    block_sum<1>(acc1, red, out);
-    put_atom_partial(J, a, QA_POP, out[0]);
-  }
+  f64::block_sums<1>(pop, 1, red, [&](int, double v) { m[0] = v; }, nw);
   __syncthreads();
+  put_atom_partial(J, a, QA_POP, m[0]);
+  __syncthreads();
+  const double cut = J.density_cutoff;
   int it = 0;
-  double change = 1e100;
-  for (; it < J.inner_maxiter; ++it) {
-    double acc[kLocalQ];
+  for (;; ++it) {
+    double acc[NQ], A[NSH], S[NSH];
 #pragma unroll
-    for (int q = 0; q < kLocalQ; ++q) acc[q] = 0.0;
+    for (int q = 0; q < NQ; ++q) acc[q] = 0.0;
+#pragma unroll
+    for (int k = 0; k < NSH; ++k) {
+      A[k] = amp[k];
+      S[k] = -sx[k];
+    }
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
-      double t[7];
-      double pro = 0.0;
+      if (base + q * kThreads >= nrad) break;
+      double e[NSH], pro = 0.0;
 #pragma unroll
-      for (int k = 0; k < 7; ++k) {
-        t[k] = 0.0;
-        if (k < nsh) {
-          const double n = par[2 * k], s = par[2 * k + 1];
-          t[k] = n * s * s * s * exp(-s * rr[q]) * kInv8Pi;
-          pro += t[k];
-        }
+      for (int k = 0; k < NSH; ++k) {
+        e[k] = f64::exp64(S[k] * rr[q], tab);
+        pro = __fma_rn(A[k], e[k], pro);
       }
-      const bool sick = (rh[q] < J.density_cutoff) || (pro < J.density_cutoff);
-      const double ratio = sick ? 0.0 : rh[q] / pro;
+      const bool sick = (rh[q] < cut) || (pro < cut);
+      const double wr = sick ? 0.0 : ww[q] * f64::div64(rh[q], sick ? 1.0 : pro);
+      const double wrr = wr * rr[q];
 #pragma unroll
-      for (int k = 0; k < 7; ++k) {
-        if (k < nsh) {
-          const double m0 = ww[q] * t[k] * ratio;
-          acc[2 * k] += m0;
-          acc[2 * k + 1] += m0 * rr[q];
-        }
+      for (int k = 0; k < NSH; ++k) {
+        acc[2 * k] = __fma_rn(e[k], wr, acc[2 * k]);
+        acc[2 * k + 1] = __fma_rn(e[k], wrr, acc[2 * k + 1]);
       }
-      const double e = oldpro[q] - pro;
-      acc[kLocalQ - 1] += ww[q] * e * e;
+      const double d = oldpro[q] - pro;
+      acc[NQ - 1] = __fma_rn(ww[q] * d, d, acc[NQ - 1]);
       oldpro[q] = pro;
     }
-    block_sum<kLocalQ>(acc, red, out);
-    if (threadIdx.x == 0) {
-      for (int k = 0; k < nsh; ++k) {
-        par[2 * k] = out[2 * k];
-        par[2 * k + 1] = 3.0 * out[2 * k] / out[2 * k + 1];
-      }
-      change = it == 0 ? 1e100 : sqrt(out[kLocalQ - 1]);
-      done_s = change < J.inner_threshold;
+    f64::block_sums<NQ>(acc, NQ, red, [&](int q, double v) { m[q] = v; }, nw);
+    __syncthreads();
+    if (threadIdx.x < NSH) {
+      const int k = threadIdx.x;
+      const double n = amp[k] * m[2 * k], s = 3.0 * m[2 * k] / m[2 * k + 1];
+      pa[2 * k] = n;
+      pa[2 * k + 1] = s;
+      sx[k] = s;
+      amp[k] = f64::mbis_amp(n, s);
+    } else if (threadIdx.x == 32) {
+      const double change = it == 0 ? 1e100 : sqrt(m[NQ - 1]);
+      state_s = change < J.inner_threshold ? 1 : it + 1 >= J.inner_maxiter ? 2 : 0;
     }
     __syncthreads();
-    if (done_s) break;
+    if (state_s) break;
   }
-  if (threadIdx.x < 2 * nsh) pa[threadIdx.x] = par[threadIdx.x];
+  // the outer change against the parameters at the start of the iteration
+  double chg[1] = {0.0};
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    if (base + q * kThreads >= nrad) break;
+    double d = 0.0;
+    for (int k = 0; k < NSH; ++k) {
+      d = __fma_rn(amp[k], f64::exp64(-sx[k] * rr[q], tab), d);
+      d = __fma_rn(-f64::mbis_amp(po[2 * k], po[2 * k + 1]), f64::exp64(-po[2 * k + 1] * rr[q], tab), d);
+    }
+    chg[0] = __fma_rn(ww[q] * d, d, chg[0]);
+  }
+  f64::block_sums<1>(chg, 1, red, [&](int, double v) { m[0] = v; }, nw);
+  __syncthreads();
+  put_atom_partial(J, a, QA_CHANGE, m[0]);
   if (threadIdx.x == 0) {
-    const bool conv = it < J.inner_maxiter;
-    atomicAdd(&J.mail->d[MD_INNER_TOTAL], (double)(conv ? it + 1 : J.inner_maxiter));
-    if (!conv) atomicOr(&J.mail->i[MI_WARN], W_INNER);
+    atomicAdd(&J.mail->d[MD_INNER_TOTAL], (double)(it + 1));
+    if (state_s == 2) atomicOr(&J.mail->i[MI_WARN], W_INNER);
+  }
+}
+
+__global__ void __launch_bounds__(kThreads) k_mbis_radial(Batch bt) {
+  __shared__ double tab[f64::kExpTab];
+  __shared__ double red[kLocalQ * kThreads];
+  int a;
+  const JobDev& J = decode_atom_lc(bt, a);
+  f64::load_exp64(tab, J.etab);
+  __syncthreads();
+  switch (J.shell_off[a + 1] - J.shell_off[a]) {
+    case 1: mbis_radial<1>(J, a, tab, red); break;
+    case 2: mbis_radial<2>(J, a, tab, red); break;
+    case 3: mbis_radial<3>(J, a, tab, red); break;
+    case 4: mbis_radial<4>(J, a, tab, red); break;
+    case 5: mbis_radial<5>(J, a, tab, red); break;
+    case 6: mbis_radial<6>(J, a, tab, red); break;
+    default: mbis_radial<7>(J, a, tab, red); break;
   }
 }
 
@@ -209,6 +292,7 @@ __global__ void __launch_bounds__(kThreads) k_nlis_radial(Batch bt) {
     for (int q = 0; q < kLocalQ; ++q) acc[q] = 0.0;
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
+      if ((int)(threadIdx.x & ~31u) + q * kThreads >= nrad) break;  // no node of this warp
       double u[7], rn[7];
       double pro = 0.0;
 #pragma unroll
@@ -257,8 +341,9 @@ __global__ void __launch_bounds__(kThreads) k_nlis_radial(Batch bt) {
 }
 
 // Outer change on the radial grids: sum_i 4 pi r_i^2 w_i (pro_new - pro_old)^2
-// (MBIS: Slater shells of both parameter sets; basis schemes: the parameter
-// differences times the unit-population shells at the nodes).
+// (NLIS: the shells of both parameter sets; basis schemes: the parameter
+// differences times the unit-population shells at the nodes; MBIS forms it
+// in k_mbis_radial).
 __global__ void __launch_bounds__(kThreads) k_change_radial(Batch bt) {
   __shared__ double red[kWarps];
   int a;
@@ -268,7 +353,6 @@ __global__ void __launch_bounds__(kThreads) k_change_radial(Batch bt) {
   const int s0 = J.shell_off[a], nsh = J.shell_off[a + 1] - s0;
   const double* pn = J.propars + J.par_off[a];
   const double* po = J.propars_old + J.par_off[a];
-  const bool mbis = J.scheme == SCHEME_MBIS;
   const bool nlis = J.scheme == SCHEME_NLIS;
   double acc = 0.0;
   for (int i = threadIdx.x; i < nrad; i += kThreads) {
@@ -278,9 +362,6 @@ __global__ void __launch_bounds__(kThreads) k_change_radial(Batch bt) {
       if (nlis) {
         d += nlis_shell(pn[3 * k], pn[3 * k + 1], pn[3 * k + 2], r);
         d -= nlis_shell(po[3 * k], po[3 * k + 1], po[3 * k + 2], r);
-      } else if (mbis) {
-        d += pn[2 * k] * pn[2 * k + 1] * pn[2 * k + 1] * pn[2 * k + 1] * exp(-pn[2 * k + 1] * r) * kInv8Pi;
-        d -= po[2 * k] * po[2 * k + 1] * po[2 * k + 1] * po[2 * k + 1] * exp(-po[2 * k + 1] * r) * kInv8Pi;
       } else {
         d += (pn[k] - po[k]) * radial_shell(J, s0 + k, r);
       }
@@ -361,6 +442,7 @@ __global__ void __launch_bounds__(kThreads) k_lisa_sc_radial(Batch bt) {
     for (int q = 0; q <= kMaxShells; ++q) acc[q] = 0.0;
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
+      if ((int)(threadIdx.x & ~31u) + q * kThreads >= nrad) break;  // no node of this warp
       double pro = 0.0;
       for (int k = 0; k < nsh; ++k) pro += par[k] * radial_shell(J, s0 + k, rr[q]);
       const bool sick = (rh[q] < J.density_cutoff) || (pro < J.density_cutoff);
@@ -398,8 +480,16 @@ __global__ void __launch_bounds__(kThreads) k_lisa_sc_radial(Batch bt) {
     }                                                                                  \
   } while (0)
 
-void launch_mbis_local(const HostBatch& hb, cudaStream_t st) {
-  HP_LAUNCH_LC(k_sph_avg, K_ATOM, kThreads);
+// at_weights on the atoms' own points with the spherical averages (FP64: the
+// promolecule pass alone came before), then the radial solves.
+void launch_mbis_local(const HostBatch& hb, cudaStream_t st, int mixed) {
+  if (mixed) {
+    HP_LAUNCH_LC(k_sph_avg, K_ATOM, kThreads);
+  } else {
+    HP_LAUNCH_LC(k_entropy64, K_POINT, kThreads);
+    k_sph_avg64<<<hb.blocks[K_ATOM] * kAvgSplit, kThreads, 0, st>>>(hb.b[K_ATOM]);
+    ++g_launch_count;
+  }
   HP_LAUNCH_LC(k_mbis_radial, K_ATOM, kThreads);
 }
 

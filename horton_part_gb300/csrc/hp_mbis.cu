@@ -390,9 +390,9 @@ __global__ void __launch_bounds__(kThreads) k_final_atweights64(Batch bt, int us
 
 void launch_rdist64(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH_MB(k_rdist64, K_POINT1, kThreads); }
 
-void launch_promol64(const HostBatch& hb, cudaStream_t st) {
+void launch_promol64(const HostBatch& hb, cudaStream_t st, bool weights) {
   HP_LAUNCH_MB(k_promol64, K_POINT1, kThreads);
-  launch_atweights(hb, st);
+  if (weights) launch_atweights(hb, st);
 }
 
 void launch_mbis_inner64(const HostBatch& hb, cudaStream_t st) {

@@ -547,20 +547,20 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
   const hp_job* j0 = jobs[0];
   const int mixed = j0->dev.mixed;  // current phase (a mixed job may finish in FP64)
   const int model = model_of(j0);
+  const bool local = j0->dev.local != 0;
   cudaStream_t st = ctx->stream;
   launch_copy_old(hb, st);
   {
     ProfScope ps(ctx, HP_KERNEL_PROMOL);
-    launch_promol(hb, st, mixed, model);
+    launch_promol(hb, st, mixed, model, !(local && model == MODEL_MBIS && !mixed));
   }
   int rc = HP_OK;
-  const bool local = j0->dev.local != 0;
   switch (j0->desc.scheme) {
     case HP_SCHEME_MBIS:
       if (local) {  // atom grids: every inner iteration of every atom in one launch
         ProfScope ps(ctx, HP_KERNEL_INNER);
         launch_inner_init(hb, st);
-        launch_mbis_local(hb, st);
+        launch_mbis_local(hb, st, mixed);
       } else if (!mixed && hb.solve_tiles > 0) {  // the same in one cooperative launch
         ProfScope ps(ctx, HP_KERNEL_INNER);
         launch_inner_init(hb, st);
@@ -615,8 +615,11 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
   if (rc) return rc;
   {
     ProfScope ps(ctx, HP_KERNEL_CHANGE);
-    if (local) launch_change_radial(hb, st);
-    else launch_change(hb, st, mixed, model);
+    if (local) {
+      if (model != MODEL_MBIS) launch_change_radial(hb, st);  // MBIS: in the radial solve
+    } else {
+      launch_change(hb, st, mixed, model);
+    }
   }
   launch_outer_finish(hb, st, 1);
   rc = check_launch();
