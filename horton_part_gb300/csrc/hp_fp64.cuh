@@ -102,6 +102,31 @@ __device__ __forceinline__ double mbis_bound_warp(const double* pn, const double
   return b;
 }
 
+// The bound sum_k |a_k - b_k| g_k(r) of a basis scheme (shells s0 .. s0 + nsh
+// - 1, which decrease with r): one warp, a shell a lane.
+__device__ __forceinline__ double basis_bound_warp(const JobDev& J, int s0, int nsh, const double* a,
+                                                   const double* b, double r, const double* tab) {
+  const int k = threadIdx.x & 31;
+  double s = 0.0;
+  if (k < nsh) {
+    const double order = J.sh_order[s0 + k];
+    const double rn = order == 2.0 ? r * r : order == 1.0 ? r : pow(r, order);
+    s = fabs(a[k] - b[k]) * J.sh_pref[s0 + k] * exp64(-J.sh_alpha[s0 + k] * rn, tab);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// fmin(fmax(x, 0), 1) by integer comparisons (NaN gives 0, as fmax does).
+__device__ __forceinline__ double clip01(double x) {
+  const int hi = __double2hiint(x);
+  if ((unsigned)hi < 0x3ff00000u) return x;
+  if (hi < 0) return 0.0;
+  const long long b = __double_as_longlong(x);
+  return b > 0x7ff0000000000000ll ? 0.0 : 1.0;
+}
+
 // Block sums of nq <= Q per-thread values: the warps' values of a lane are
 // added first (from shared memory, warp q for quantity q), then the lanes,
 // which takes 12 warp-wide additions a quantity instead of 48. put(q, sum)

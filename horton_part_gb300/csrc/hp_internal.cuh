@@ -213,8 +213,11 @@ struct JobDev {
   // FP64 kernels (hp_fp64.cuh)
   const double* etab;     // 2^(j/512), j < 512
   double* rd;             // MBIS: distances [natom][npoint], or null (recomputed)
-  double* oldpro;         // MBIS: pro-atoms of the last inner iteration [natom][npoint], or null;
-  int* oldok;             // valid where oldok[natom][ntile] is set
+  double* oldpro;         // MBIS, aLISA sc with G: pro-atoms of the last inner iteration
+                          // [natom][npoint], or null; valid where oldok[natom][ntile] is set
+  int* oldok;
+  unsigned* smask;        // jobs with gmat: per (atom, tile) the atom's shells that are nonzero
+                          // somewhere on the tile [natom][ntile], bit k = its shell k
   double* hist_propars;   // [maxiter][nparam]
   double* hist_charges;   // [maxiter][natom]
   double* hist_ent;       // [maxiter]
@@ -537,6 +540,7 @@ constexpr int kFuseCtas = 2 * 152;
 struct HostBatch {
   Batch b[K_NKIND];
   int blocks[K_NKIND];
+  bool any_g = false, any_nog = false;  // some job stores the FP64 basis matrix / some does not
   int solve_tiles = 0;  // K_SOLVE: tiles per block, 0 when the batch does not take it
   int nact_max = 0;  // fused gLISA: most active rows of a tile over the batch's jobs
 };
@@ -558,7 +562,6 @@ void launch_nlis_local(const HostBatch& hb, cudaStream_t st);  // spherical aver
 void launch_gisa(const HostBatch& hb, cudaStream_t st, int mixed);
 void launch_lisa_sc_inner(const HostBatch& hb, cudaStream_t st, int mixed);
 void launch_lisa_newton_inner(const HostBatch& hb, cudaStream_t st, int mixed, int modified);
-void launch_glisa_basis(const HostBatch& hb, cudaStream_t st);
 void launch_glisa_pro(const HostBatch& hb, cudaStream_t st);
 void launch_glisa_grad(const HostBatch& hb, cudaStream_t st);
 void launch_glisa_hess(const HostBatch& hb, cudaStream_t st);
@@ -642,8 +645,8 @@ void launch_final_atweights_mx(const HostBatch& hb, cudaStream_t st, int model, 
 // spherical averages + radial inner solve + change (FP64: and the at_weights)
 void launch_mbis_local(const HostBatch& hb, cudaStream_t st, int mixed);
 void launch_change_radial(const HostBatch& hb, cudaStream_t st);
-void launch_gisa_local(const HostBatch& hb, cudaStream_t st);     // spherical averages + radial moments
-void launch_lisa_sc_local(const HostBatch& hb, cudaStream_t st);  // spherical averages + radial sc solve
+void launch_gisa_local(const HostBatch& hb, cudaStream_t st, int mixed);     // spherical averages + radial moments
+void launch_lisa_sc_local(const HostBatch& hb, cudaStream_t st, int mixed);  // spherical averages + radial sc solve
 void launch_gisa_qp(const HostBatch& hb, cudaStream_t st);        // k_gisa_qp alone
 
 // FP64 MBIS (hp_mbis.cu)
@@ -654,6 +657,14 @@ int mbis_solve_capacity();
 void launch_mbis_solve64(const HostBatch& hb, cudaStream_t st);  // every inner iteration (K_SOLVE)
 void launch_change64(const HostBatch& hb, cudaStream_t st);
 void launch_final_atweights64(const HostBatch& hb, cudaStream_t st, int use_old);
+
+// FP64 basis schemes over the stored G (hp_basis.cu); jobs without one are skipped
+void launch_basis64(const HostBatch& hb, cudaStream_t st);
+void launch_promol_g64(const HostBatch& hb, cudaStream_t st);
+void launch_gisa_moments64(const HostBatch& hb, cudaStream_t st);  // at_weights and q-vector moments
+void launch_lisa_sc64(const HostBatch& hb, cudaStream_t st);
+void launch_change_g64(const HostBatch& hb, cudaStream_t st);
+void launch_entropy64(const HostBatch& hb, cudaStream_t st);       // entropy partials (hp_local.cu)
 
 // float-float MBIS (hp_ff.cu)
 void launch_promol_ff(const HostBatch& hb, cudaStream_t st);

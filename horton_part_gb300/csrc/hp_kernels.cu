@@ -251,6 +251,7 @@ template <typename T, int MODEL>
 __global__ void __launch_bounds__(kThreads) k_promol(Batch bt) {
   int blk;
   const JobDev& J = decode_local(bt, blk);
+  if (MODEL == MODEL_BASIS && J.gmat) return;  // k_promol_g64
   const int p = blk * kThreads + threadIdx.x;
   if (p >= J.npoint) return;
   double promol = 0.0;
@@ -272,6 +273,7 @@ __global__ void __launch_bounds__(kThreads) k_atweights(Batch bt) {
   const JobDev* Jp;
   const AtomTile at = decode_atom_tile(bt, Jp);
   const JobDev& J = *Jp;
+  if (J.scheme == SCHEME_GISA && J.gmat) return;  // k_gisa_moments64
   double acc[2] = {0.0, 0.0};
   float vmax = 0.0f;  // largest rho_a on the tile (per-atom cutoff)
   double* ra = J.rhoa + (size_t)at.atom * J.npoint;
@@ -280,10 +282,10 @@ __global__ void __launch_bounds__(kThreads) k_atweights(Batch bt) {
     if (p >= J.npoint) continue;
     const double promol = J.promol[p];
     const double rho = J.rho[p];
-    const double aw = fmin(fmax(ra[p] * J.invpro[p], 0.0), 1.0);
+    const double aw = f64::clip01(ra[p] * J.invpro[p]);
     const double v = aw * rho;
     ra[p] = v;
-    vmax = fmaxf(vmax, v > 3e38 ? 3e38f : (float)v);
+    if (J.amax) vmax = fmaxf(vmax, v > 3e38 ? 3e38f : (float)v);
     acc[0] += J.w[p] * v;
     if (at.atom == 0) {
       const bool sick = (promol < J.density_cutoff) || (rho < J.density_cutoff);
@@ -328,6 +330,7 @@ __global__ void __launch_bounds__(kThreads) k_change(Batch bt) {
   const JobDev* Jp;
   const AtomTile at = decode_atom_tile(bt, Jp);
   const JobDev& J = *Jp;
+  if (MODEL == MODEL_BASIS && J.gmat) return;  // k_change_g64
   if (MODEL != MODEL_NLIS && J.tgeo) {  // per-atom cutoff: bound of the pair's change term
     const double r = tile_rmin(J, at.atom, at.tile);
     const int s0 = J.shell_off[at.atom], nsh = J.shell_off[at.atom + 1] - s0;
@@ -347,17 +350,8 @@ __global__ void __launch_bounds__(kThreads) k_change(Batch bt) {
     const int p = point_of(J, at.tile, i);
     if (p >= J.npoint) continue;
     const T r = dist_for<T, MODEL>(J, p, at.atom);
-    double d;
-    if (MODEL == MODEL_BASIS && J.gmat) {
-      // stored basis: one sum over exact FP64 coefficient differences
-      d = 0.0;
-      const int s0 = J.shell_off[at.atom], s1 = J.shell_off[at.atom + 1];
-      for (int s = s0; s < s1; ++s)
-        d += (J.propars[s] - J.propars_old[s]) * J.gmat[(size_t)s * J.npoint + p];
-    } else {
-      d = (double)proatom<T, MODEL>(J, at.atom, J.propars, r, p) -
-          (double)proatom<T, MODEL>(J, at.atom, J.propars_old, r, p);
-    }
+    const double d = (double)proatom<T, MODEL>(J, at.atom, J.propars, r, p) -
+                     (double)proatom<T, MODEL>(J, at.atom, J.propars_old, r, p);
     acc += J.w[p] * d * d;
   }
   const double s = block_sum1(acc, red);
@@ -580,6 +574,7 @@ __global__ void __launch_bounds__(kThreads) k_basis_qvec(Batch bt) {
   const JobDev* Jp;
   const AtomTile at = decode_atom_tile(bt, Jp);
   const JobDev& J = *Jp;
+  if (J.gmat) return;  // k_gisa_moments64
   const int s0 = J.shell_off[at.atom];
   const int nsh = J.shell_off[at.atom + 1] - s0;
   double acc[kMaxShells];
@@ -787,7 +782,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_lisa_sc_inner(Batch bt) {
   const JobDev* Jp;
   const AtomTile at = decode_atom_tile(bt, Jp);
   const JobDev& J = *Jp;
-  if (!J.active[at.atom]) return;
+  if (J.gmat || !J.active[at.atom]) return;  // gmat: k_lisa_sc64
   const int s0 = J.shell_off[at.atom];
   const int nsh = J.shell_off[at.atom + 1] - s0;
   const double* pc = J.cur + J.par_off[at.atom];
@@ -1121,33 +1116,6 @@ __global__ void k_lisa_ls_pick(Batch bt) {
 // ---------------------------------------------------------------------------
 // gLISA (glisa.py)
 // ---------------------------------------------------------------------------
-
-// G[m][p] = unit-population basis function m at point p (gisa.py:91-106 with
-// force_on_molgrid=True).
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_glisa_basis(Batch bt) {
-  int tile;
-  const JobDev& J = decode_local(bt, tile);
-  // jobs that recompute their shells keep no basis matrix; float-float planes
-  // without an FP64 copy are written by k_glisa_basis_ff
-  if (!J.gmat) return;
-  for (int i = 0; i < J.ppt; ++i) {
-    const int p = point_of(J, tile, i);
-    if (p >= J.npoint) continue;
-    for (int a = 0; a < J.natom; ++a) {
-      const T r = Dist<T>::r(J, p, a);
-      for (int s = J.shell_off[a]; s < J.shell_off[a + 1]; ++s) {
-        const double g = (double)shell_value<T>(J, s, r);
-        const size_t e = (size_t)s * J.npoint + p;
-        if (J.gmat) J.gmat[e] = g;
-        if (J.gmat32) {
-          const float hi = (float)g;
-          J.gmat32[e] = hi;
-        }
-      }
-    }
-  }
-}
 
 // rho0 = G^T c (glisa.py:346-348); d1 = w rho/rho0, d2 = w rho/rho0^2 (0 where
 // sick); entropy and negativity partials (glisa.py:441-450, 784).
@@ -2377,31 +2345,6 @@ __global__ void k_glisa_apply(Batch bt, int mode) {
   }
 }
 
-// Change from stored basis values (glisa.py:776 via compute_change).
-__global__ void __launch_bounds__(kThreads) k_glisa_change(Batch bt) {
-  __shared__ double red[kWarps];
-  const JobDev* Jp;
-  const AtomTile at = decode_atom_tile(bt, Jp);
-  const JobDev& J = *Jp;
-  if (glisa_idle(J)) return;
-  const int s0 = J.shell_off[at.atom], s1 = J.shell_off[at.atom + 1];
-  double acc = 0.0;
-  for (int i = 0; i < J.ppt; ++i) {
-    const int p = point_of(J, at.tile, i);
-    if (p >= J.npoint) continue;
-    double r1 = 0.0, r2 = 0.0;
-    for (int m = s0; m < s1; ++m) {
-      const double g = J.gmat[(size_t)m * J.npoint + p];
-      r1 += J.propars[m] * g;
-      r2 += J.propars_old[m] * g;
-    }
-    const double d = r1 - r2;
-    acc += J.w[p] * d * d;
-  }
-  const double s = block_sum1(acc, red);
-  if (threadIdx.x == 0) apart_ptr(J, at.atom, QA_CHANGE)[at.tile] = s;
-}
-
 // gLISA convergence bookkeeping: negativity of the promolecule used in the
 // last iteration and the population check (glisa.py:786-798).
 __global__ void k_glisa_check(Batch bt) {
@@ -2686,14 +2629,18 @@ void launch_copy_old(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_copy_ol
 
 // FP32 variants live in hp_mixed.cu, float-float (MBIS) in hp_ff.cu; `mixed`
 // is the job group's evaluation phase (Phase).
-// weights false: without the at_weights pass (FP64 MBIS on atom grids).
+// weights false: without the at_weights pass (FP64 on atom grids; GISA jobs
+// with a stored G).
 void launch_promol(const HostBatch& hb, cudaStream_t st, int mixed, int model, bool weights) {
   if (mixed == PH_FF && model == MODEL_MBIS) return launch_promol_ff(hb, st);
   if (mixed) return launch_promol_mx(hb, st, model);
   if (model == MODEL_MBIS) return launch_promol64(hb, st, weights);
   if (model == MODEL_NLIS) HP_LAUNCH((k_promol<double, MODEL_NLIS>), K_POINT1, kThreads);
-  else HP_LAUNCH((k_promol<double, MODEL_BASIS>), K_POINT1, kThreads);
-  HP_LAUNCH(k_atweights, K_ATOM_TILE, kThreads);
+  else {
+    if (hb.any_g) launch_promol_g64(hb, st);
+    if (hb.any_nog) HP_LAUNCH((k_promol<double, MODEL_BASIS>), K_POINT1, kThreads);
+  }
+  if (weights) HP_LAUNCH(k_atweights, K_ATOM_TILE, kThreads);
 }
 
 void launch_gisa_qp(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_gisa_qp, K_ATOM, 32); }
@@ -2716,7 +2663,10 @@ void launch_change(const HostBatch& hb, cudaStream_t st, int mixed, int model) {
   if (mixed) return launch_change_mx(hb, st, model);
   if (model == MODEL_MBIS) return launch_change64(hb, st);
   if (model == MODEL_NLIS) HP_LAUNCH((k_change<double, MODEL_NLIS>), K_ATOM_TILE, kThreads);
-  else HP_LAUNCH((k_change<double, MODEL_BASIS>), K_ATOM_TILE, kThreads);
+  else {
+    if (hb.any_g) launch_change_g64(hb, st);
+    if (hb.any_nog) HP_LAUNCH((k_change<double, MODEL_BASIS>), K_ATOM_TILE, kThreads);
+  }
 }
 
 void launch_outer_finish(const HostBatch& hb, cudaStream_t st, int with_charges) {
@@ -2742,14 +2692,25 @@ void launch_nlis_inner(const HostBatch& hb, cudaStream_t st) {
 }
 
 void launch_gisa(const HostBatch& hb, cudaStream_t st, int mixed) {
-  if (mixed) launch_basis_qvec_mx(hb, st);
-  else HP_LAUNCH(k_basis_qvec<double>, K_ATOM_TILE, kThreads);
+  if (mixed) {
+    launch_basis_qvec_mx(hb, st);
+  } else {
+    if (hb.any_g) {
+      launch_entropy64(hb, st);
+      launch_gisa_moments64(hb, st);
+    }
+    if (hb.any_nog) HP_LAUNCH(k_basis_qvec<double>, K_ATOM_TILE, kThreads);
+  }
   HP_LAUNCH(k_gisa_qp, K_ATOM, 32);
 }
 
 void launch_lisa_sc_inner(const HostBatch& hb, cudaStream_t st, int mixed) {
-  if (mixed) launch_lisa_sc_inner_mx(hb, st);
-  else launch_inner_kernel(k_lisa_sc_inner<double>, hb, K_ATOM_TILE, st);
+  if (mixed) {
+    launch_lisa_sc_inner_mx(hb, st);
+  } else {
+    if (hb.any_g) launch_lisa_sc64(hb, st);
+    if (hb.any_nog) launch_inner_kernel(k_lisa_sc_inner<double>, hb, K_ATOM_TILE, st);
+  }
 }
 
 // Newton keeps FP64 evaluation (its Hessian needs it); mixed jobs are
@@ -2762,10 +2723,6 @@ void launch_lisa_newton_inner(const HostBatch& hb, cudaStream_t st, int mixed, i
     HP_LAUNCH(k_lisa_ls<double>, K_ATOM_TILE, kThreads);
     HP_LAUNCH(k_lisa_ls_pick, K_ATOM, 32);
   }
-}
-
-void launch_glisa_basis(const HostBatch& hb, cudaStream_t st) {
-  HP_LAUNCH(k_glisa_basis<double>, K_POINT, kThreads);
 }
 
 void launch_glisa_pro(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_glisa_pro, K_POINT, kThreads); }
@@ -2834,9 +2791,7 @@ void launch_glisa_ls(const HostBatch& hb, cudaStream_t st, int first, int count)
   HP_LAUNCH(k_glisa_ls_pick, K_JOB, 32, first, count);
 }
 
-void launch_glisa_change(const HostBatch& hb, cudaStream_t st) {
-  HP_LAUNCH(k_glisa_change, K_ATOM_TILE, kThreads);
-}
+void launch_glisa_change(const HostBatch& hb, cudaStream_t st) { launch_change_g64(hb, st); }
 
 void launch_glisa_check(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_glisa_check, K_JOB, 32); }
 

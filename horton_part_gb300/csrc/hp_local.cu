@@ -100,11 +100,13 @@ __global__ void __launch_bounds__(kThreads) k_sph_avg64(Batch bt) {
   }
 }
 
-// The entropy partials of k_atweights, one block per point tile.
+// The entropy partials of k_atweights, one block per point tile (atom grids,
+// and GISA jobs with a stored G).
 __global__ void __launch_bounds__(kThreads) k_entropy64(Batch bt) {
   __shared__ double red[kThreads];
   int tile;
   const JobDev& J = decode_atom_lc(bt, tile);  // (the block's index within its job)
+  if (!J.local && !J.gmat) return;
   double acc[1] = {0.0};
   const int p1 = min((tile + 1) * J.tile_points, J.npoint);
   for (int p = tile * J.tile_points + threadIdx.x; p < p1; p += kThreads) {
@@ -480,16 +482,26 @@ __global__ void __launch_bounds__(kThreads) k_lisa_sc_radial(Batch bt) {
     }                                                                                  \
   } while (0)
 
-// at_weights on the atoms' own points with the spherical averages (FP64: the
-// promolecule pass alone came before), then the radial solves.
-void launch_mbis_local(const HostBatch& hb, cudaStream_t st, int mixed) {
+void launch_entropy64(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH_LC(k_entropy64, K_POINT, kThreads); }
+
+namespace {
+
+// Spherical averages of the AIM densities; FP64 jobs form the at_weights
+// there, on the atoms' own points (only the promolecule pass came before).
+void launch_averages(const HostBatch& hb, cudaStream_t st, int mixed) {
   if (mixed) {
     HP_LAUNCH_LC(k_sph_avg, K_ATOM, kThreads);
-  } else {
-    HP_LAUNCH_LC(k_entropy64, K_POINT, kThreads);
-    k_sph_avg64<<<hb.blocks[K_ATOM] * kAvgSplit, kThreads, 0, st>>>(hb.b[K_ATOM]);
-    ++g_launch_count;
+    return;
   }
+  launch_entropy64(hb, st);
+  k_sph_avg64<<<hb.blocks[K_ATOM] * kAvgSplit, kThreads, 0, st>>>(hb.b[K_ATOM]);
+  ++g_launch_count;
+}
+
+}  // namespace
+
+void launch_mbis_local(const HostBatch& hb, cudaStream_t st, int mixed) {
+  launch_averages(hb, st, mixed);
   HP_LAUNCH_LC(k_mbis_radial, K_ATOM, kThreads);
 }
 
@@ -498,17 +510,17 @@ void launch_change_radial(const HostBatch& hb, cudaStream_t st) {
 }
 
 void launch_nlis_local(const HostBatch& hb, cudaStream_t st) {
-  HP_LAUNCH_LC(k_sph_avg, K_ATOM, kThreads);
+  launch_averages(hb, st, 0);
   HP_LAUNCH_LC(k_nlis_radial, K_ATOM, kThreads);
 }
 
-void launch_gisa_local(const HostBatch& hb, cudaStream_t st) {
-  HP_LAUNCH_LC(k_sph_avg, K_ATOM, kThreads);
+void launch_gisa_local(const HostBatch& hb, cudaStream_t st, int mixed) {
+  launch_averages(hb, st, mixed);
   HP_LAUNCH_LC(k_basis_radial_qvec, K_ATOM, kThreads);
 }
 
-void launch_lisa_sc_local(const HostBatch& hb, cudaStream_t st) {
-  HP_LAUNCH_LC(k_sph_avg, K_ATOM, kThreads);
+void launch_lisa_sc_local(const HostBatch& hb, cudaStream_t st, int mixed) {
+  launch_averages(hb, st, mixed);
   HP_LAUNCH_LC(k_lisa_sc_radial, K_ATOM, kThreads);
 }
 

@@ -200,7 +200,7 @@ __device__ __forceinline__ double* inner_partials(const JobDev& J, int a, int pa
 // distance, the old pro-atom's exponentials, CUDA's exp and divide and the
 // sums of seven shells were all formed per pair. Two outer iterations of a
 // 22-atom chain of 320k points: 116.7 -> 32.6 ms.
-__global__ void __launch_bounds__(kThreads) k_mbis_inner64(Batch bt) {
+__global__ void __launch_bounds__(kThreads, 3) k_mbis_inner64(Batch bt) {
   __shared__ double tab[f64::kExpTab];
   __shared__ double red[kQ * kThreads];
   __shared__ int skip_s;

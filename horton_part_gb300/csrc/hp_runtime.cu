@@ -123,7 +123,7 @@ struct hp_job {
   int64_t g_active = -1; // fused gLISA: G values in the tiles' active rows (-1: not read yet)
   double skipped = 0.0;  // point-atom evaluations skipped by the per-atom cutoff
   bool host_driven = false;  // finished by hp_glisa_finish (histories kept by the host)
-  // FP64 MBIS: the stored distances and pro-atoms (JobDev::rd, oldpro,
+  // FP64 jobs: the stored distances and pro-atoms (JobDev::rd, oldpro,
   // oldok), given back when another allocation needs the room (make_room)
   void* keep_mem = nullptr;
   size_t keep_bytes = 0;
@@ -166,14 +166,17 @@ cudaError_t job_alloc_retry(hp_ctx* ctx, void** p, size_t bytes) {
   return job_alloc(ctx, p, bytes);
 }
 
-// FP64 MBIS: storage for the pair distances and, on the molecular grid, the
-// pro-atoms of the last inner iteration, where it takes at most half of what
-// is left of the budget.
+// FP64 jobs: storage for the pair distances (MBIS) and, on the molecular
+// grid, the pro-atoms of the last inner iteration (MBIS, aLISA sc with a
+// stored G), where it takes at most half of what is left of the budget.
 void alloc_kept(hp_ctx* ctx, hp_job* j) {
   JobDev& J = j->dev;
-  if (J.scheme != SCHEME_MBIS || J.mixed) return;
+  const bool mbis = J.scheme == SCHEME_MBIS && !J.mixed;
+  const bool lisa = J.scheme == SCHEME_LISA && J.solver == SOLVER_SC && J.gmat && !J.local;
+  if (!mbis && !lisa) return;
+  const bool old = !J.local;
   const size_t pair = align_up(8 * (size_t)J.natom * (size_t)J.npoint);
-  const size_t bytes = J.local ? pair : 2 * pair + align_up(4 * (size_t)J.natom * J.ntile);
+  const size_t bytes = (mbis ? pair : 0) + (old ? pair + align_up(4 * (size_t)J.natom * J.ntile) : 0);
   const size_t room = ctx->budget > ctx->used ? ctx->budget - ctx->used : 0;
   if (bytes > room / 2) return;
   void* mem = nullptr;
@@ -186,10 +189,14 @@ void alloc_kept(hp_ctx* ctx, hp_job* j) {
   j->bytes += bytes;
   ctx->used += bytes;
   ctx->kept += bytes;
-  J.rd = reinterpret_cast<double*>(mem);
-  if (!J.local) {
-    J.oldpro = reinterpret_cast<double*>((char*)mem + pair);
-    J.oldok = reinterpret_cast<int*>((char*)mem + 2 * pair);
+  char* at = (char*)mem;
+  if (mbis) {
+    J.rd = reinterpret_cast<double*>(at);
+    at += pair;
+  }
+  if (old) {
+    J.oldpro = reinterpret_cast<double*>(at);
+    J.oldok = reinterpret_cast<int*>(at + pair);
   }
 }
 
@@ -307,6 +314,8 @@ int build_batch(hp_ctx* ctx, const std::vector<hp_job*>& jobs, HostBatch& hb) {
   const int n = (int)jobs.size();
   hb.nact_max = 0;
   hb.solve_tiles = solve_tiles(jobs);
+  hb.any_g = hb.any_nog = false;
+  for (const hp_job* j : jobs) (j->dev.gmat ? hb.any_g : hb.any_nog) = true;
   for (int j = 0; j < n; ++j) {
     ctx->batch_host[j] = jobs[j]->dev;
     hb.nact_max = std::max(hb.nact_max, jobs[j]->dev.nact_max);
@@ -513,7 +522,7 @@ int job_init(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatch& hb)
   if (any_geo) launch_tile_rmin(hb, ctx->stream);
   if (any_rd) launch_rdist64(hb, ctx->stream);
   if (any_rdist) launch_rdist_ff(hb, ctx->stream);
-  if (any_basis) launch_glisa_basis(hb, ctx->stream);
+  if (any_basis) launch_basis64(hb, ctx->stream);
   if (any_basis_ff) launch_glisa_basis_ff(hb, ctx->stream);
   int fuse_shells = 0;
   for (hp_job* j : jobs)
@@ -552,7 +561,9 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
   launch_copy_old(hb, st);
   {
     ProfScope ps(ctx, HP_KERNEL_PROMOL);
-    launch_promol(hb, st, mixed, model, !(local && model == MODEL_MBIS && !mixed));
+    // FP64 on atom grids, and GISA with a stored G: at_weights in their own passes
+    const bool own = !mixed && (local || (j0->desc.scheme == HP_SCHEME_GISA && !hb.any_nog));
+    launch_promol(hb, st, mixed, model, !own);
   }
   int rc = HP_OK;
   switch (j0->desc.scheme) {
@@ -587,7 +598,7 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
     case HP_SCHEME_GISA: {
       ProfScope ps(ctx, HP_KERNEL_INNER);
       if (local) {  // moments on the radial grids, the same quadratic program
-        launch_gisa_local(hb, st);
+        launch_gisa_local(hb, st, mixed);
         launch_gisa_qp(hb, st);
       } else {
         launch_gisa(hb, st, mixed);
@@ -598,7 +609,7 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
       if (local) {  // atom grids: every inner iteration of every atom in one launch
         ProfScope ps(ctx, HP_KERNEL_INNER);
         launch_inner_init(hb, st);
-        launch_lisa_sc_local(hb, st);
+        launch_lisa_sc_local(hb, st, mixed);
       } else if (j0->dev.solver == SOLVER_SC)
         rc = run_inner(ctx, jobs, hb, [&] {
           ProfScope ps(ctx, HP_KERNEL_INNER);
@@ -1256,7 +1267,9 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   const size_t gbytes = 8 * (size_t)S * N;
   const size_t firm = ctx->used - ctx->kept;
   const size_t room = ctx->budget > firm ? ctx->budget - firm : 0;
-  if (!glisa && !mbis && !nlis && !mixed && gbytes <= room / 2) add(&J.gmat, gbytes);
+  const bool gstore = !glisa && !mbis && !nlis && !mixed && gbytes <= room / 2;
+  if (gstore) add(&J.gmat, gbytes);
+  if (gstore || (glisa && !gff)) add(&J.smask, 4 * (size_t)A * ntile);
   if (glisa) {
     if (!gff) add(&J.gmat, 8 * (size_t)S * N);
     add(&J.gpart, 8 * (size_t)S * ntile);
