@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(kThreads) k_basis64(Batch bt) {
 
 // Pro-atoms and promolecule (core/stockholder.py:153-175), one thread per
 // point; a block's 256 points lie in one tile, so its masks are uniform. The
-// rows of an atom go four at a time, their loads together. The reference adds
+// rows of an atom go two at a time, their loads together (four or eight: 1.5
+// and 4 % more of the GISA job, FP64 work on padding). The reference adds
 // 1e-100 per atom: a sum of 1e-80 or more does not change by it, and the
 // addition is left out there.
 __global__ void __launch_bounds__(kThreads) k_promol_g64(Batch bt) {
@@ -128,18 +129,19 @@ __global__ void __launch_bounds__(kThreads) k_promol_g64(Batch bt) {
     const double* __restrict__ g0 = G + s0 * N + p;
     double pro = 0.0;
     while (mask) {
-      int k[4];
-      double c[4], g[4];
+      constexpr int kU = 2;
+      int k[kU];
+      double c[kU], g[kU];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < kU; ++u) {
         k[u] = mask ? __ffs((int)mask) - 1 : k[u > 0 ? u - 1 : 0];
         c[u] = mask ? par[s0 + k[u]] : 0.0;
         mask &= mask - 1;
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) g[u] = g0[k[u] * N];
+      for (int u = 0; u < kU; ++u) g[u] = g0[k[u] * N];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) pro = __fma_rn(c[u], g[u], pro);
+      for (int u = 0; u < kU; ++u) pro = __fma_rn(c[u], g[u], pro);
     }
     J.rhoa[a * N + p] = pro;
     promol += pro;
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(kThreads) k_promol_g64(Batch bt) {
 // GISA moments (gisa.py:257-279): at_weights, population sum w rho_a and
 // q-vector sums sum w g_k rho_a of one (atom, tile), from the pro-atoms of
 // k_promol_g64 (rhoa is not written back: GISA reads it nowhere else).
-__global__ void __launch_bounds__(kThreads, 2) k_gisa_moments64(Batch bt) {
+__global__ void __launch_bounds__(kThreads, 3) k_gisa_moments64(Batch bt) {
   __shared__ double red[(kMaxShells + 1) * kThreads];
   int a, tile;
   const JobDev& J = decode_at_bs(bt, a, tile);
@@ -193,7 +195,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_gisa_moments64(Batch bt) {
 
 // aLISA self-consistent iteration (alisa.py:193-291), one (atom, tile): the
 // moments sum w c_k g_k rho_a / pro and the change sum w (oldpro - pro)^2.
-__global__ void __launch_bounds__(kThreads, 2) k_lisa_sc64(Batch bt) {
+__global__ void __launch_bounds__(kThreads, 3) k_lisa_sc64(Batch bt) {
   constexpr int Q = kMaxShells + 1;
   __shared__ double red[Q * kThreads];
   __shared__ double tab[f64::kExpTab];
@@ -280,7 +282,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_lisa_sc64(Batch bt) {
 }
 
 // Outer change sum w (sum_k (c - c_old)_k g_k)^2 (core/iterstock.py:32-45).
-__global__ void __launch_bounds__(kThreads, 2) k_change_g64(Batch bt) {
+__global__ void __launch_bounds__(kThreads, 3) k_change_g64(Batch bt) {
   __shared__ double red[kThreads];
   __shared__ double tab[f64::kExpTab];
   __shared__ double c[kMaxShells];

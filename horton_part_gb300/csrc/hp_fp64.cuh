@@ -154,4 +154,22 @@ __device__ __forceinline__ void block_sums(const double (&acc)[Q], int nq, doubl
 }
 
 }  // namespace f64
+
+// One tile of the entropy integral sum w rho ln(rho / promol)
+// (core/stockholder.py:145-151) into jpart, for jobs whose at_weights are not
+// formed by k_atweights (atom grids, a stored G). red: kThreads doubles.
+__device__ __forceinline__ void entropy_tile(const JobDev& J, int tile, double* red) {
+  if (!J.local && !J.gmat) return;
+  double acc[1] = {0.0};
+  const int p1 = min((tile + 1) * J.tile_points, J.npoint);
+  for (int p = tile * J.tile_points + threadIdx.x; p < p1; p += kThreads) {
+    const double promol = J.promol[p], rho = J.rho[p];
+    if (!((promol < J.density_cutoff) || (rho < J.density_cutoff)))
+      acc[0] += J.w[p] * rho * log(rho / promol);
+  }
+  f64::block_sums<1>(acc, 1, red, [&](int, double v) {
+    J.jpart[(size_t)QJ_ENTROPY * J.ntile + tile] = v;
+  });
+}
+
 }  // namespace hp

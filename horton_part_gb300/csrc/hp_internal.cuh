@@ -647,7 +647,8 @@ void launch_mbis_local(const HostBatch& hb, cudaStream_t st, int mixed);
 void launch_change_radial(const HostBatch& hb, cudaStream_t st);
 void launch_gisa_local(const HostBatch& hb, cudaStream_t st, int mixed);     // spherical averages + radial moments
 void launch_lisa_sc_local(const HostBatch& hb, cudaStream_t st, int mixed);  // spherical averages + radial sc solve
-void launch_gisa_qp(const HostBatch& hb, cudaStream_t st);        // k_gisa_qp alone
+// k_gisa_qp; entropy: with the entropy tiles of the jobs that store G
+void launch_gisa_qp(const HostBatch& hb, cudaStream_t st, bool entropy = false);
 
 // FP64 MBIS (hp_mbis.cu)
 void launch_rdist64(const HostBatch& hb, cudaStream_t st);  // rd of the batch's jobs
@@ -664,7 +665,6 @@ void launch_promol_g64(const HostBatch& hb, cudaStream_t st);
 void launch_gisa_moments64(const HostBatch& hb, cudaStream_t st);  // at_weights and q-vector moments
 void launch_lisa_sc64(const HostBatch& hb, cudaStream_t st);
 void launch_change_g64(const HostBatch& hb, cudaStream_t st);
-void launch_entropy64(const HostBatch& hb, cudaStream_t st);       // entropy partials (hp_local.cu)
 
 // float-float MBIS (hp_ff.cu)
 void launch_promol_ff(const HostBatch& hb, cudaStream_t st);

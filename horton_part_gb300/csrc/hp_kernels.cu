@@ -622,7 +622,7 @@ __device__ __forceinline__ int warp_argmin_d(double v, double& vmin) {
   return idx;
 }
 
-// One warp per atom: the GISA quadratic program (gisa.py:348-421)
+// The GISA quadratic program of one atom (gisa.py:348-421)
 //   min 1/2 x^T P x + q^T x,  x >= 0,  sum x = int w rho_a,
 // P precomputed per atom (twice the Gaussian overlap), q_k = -2 int w g_k rho_a.
 // Exact primal active-set method (Nocedal & Wright, Algorithm 16.3) started at
@@ -630,22 +630,39 @@ __device__ __forceinline__ int warp_argmin_d(double v, double& vmin) {
 // owns variable k; the equality-constrained step on the free set solves
 // P_FF u = -g_F and P_FF v = 1 with one Cholesky factor, lambda = sum u / sum v,
 // p = u - lambda v.
-__global__ void k_gisa_qp(Batch bt) {
+//
+// A block of kThreads threads per atom: its warps sum the tile partials, then
+// warp 0 solves. The solve is one long chain of dependent FP64 operations, so
+// divisions are few (a reciprocal per pivot). Behind the atoms' blocks the
+// same launch carries the entropy tiles of jobs with a stored G (pt), whose
+// logarithms take the FP64 pipes that the solves leave idle.
+__global__ void __launch_bounds__(kThreads) k_gisa_qp(Batch bt, int nqp, Batch pt) {
   __shared__ double Ps[kMaxShells][kMaxShells + 1];
   __shared__ double M[kMaxShells][kMaxShells + 1];
   __shared__ double rhs[2][kMaxShells];
+  __shared__ double dinv[kMaxShells];
+  __shared__ double qsum[kMaxShells + 1];
+  __shared__ double red[kThreads];
   __shared__ int bad;
+  if ((int)blockIdx.x >= nqp) {
+    const int b = blockIdx.x - nqp;
+    const int j = find_job(pt, b);
+    entropy_tile(pt.jobs[j], b - pt.prefix[j], red);
+    return;
+  }
   int a;
   const JobDev& J = decode_local(bt, a);
   const int lane = threadIdx.x & 31;
   const int s0 = J.shell_off[a];
   const int n = J.shell_off[a + 1] - s0;
-  double qi = 0.0;
-  for (int k = 0; k < n; ++k) {
-    const double v = -2.0 * warp_tile_sum(J, apart_ptr(J, a, QA_INNER + k), J.ntile);
-    if (lane == k) qi = v;
+  for (int k = threadIdx.x >> 5; k <= n; k += kWarps) {
+    const double v = warp_tile_sum(J, apart_ptr(J, a, k < n ? QA_INNER + k : (int)QA_POP), J.ntile);
+    if (lane == 0) qsum[k] = v;
   }
-  const double pop = warp_tile_sum(J, apart_ptr(J, a, QA_POP), J.ntile);
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const double qi = lane < n ? -2.0 * qsum[lane] : 0.0;
+  const double pop = qsum[n];
   const double* P = J.qp_p + J.qp_off[a];
   for (int e = lane; e < n * n; e += 32) Ps[e / n][e % n] = P[e];
   if (lane == 0) bad = 0;
@@ -707,9 +724,10 @@ __global__ void k_gisa_qp(Batch bt) {
         const double d = M[k][k];
         if (!(d > 0.0)) bad = 1;
         M[k][k] = sqrt(fmax(d, 1e-300));
+        dinv[k] = 1.0 / M[k][k];
       }
       __syncwarp();
-      if (lane > k && lane < nf) M[lane][k] /= M[k][k];
+      if (lane > k && lane < nf) M[lane][k] *= dinv[k];
       __syncwarp();
       if (lane > k && lane < nf)
         for (int j = k + 1; j <= lane; ++j) M[lane][j] -= M[lane][k] * M[j][k];
@@ -725,12 +743,12 @@ __global__ void k_gisa_qp(Batch bt) {
       for (int i = 0; i < nf; ++i) {
         double v = b[i];
         for (int j = 0; j < i; ++j) v -= M[i][j] * b[j];
-        b[i] = v / M[i][i];
+        b[i] = v * dinv[i];
       }
       for (int i = nf - 1; i >= 0; --i) {
         double v = b[i];
         for (int j = i + 1; j < nf; ++j) v -= M[j][i] * b[j];
-        b[i] = v / M[i][i];
+        b[i] = v * dinv[i];
       }
     }
     __syncwarp();
@@ -2643,7 +2661,12 @@ void launch_promol(const HostBatch& hb, cudaStream_t st, int mixed, int model, b
   if (weights) HP_LAUNCH(k_atweights, K_ATOM_TILE, kThreads);
 }
 
-void launch_gisa_qp(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_gisa_qp, K_ATOM, 32); }
+void launch_gisa_qp(const HostBatch& hb, cudaStream_t st, bool entropy) {
+  if (hb.blocks[K_ATOM] <= 0) return;
+  const int nqp = hb.blocks[K_ATOM], nent = entropy ? hb.blocks[K_POINT] : 0;
+  k_gisa_qp<<<nqp + nent, kThreads, 0, st>>>(hb.b[K_ATOM], nqp, hb.b[K_POINT]);
+  ++g_launch_count;
+}
 
 void launch_atweights(const HostBatch& hb, cudaStream_t st) {
   HP_LAUNCH(k_atweights, K_ATOM_TILE, kThreads);
@@ -2695,13 +2718,10 @@ void launch_gisa(const HostBatch& hb, cudaStream_t st, int mixed) {
   if (mixed) {
     launch_basis_qvec_mx(hb, st);
   } else {
-    if (hb.any_g) {
-      launch_entropy64(hb, st);
-      launch_gisa_moments64(hb, st);
-    }
+    if (hb.any_g) launch_gisa_moments64(hb, st);
     if (hb.any_nog) HP_LAUNCH(k_basis_qvec<double>, K_ATOM_TILE, kThreads);
   }
-  HP_LAUNCH(k_gisa_qp, K_ATOM, 32);
+  launch_gisa_qp(hb, st, !mixed && hb.any_g);
 }
 
 void launch_lisa_sc_inner(const HostBatch& hb, cudaStream_t st, int mixed) {

@@ -100,23 +100,12 @@ __global__ void __launch_bounds__(kThreads) k_sph_avg64(Batch bt) {
   }
 }
 
-// The entropy partials of k_atweights, one block per point tile (atom grids,
-// and GISA jobs with a stored G).
+// The entropy partials of k_atweights, one block per point tile.
 __global__ void __launch_bounds__(kThreads) k_entropy64(Batch bt) {
   __shared__ double red[kThreads];
   int tile;
   const JobDev& J = decode_atom_lc(bt, tile);  // (the block's index within its job)
-  if (!J.local && !J.gmat) return;
-  double acc[1] = {0.0};
-  const int p1 = min((tile + 1) * J.tile_points, J.npoint);
-  for (int p = tile * J.tile_points + threadIdx.x; p < p1; p += kThreads) {
-    const double promol = J.promol[p], rho = J.rho[p];
-    if (!((promol < J.density_cutoff) || (rho < J.density_cutoff)))
-      acc[0] += J.w[p] * rho * log(rho / promol);
-  }
-  f64::block_sums<1>(acc, 1, red, [&](int, double v) {
-    J.jpart[(size_t)QJ_ENTROPY * J.ntile + tile] = v;
-  });
+  entropy_tile(J, tile, red);
 }
 
 // Inner MBIS fixed point of every atom on its radial grid (one block per
@@ -482,8 +471,6 @@ __global__ void __launch_bounds__(kThreads) k_lisa_sc_radial(Batch bt) {
     }                                                                                  \
   } while (0)
 
-void launch_entropy64(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH_LC(k_entropy64, K_POINT, kThreads); }
-
 namespace {
 
 // Spherical averages of the AIM densities; FP64 jobs form the at_weights
@@ -493,7 +480,7 @@ void launch_averages(const HostBatch& hb, cudaStream_t st, int mixed) {
     HP_LAUNCH_LC(k_sph_avg, K_ATOM, kThreads);
     return;
   }
-  launch_entropy64(hb, st);
+  HP_LAUNCH_LC(k_entropy64, K_POINT, kThreads);
   k_sph_avg64<<<hb.blocks[K_ATOM] * kAvgSplit, kThreads, 0, st>>>(hb.b[K_ATOM]);
   ++g_launch_count;
 }

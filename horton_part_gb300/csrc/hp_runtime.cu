@@ -59,7 +59,7 @@ struct hp_ctx {
   JobDev* batch_dev = nullptr;     // JobDev array of the current batch
   JobDev* batch_host = nullptr;    // pinned staging
   double* exp_tab = nullptr;       // 2^(j/512), j < 512 (JobDev::etab)
-  int* prefix_dev = nullptr;       // [K_NKIND][kMaxSlots + 1]
+  int* prefix_dev = nullptr;       // [K_NKIND][jobs of the batch + 1]
   int* prefix_host = nullptr;      // pinned staging
   // kernel timing (hp_ctx_profile)
   bool prof = false;
@@ -323,18 +323,17 @@ int build_batch(hp_ctx* ctx, const std::vector<hp_job*>& jobs, HostBatch& hb) {
   HP_CK(cudaMemcpyAsync(ctx->batch_dev, ctx->batch_host, sizeof(JobDev) * n,
                         cudaMemcpyHostToDevice, ctx->stream));
   for (int k = 0; k < K_NKIND; ++k) {
-    int* pre = ctx->prefix_host + (size_t)k * (kMaxSlots + 1);
+    int* pre = ctx->prefix_host + (size_t)k * (n + 1);
     pre[0] = 0;
     for (int j = 0; j < n; ++j)
       pre[j + 1] = pre[j] + (k == K_SOLVE ? solve_blocks(jobs[j]->dev, hb.solve_tiles) : blocks_for(jobs[j]->dev, k));
     hb.blocks[k] = pre[n];
     hb.b[k].jobs = ctx->batch_dev;
-    hb.b[k].prefix = ctx->prefix_dev + (size_t)k * (kMaxSlots + 1);
+    hb.b[k].prefix = ctx->prefix_dev + (size_t)k * (n + 1);
     hb.b[k].njobs = n;
   }
   HP_CK(cudaMemcpyAsync(ctx->prefix_dev, ctx->prefix_host,
-                        sizeof(int) * K_NKIND * (kMaxSlots + 1), cudaMemcpyHostToDevice,
-                        ctx->stream));
+                        sizeof(int) * K_NKIND * (n + 1), cudaMemcpyHostToDevice, ctx->stream));
   return HP_OK;
 }
 
