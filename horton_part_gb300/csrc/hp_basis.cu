@@ -11,6 +11,7 @@
 // exponents 0.05 to 300).
 #include <math.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "hp_inner.cuh"
@@ -336,6 +337,429 @@ __global__ void __launch_bounds__(kThreads, 3) k_change_g64(Batch bt) {
   f64::block_sums<1>(acc, 1, red, [&](int, double v) { *out = v; });
 }
 
+// The tile's active rows with their coefficients in shared memory, for the
+// passes that take every row at a point: eight rows' loads go together (with
+// the bit masks read per point two were in flight and the pass took 1.5
+// times as long). Zero weights pad the list to a multiple of eight.
+constexpr int kListRows = 1024;
+struct RowList {
+  double c[kListRows];
+  int row[kListRows];
+  int n;
+};
+
+__device__ __forceinline__ void load_rows(const JobDev& J, int tile, const double* vec, RowList* L) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int n = 0;
+    for (int a0 = 0; a0 < J.natom; a0 += 32) {
+      const int a = a0 + lane;
+      unsigned m = a < J.natom ? J.smask[(size_t)a * J.ntile + tile] : 0u;
+      const int mine = __popc(m);
+      int pos = mine;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, pos, o);
+        if (lane >= o) pos += x;
+      }
+      int at = n + pos - mine;
+      for (; m; m &= m - 1) L->row[at++] = J.shell_off[a] + __ffs((int)m) - 1;
+      n += __shfl_sync(0xffffffffu, pos, 31);
+    }
+    __syncwarp();
+    const int n8 = (n + 7) & ~7;
+    for (int i = n + lane; i < n8; i += 32) L->row[i] = n > 0 ? L->row[n - 1] : 0;
+    if (lane == 0) L->n = n;
+  }
+  __syncthreads();
+  const int n = L->n;
+  for (int i = threadIdx.x; i < ((n + 7) & ~7); i += blockDim.x) L->c[i] = i < n ? vec[L->row[i]] : 0.0;
+  __syncthreads();
+}
+
+// sum over the rows of the list of c G[row][p], even and odd rows in chains of
+// their own.
+__device__ __forceinline__ double dot_list(const JobDev& J, const RowList* L, int p) {
+  const size_t N = J.npoint;
+  const double* __restrict__ G = J.gmat + p;
+  double y0 = 0.0, y1 = 0.0;
+  for (int i = 0; i < L->n; i += 8) {
+    double g[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) g[u] = G[L->row[i + u] * N];
+#pragma unroll
+    for (int u = 0; u < 8; u += 2) {
+      y0 = __fma_rn(L->c[i + u], g[u], y0);
+      y1 = __fma_rn(L->c[i + u + 1], g[u + 1], y1);
+    }
+  }
+  return y0 + y1;
+}
+
+// The same without a list (jobs of more than kListRows shells).
+__device__ __forceinline__ double dot_rows(const JobDev& J, int tile, int p, const double* __restrict__ vec) {
+  const size_t N = J.npoint;
+  double y = 0.0;
+  for (int a = 0; a < J.natom; ++a) {
+    const int s0 = J.shell_off[a];
+    for (unsigned mask = J.smask[(size_t)a * J.ntile + tile]; mask; mask &= mask - 1) {
+      const int m = s0 + __ffs((int)mask) - 1;
+      y = __fma_rn(vec[m], J.gmat[m * N + p], y);
+    }
+  }
+  return y;
+}
+
+// rho0 = G^T c (glisa.py:346-348); d1 = w rho/rho0, d2 = w rho/rho0^2 (0 where
+// sick); entropy and negativity partials (glisa.py:441-450, 784).
+__global__ void __launch_bounds__(kThreads) k_glisa_pro(Batch bt) {
+  __shared__ double red[2 * kThreads];
+  __shared__ RowList rows;
+  int tile;
+  const JobDev& J = decode_local_bs(bt, tile);
+  if (glisa_idle(J)) return;
+  const bool list = J.nshell <= kListRows;
+  if (list) load_rows(J, tile, J.propars, &rows);
+  double acc[2] = {0.0, 0.0};
+  const int p1 = min((tile + 1) * J.tile_points, J.npoint);
+  for (int p = tile * J.tile_points + threadIdx.x; p < p1; p += kThreads) {
+    const double rho0 = list ? dot_list(J, &rows, p) : dot_rows(J, tile, p, J.propars);
+    const double rho = J.rho[p];
+    const double w = J.w[p];
+    const bool sick = (rho < J.density_cutoff) || (rho0 < J.density_cutoff);
+    const double inv = sick ? 0.0 : 1.0 / (sick ? 1.0 : rho0);
+    const double ratio = rho * inv;
+    const double d2 = w * ratio * inv;
+    J.dvec1[p] = w * ratio;
+    J.dvec2[p] = d2;
+    J.rho0[p] = rho0;
+    if (J.hess_s) J.hess_s[p] = sqrtf((float)d2);
+    if (!sick) acc[0] += w * rho * log(ratio);
+    if (rho0 < J.negative_cutoff) acc[1] += 1.0;
+  }
+  f64::block_sums<2>(acc, 2, red, [&](int q, double v) {
+    J.jpart[(size_t)(q == 0 ? QJ_ENTROPY : QJ_NEG) * J.ntile + tile] = v;
+  });
+}
+
+// gpart[m][tile] = sum_p G[m][p] v[p] with v = d1 (gradient) or v = hvec
+// (Hessian-vector product of the refinement); a warp per shell, zero where
+// the shell is inactive.
+__global__ void __launch_bounds__(kThreads) k_glisa_grad(Batch bt, int use_hvec) {
+  int tile;
+  const JobDev& J = decode_local_bs(bt, tile);
+  if (glisa_idle(J)) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int p0 = tile * J.tile_points;
+  const int p1 = min(p0 + J.tile_points, J.npoint);
+  const double* __restrict__ v = use_hvec ? J.hvec : J.dvec1;
+  int a = 0, s1 = J.shell_off[1];  // the atom of shell m (m grows)
+  for (int m = warp; m < J.nshell; m += kWarps) {
+    while (m >= s1) s1 = J.shell_off[++a + 1];
+    double s = 0.0;
+    if ((J.smask[(size_t)a * J.ntile + tile] >> (m - J.shell_off[a])) & 1u) {
+      const double* __restrict__ g = J.gmat + (size_t)m * J.npoint;
+#pragma unroll 8
+      for (int p = p0 + lane; p < p1; p += 32) s = __fma_rn(g[p], v[p], s);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    }
+    if (lane == 0) J.gpart[(size_t)m * J.ntile + tile] = s;
+  }
+}
+
+// Trial objective differences: tpart[t][tile] = this tile's part of
+// f(c_t) - f(c), f(c) = sum over healthy points of w rho ln(rho / rho0(c)).
+//   rho0_t = sum_m max(c_m + a_t delta_m, 0) g_m
+//          = rho0 + a_t (G^T delta) + sum_{m clipped at t} -(c_m + a_t delta_m) g_m,
+// one pass over G plus the few clipped shells. Where a point is healthy for
+// both, its term is -w rho log1p((rho0_t - rho0) / rho0): the relative change
+// is formed in FP64 and goes through the FP32 log1pf, which keeps each term
+// (and the difference the Armijo test compares) accurate to ~1e-7 of itself
+// without an FP64 log per trial; the few points whose sick status differs
+// between rho0 and rho0_t take FP64 logs. Sums in float-float per thread.
+__global__ void __launch_bounds__(kThreads) k_glisa_trials(Batch bt) {
+  __shared__ double red[2 * kTrials * kThreads];
+  __shared__ RowList rows;
+  int tile;
+  const JobDev& J = decode_local_bs(bt, tile);
+  if (glisa_idle(J)) return;
+  const bool list = J.nshell <= kListRows;
+  if (list) load_rows(J, tile, J.delta, &rows);
+  float ah[kTrials], al[kTrials], an[kTrials];
+#pragma unroll
+  for (int t = 0; t < kTrials; ++t) ah[t] = al[t] = an[t] = 0.0f;
+  const int nclip = J.clip[J.nshell];
+  const double cut = J.density_cutoff;
+  const int p1 = min((tile + 1) * J.tile_points, J.npoint);
+  for (int p = tile * J.tile_points + threadIdx.x; p < p1; p += kThreads) {
+    const double u = list ? dot_list(J, &rows, p) : dot_rows(J, tile, p, J.delta);
+    // corr_t = -sum_{m clipped at t} (c_m + 2^-t delta_m) g_m: the clipped
+    // sets shrink as t grows, so walk the list (sorted by t_m, largest first)
+    // once, keeping the running sums of c g and delta g
+    double corr[kTrials];
+    {
+      double sc = 0.0, sd = 0.0;
+      int k = 0;
+#pragma unroll
+      for (int t = kTrials - 1; t >= 0; --t) {
+        for (; k < nclip && J.clip[J.nshell + 1 + k] > t; ++k) {
+          const int m = J.clip[k];
+          const double g = J.gmat[(size_t)m * J.npoint + p];
+          sc = __fma_rn(J.propars[m], g, sc);
+          sd = __fma_rn(J.delta[m], g, sd);
+        }
+        corr[t] = -__fma_rn(ldexp(1.0, -t), sd, sc);
+      }
+    }
+    const double rho = J.rho[p], w = J.w[p], r0 = J.rho0[p];
+    const bool rs = rho < cut;
+    const bool h0 = !(rs || r0 < cut);
+    const double inv = h0 ? 1.0 / (h0 ? r0 : 1.0) : 0.0;
+    const float wr = (float)(w * rho);
+#pragma unroll
+    for (int t = 0; t < kTrials; ++t) {
+      const double dr = __fma_rn(ldexp(1.0, -t), u, corr[t]);
+      const double rt = r0 + dr;
+      const bool ht = !(rs || rt < cut);
+      float term = 0.0f;
+      if (h0 && ht) {
+        term = -wr * log1pf((float)(dr * inv));
+        an[t] += fabsf(term);
+      } else if (h0 || ht) {
+        const double big = ht ? w * rho * log(rho / rt) : -(w * rho * log(rho / r0));
+        const float bh = (float)big;
+        term = bh;
+        al[t] += (float)(big - (double)bh);
+      }
+      const float s = ah[t] + term;  // TwoSum into (ah, al)
+      const float bb = s - ah[t];
+      al[t] += (ah[t] - (s - bb)) + (term - bb);
+      ah[t] = s;
+    }
+  }
+  double acc[2 * kTrials];
+#pragma unroll
+  for (int t = 0; t < kTrials; ++t) {
+    acc[t] = (double)ah[t] + (double)al[t];
+    acc[kTrials + t] = (double)an[t];
+  }
+  f64::block_sums<2 * kTrials>(acc, 2 * kTrials, red,
+                               [&](int q, double v) { J.tpart[(size_t)q * J.ntile + tile] = v; });
+}
+
+// ---------------------------------------------------------------------------
+// gLISA Hessian H_ij = sum_p (w rho / rho0^2)(p) g_i(p) g_j(p) (glisa.py:457-470)
+//
+// FP64 FMAs on the lower triangle of the rows that are active on the tile:
+// sum over tiles of points x nact (nact + 1) / 2, about a third of the full
+// triangle (and a seventh of what padded 64 x 64 tiles of all rows issue).
+// Bound by the FP64 pipe.
+//
+// One persistent block per SM and partial (hsched: units of hunit points of
+// one tile, longest processing time first, ascending within a block). For a
+// tile the active rows are compacted and their triangle is cut into 4 x 4
+// register blocks dealt densely to the threads, so that no issue slot goes
+// to inactive rows; when they fill less than half of the warps, groups of
+// warps take the stage's points in turn (the FP64 pipes are per quarter of
+// the SM, so 4 or 6 busy warps leave some idle); consecutive units of a tile keep the accumulators, which
+// are added to the block's packed triangle in L2 when the tile changes (a
+// few instructions per element against hundreds of points). Points pass
+// through shared memory 16 at a time, rows scaled by w rho / rho0^2 beside
+// the plain ones, two buffers.
+//
+// 20-atom molecule (604,000 points, 150 shells): 30.4 -> 5.5 ms; 10 atoms, 66,000
+// points, 72 shells: 1520 -> 293 us.
+// ---------------------------------------------------------------------------
+constexpr int kH64Threads = 512;
+constexpr int kH64K = 16;  // points per stage
+constexpr int kH64Stage = kH64Rows * kH64K / kH64Threads;  // staged values per thread at most
+
+__device__ __forceinline__ void tri_of(int e, int& i, int& j) {
+  i = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+  while (i * (i + 1) / 2 > e) --i;
+  while ((i + 1) * (i + 2) / 2 <= e) ++i;
+  j = e - i * (i + 1) / 2;
+}
+
+__global__ void __launch_bounds__(kH64Threads, 1) k_glisa_hess64(Batch bt, int ld) {
+  extern __shared__ double hsm[];  // [2 buffers][plain, scaled][kH64K][ld]
+  __shared__ int row[kH64Rows];
+  __shared__ int nact_s;
+  int local;
+  const JobDev& J = decode_local_bs(bt, local);
+  if (!J.hsched || glisa_idle(J)) return;
+  const int S = J.nshell;
+  const size_t N = J.npoint;
+  double* H = J.hpart + (size_t)local * (S * (S + 1) / 2);
+  for (int e = threadIdx.x; e < S * (S + 1) / 2; e += kH64Threads) H[e] = 0.0;
+  const int* units = J.hsched + J.hbuf + 1;
+  const int upt = (J.tile_points + J.hunit - 1) / J.hunit;
+  const int plane = kH64K * ld;
+  double acc[2][16];
+  int tile = -1, nact = 0, nb = 0, base = 0;
+  int ngrp = 1, grp = 0;  // groups over the stage's points, this thread's one
+  int bi[2], bj[2];
+  auto flush = [&]() {
+    // the groups' sums onto group 0's, group by group through shared memory
+    // (the stage buffers are free: sweep ends at a barrier), then one read and
+    // write per element, the reads together
+    const int width = max(32, (nb + 31) & ~31);
+    for (int g = 1; g < ngrp; ++g) {
+      const int lane = (int)threadIdx.x - grp * width;
+      if (grp == g) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) hsm[q * width + lane] = acc[0][q];
+      }
+      __syncthreads();
+      if (grp == 0) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) acc[0][q] += hsm[q * width + lane];
+      }
+      __syncthreads();
+    }
+    if (grp != 0) return;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (bi[t] < 0) continue;
+      double h[16];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const int i = 4 * bi[t] + u, j = 4 * bj[t] + v;
+          h[4 * u + v] = i < nact && j <= i ? H[row[i] * (row[i] + 1) / 2 + row[j]] : 0.0;
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const int i = 4 * bi[t] + u, j = 4 * bj[t] + v;
+          if (i < nact && j <= i) H[row[i] * (row[i] + 1) / 2 + row[j]] = h[4 * u + v] + acc[t][4 * u + v];
+        }
+    }
+  };
+  auto assign = [&]() {  // this thread's 4 x 4 blocks of the pass that starts at block `base`
+    const int width = max(32, (nb + 31) & ~31);
+    ngrp = 1;
+    while (2 * ngrp * width <= kH64Threads && ngrp < 8) ngrp *= 2;
+    grp = ngrp > 1 ? (int)threadIdx.x / width : 0;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const int e = base + t * kH64Threads + (int)threadIdx.x - grp * width;
+      bi[t] = bj[t] = -1;
+      if (e < nb && grp < ngrp && (ngrp == 1 || t == 0)) tri_of(e, bi[t], bj[t]);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) acc[t][q] = 0.0;
+    }
+  };
+  // the points [q0, q1) of the current tile into the accumulators
+  auto sweep = [&](int q0, int q1) {
+    const int rows4 = (nact + 3) & ~3;
+    // thread: point sk of the stage, rows sr, sr + 32, ...
+    const int sk = threadIdx.x % kH64K, sr = threadIdx.x / kH64K;
+    double pre[kH64Stage], prd = 0.0;
+    auto fetch = [&](int q) {
+      const int p = q + sk;
+      prd = p < q1 ? J.dvec2[p] : 0.0;
+#pragma unroll
+      for (int c = 0; c < kH64Stage; ++c) {
+        const int r = sr + c * (kH64Threads / kH64K);
+        pre[c] = r < nact && p < q1 ? J.gmat[row[r] * N + p] : 0.0;
+      }
+    };
+    auto store = [&](int b) {
+      double* X = hsm + b * 2 * plane + sk * ld;
+#pragma unroll
+      for (int c = 0; c < kH64Stage; ++c) {
+        const int r = sr + c * (kH64Threads / kH64K);
+        if (r < rows4) {
+          X[r] = pre[c];
+          X[plane + r] = pre[c] * prd;
+        }
+      }
+    };
+    fetch(q0);
+    store(0);
+    __syncthreads();
+    int b = 0;
+    const bool two = nb - base > kH64Threads;
+    for (int q = q0; q < q1; q += kH64K) {
+      const bool more = q + kH64K < q1;
+      if (more) fetch(q + kH64K);
+      const double* X = hsm + b * 2 * plane;
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        if (t == 1 && !two) break;
+        if (bi[t] < 0) continue;
+        const double* xa = X + 4 * bi[t];
+        const double* xb = X + plane + 4 * bj[t];
+#pragma unroll 2
+        for (int k = grp; k < kH64K; k += ngrp) {
+          const double2 a0 = *reinterpret_cast<const double2*>(xa + k * ld);
+          const double2 a1 = *reinterpret_cast<const double2*>(xa + k * ld + 2);
+          const double2 b0 = *reinterpret_cast<const double2*>(xb + k * ld);
+          const double2 b1 = *reinterpret_cast<const double2*>(xb + k * ld + 2);
+          const double av[4] = {a0.x, a0.y, a1.x, a1.y}, bv[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) acc[t][4 * u + v] = __fma_rn(av[u], bv[v], acc[t][4 * u + v]);
+        }
+      }
+      if (more) store(b ^ 1);
+      __syncthreads();
+      b ^= 1;
+    }
+  };
+  for (int k = J.hsched[local]; k < J.hsched[local + 1]; ++k) {
+    const int u = units[k];
+    const int t = u / upt;
+    if (t != tile) {
+      if (tile >= 0 && nb <= 2 * kH64Threads) flush();
+      __syncthreads();  // row is read by flush; H by the block's other threads
+      tile = t;
+      if (threadIdx.x < 32) {  // compact the active rows, atom by atom
+        int n = 0;
+        for (int a0 = 0; a0 < J.natom; a0 += 32) {
+          const int a = a0 + threadIdx.x;
+          unsigned m = a < J.natom ? J.smask[(size_t)a * J.ntile + tile] : 0u;
+          int pos = __popc(m);
+          for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, pos, o);
+            if ((int)threadIdx.x >= o) pos += x;
+          }
+          const int total = __shfl_sync(0xffffffffu, pos, 31);
+          int at = n + pos - __popc(m);
+          for (; m; m &= m - 1) row[at++] = J.shell_off[a] + __ffs((int)m) - 1;
+          n += total;
+        }
+        if (threadIdx.x == 0) nact_s = n;
+      }
+      __syncthreads();
+      nact = nact_s;
+      const int nq = (nact + 3) >> 2;
+      nb = nq * (nq + 1) / 2;
+      base = 0;
+      assign();
+    }
+    const int q0 = tile * J.tile_points + (u - t * upt) * J.hunit;
+    const int q1 = min(min(q0 + J.hunit, (tile + 1) * J.tile_points), J.npoint);
+    if (nact == 0 || q0 >= q1) continue;
+    if (nb <= 2 * kH64Threads) {
+      sweep(q0, q1);
+    } else {  // more blocks than the accumulators hold: passes over the unit
+      for (base = 0; base < nb; base += 2 * kH64Threads) {
+        assign();
+        sweep(q0, q1);
+        flush();
+      }
+      base = 0;
+      __syncthreads();
+    }
+  }
+  if (tile >= 0 && nb <= 2 * kH64Threads) flush();
+}
+
 #define HP_LAUNCH_BS(kernel, kind, threads, ...)                                       \
   do {                                                                                 \
     if (hb.blocks[kind] > 0) {                                                         \
@@ -344,12 +768,37 @@ __global__ void __launch_bounds__(kThreads, 3) k_change_g64(Batch bt) {
     }                                                                                  \
   } while (0)
 
+void launch_glisa_pro(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH_BS(k_glisa_pro, K_POINT, kThreads); }
+void launch_glisa_grad(const HostBatch& hb, cudaStream_t st, int use_hvec) {
+  HP_LAUNCH_BS(k_glisa_grad, K_POINT, kThreads, use_hvec);
+}
+void launch_glisa_trials64(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH_BS(k_glisa_trials, K_POINT, kThreads); }
 void launch_basis64(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH_BS(k_basis64, K_POINT, kThreads); }
 void launch_promol_g64(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH_BS(k_promol_g64, K_POINT1, kThreads); }
 void launch_gisa_moments64(const HostBatch& hb, cudaStream_t st) {
   HP_LAUNCH_BS(k_gisa_moments64, K_ATOM_TILE, kThreads);
 }
 void launch_lisa_sc64(const HostBatch& hb, cudaStream_t st) { launch_inner_kernel(k_lisa_sc64, hb, K_ATOM_TILE, st); }
+// rows: most shells of a job of the batch that takes the kernel (0: none).
+void launch_glisa_hess64(const HostBatch& hb, cudaStream_t st, int rows) {
+  if (rows <= 0 || hb.blocks[K_HESS] <= 0) return;
+  // an even row stride, 2 mod 4: 16-byte loads, the staging's columns spread
+  // over the banks. The groups' sums (flush) take 16 values for each of nb
+  // threads rounded up to 32, nb = nq (nq + 1) / 2 with nq = ceil(nact / 4):
+  // at most 4 ld of them, from ld = 10 on
+  const int ld = std::max(10, ((rows + 3) & ~3) + 2);
+  const size_t smem = sizeof(double) * 4 * kH64K * (size_t)ld;
+  static int configured = -1;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (configured != dev) {
+    cudaFuncSetAttribute(k_glisa_hess64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(sizeof(double) * 4 * kH64K * (kH64Rows + 2)));
+    configured = dev;
+  }
+  k_glisa_hess64<<<hb.blocks[K_HESS], kH64Threads, smem, st>>>(hb.b[K_HESS], ld);
+  ++g_launch_count;
+}
 void launch_change_g64(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH_BS(k_change_g64, K_ATOM_TILE, kThreads); }
 
 }  // namespace hp

@@ -65,6 +65,17 @@ __device__ __forceinline__ double div64(double a, double d) {
   return a * y;
 }
 
+// 1 / sqrt(d) from the hardware's approximation and one third-order step
+// y (1 + e/2 + 3 e^2/8), e = 1 - d y^2 (within 2 ulp); d outside 2^-959 ..
+// 2^960 by sqrt and a division.
+__device__ __forceinline__ double rsqrt64(double d) {
+  if ((unsigned)(__double2hiint(d) - 0x04000000) >= 0x78000000u) return 1.0 / sqrt(d);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = __fma_rn(-d * y, y, 1.0);
+  return __fma_rn(y * e, __fma_rn(0.375, e, 0.5), y);
+}
+
 // Distance from grid point p to atom a, in one fixed sequence of roundings:
 // the stored value (JobDev::rd) and a recomputed one are the same bits.
 __device__ __forceinline__ double dist64(const JobDev& J, int p, int a) {

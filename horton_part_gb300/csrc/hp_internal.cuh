@@ -216,6 +216,9 @@ struct JobDev {
   double* oldpro;         // MBIS, aLISA sc with G: pro-atoms of the last inner iteration
                           // [natom][npoint], or null; valid where oldok[natom][ntile] is set
   int* oldok;
+  int* hsched;            // gLISA FP64, at most kH64Rows shells: schedule of k_glisa_hess64, or null:
+                          // block b's units are entries [hsched[b], hsched[b + 1]) behind hbuf + 1 offsets
+  int hbuf, hunit;        // its blocks (packed FP64 partial triangles in hpart), points per unit
   unsigned* smask;        // jobs with gmat: per (atom, tile) the atom's shells that are nonzero
                           // somewhere on the tile [natom][ntile], bit k = its shell k
   double* hist_propars;   // [maxiter][nparam]
@@ -541,6 +544,8 @@ struct HostBatch {
   Batch b[K_NKIND];
   int blocks[K_NKIND];
   bool any_g = false, any_nog = false;  // some job stores the FP64 basis matrix / some does not
+  int hess64_rows = 0;  // most shells of a job on k_glisa_hess64 (0: none)
+  bool hess_old = false;  // some FP64 gLISA job takes k_glisa_hess
   int solve_tiles = 0;  // K_SOLVE: tiles per block, 0 when the batch does not take it
   int nact_max = 0;  // fused gLISA: most active rows of a tile over the batch's jobs
 };
@@ -563,7 +568,8 @@ void launch_gisa(const HostBatch& hb, cudaStream_t st, int mixed);
 void launch_lisa_sc_inner(const HostBatch& hb, cudaStream_t st, int mixed);
 void launch_lisa_newton_inner(const HostBatch& hb, cudaStream_t st, int mixed, int modified);
 void launch_glisa_pro(const HostBatch& hb, cudaStream_t st);
-void launch_glisa_grad(const HostBatch& hb, cudaStream_t st);
+void launch_glisa_grad(const HostBatch& hb, cudaStream_t st, int use_hvec = 0);
+void launch_glisa_trials64(const HostBatch& hb, cudaStream_t st);
 void launch_glisa_hess(const HostBatch& hb, cudaStream_t st);
 void launch_glisa_reduce(const HostBatch& hb, cudaStream_t st);
 void launch_glisa_solve(const HostBatch& hb, cudaStream_t st, int projected, int max_shells, int tc);
@@ -665,6 +671,9 @@ void launch_promol_g64(const HostBatch& hb, cudaStream_t st);
 void launch_gisa_moments64(const HostBatch& hb, cudaStream_t st);  // at_weights and q-vector moments
 void launch_lisa_sc64(const HostBatch& hb, cudaStream_t st);
 void launch_change_g64(const HostBatch& hb, cudaStream_t st);
+constexpr int kH64Rows = 224;   // shells of k_glisa_hess64 (two buffers of 16 points in shared memory)
+constexpr int kH64Blocks = 152; // its blocks per job: one per SM
+void launch_glisa_hess64(const HostBatch& hb, cudaStream_t st, int rows);
 
 // float-float MBIS (hp_ff.cu)
 void launch_promol_ff(const HostBatch& hb, cudaStream_t st);

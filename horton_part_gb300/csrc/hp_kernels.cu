@@ -1135,63 +1135,8 @@ __global__ void k_lisa_ls_pick(Batch bt) {
 // gLISA (glisa.py)
 // ---------------------------------------------------------------------------
 
-// rho0 = G^T c (glisa.py:346-348); d1 = w rho/rho0, d2 = w rho/rho0^2 (0 where
-// sick); entropy and negativity partials (glisa.py:441-450, 784).
-__global__ void __launch_bounds__(kThreads) k_glisa_pro(Batch bt) {
-  __shared__ double red[kWarps * 2];
-  __shared__ double out[2];
-  int tile;
-  const JobDev& J = decode_local(bt, tile);
-  if (glisa_idle(J)) return;
-  double acc[2] = {0.0, 0.0};
-  for (int i = 0; i < J.ppt; ++i) {
-    const int p = point_of(J, tile, i);
-    if (p >= J.npoint) continue;
-    double rho0 = 0.0;
-#pragma unroll 8
-    for (int m = 0; m < J.nshell; ++m) rho0 += J.gmat[(size_t)m * J.npoint + p] * J.propars[m];
-    const double rho = J.rho[p];
-    const double w = J.w[p];
-    const bool sick = (rho < J.density_cutoff) || (rho0 < J.density_cutoff);
-    const double inv = sick ? 0.0 : 1.0 / rho0;
-    const double ratio = rho * inv;
-    const double d2 = w * ratio * inv;
-    J.dvec1[p] = w * ratio;
-    J.dvec2[p] = d2;
-    J.rho0[p] = rho0;
-    if (J.hess_s) J.hess_s[p] = sqrtf((float)d2);
-    if (!sick) acc[0] += w * rho * log(ratio);
-    if (rho0 < J.negative_cutoff) acc[1] += 1.0;
-  }
-  block_sum<2>(acc, red, out);
-  if (threadIdx.x == 0) {
-    J.jpart[(size_t)QJ_ENTROPY * J.ntile + tile] = out[0];
-    J.jpart[(size_t)QJ_NEG * J.ntile + tile] = out[1];
-  }
-}
-
-// gpart[m][tile] = sum_p G[m][p] v[p] with v = d1 (gradient) or v = hvec
-// (Hessian-vector product of the refinement); one warp per row m.
-__global__ void __launch_bounds__(kThreads) k_glisa_grad(Batch bt, int use_hvec) {
-  int tile;
-  const JobDev& J = decode_local(bt, tile);
-  if (glisa_idle(J)) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int p0 = tile * J.tile_points;
-  const int p1 = min(p0 + J.tile_points, J.npoint);
-  const double* v = use_hvec ? J.hvec : J.dvec1;
-  for (int m = warp; m < J.nshell; m += kWarps) {
-    const double* g = J.gmat + (size_t)m * J.npoint;
-    double s = 0.0;
-#pragma unroll 8
-    for (int p = p0 + lane; p < p1; p += 32) s += g[p] * v[p];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) J.gpart[(size_t)m * J.ntile + tile] = s;
-  }
-}
-
-// Hessian partials: 64x64 tile (ti, tj), ti >= tj, over one point split.
+// Hessian partials: 64x64 tile (ti, tj), ti >= tj, over one point split
+// (jobs of more than kH64Rows shells; the others: k_glisa_hess64).
 constexpr int kHT = 64;
 constexpr int kHK = 16;
 
@@ -1200,7 +1145,7 @@ __global__ void __launch_bounds__(kThreads) k_glisa_hess(Batch bt) {
   __shared__ double Bs[kHK][kHT + 1];
   int local;
   const JobDev& J = decode_local(bt, local);
-  if (glisa_idle(J)) return;
+  if (J.hsched || glisa_idle(J)) return;  // hsched: k_glisa_hess64
   const int npair = J.htiles * (J.htiles + 1) / 2;
   const int split = local / npair;
   int pr = local - split * npair;
@@ -1324,6 +1269,48 @@ __global__ void __launch_bounds__(kReduceThreads) k_glisa_reduce(Batch bt) {
         if (cw < chunks && ew < E) {
           double v = 0.0;
           for (int q = 0; q < W; ++q) v += wsum[warp * W + q][lane];
+          int i = (int)((sqrtf(8.0f * (float)ew + 1.0f) - 1.0f) * 0.5f);
+          while (i * (i + 1) / 2 > ew) --i;
+          while ((i + 1) * (i + 2) / 2 <= ew) ++i;
+          const int j = ew - i * (i + 1) / 2;
+          J.hess[(size_t)i * M + j] = v;
+          J.hess[(size_t)j * M + i] = v;
+        }
+      }
+      __syncthreads();
+    }
+  } else if (J.hsched) {
+    // packed FP64 triangles of k_glisa_hess64: as above, plain FP64 sums
+    __shared__ double wsum64[kReduceWarps][32];
+    const int E = M * (M + 1) / 2;
+    const int chunks = (E + 31) / 32;
+    const int G = min((chunks + nblk - 1) / nblk, kReduceWarps);
+    const int W = kReduceWarps / G;
+    for (int c0 = local * G; c0 < chunks; c0 += nblk * G) {
+      const int g = warp / W, sub = warp - g * W;
+      const int c = c0 + g;
+      const int ec = c * 32 + lane;
+      double s = 0.0;
+      if (g < G && c < chunks && ec < E) {
+        constexpr int kU = 8;
+        int sp = sub;
+        for (; sp + (kU - 1) * W < J.hbuf; sp += kU * W) {
+          double x[kU];
+#pragma unroll
+          for (int u = 0; u < kU; ++u) x[u] = J.hpart[(size_t)(sp + u * W) * E + ec];
+#pragma unroll
+          for (int u = 0; u < kU; ++u) s += x[u];
+        }
+        for (; sp < J.hbuf; sp += W) s += J.hpart[(size_t)sp * E + ec];
+      }
+      wsum64[warp][lane] = s;
+      __syncthreads();
+      if (warp < G) {
+        const int cw = c0 + warp;
+        const int ew = cw * 32 + lane;
+        if (cw < chunks && ew < E) {
+          double v = 0.0;
+          for (int q = 0; q < W; ++q) v += wsum64[warp * W + q][lane];
           int i = (int)((sqrtf(8.0f * (float)ew + 1.0f) - 1.0f) * 0.5f);
           while (i * (i + 1) / 2 > ew) --i;
           while ((i + 1) * (i + 2) / 2 <= ew) ++i;
@@ -1461,12 +1448,15 @@ __device__ void chol_solve_block(const double* L, const double* dinv, int n, dou
 // the Newton step's 200 KB of dynamic shared memory.
 constexpr int kNewtonF32Max = 224;
 
-// chol_factor in FP32, for the factor of the tensor-core Hessian: that
-// matrix carries ~1e-7 relative error already, so an FP32 factor is as good a
-// preconditioner for the FP64-residual refinement as an FP64 one (same
-// direction error after each refinement step), at 1/64 of the FP64 cost per
-// operation on GB300. Same layout: factor in the lower triangle, its
-// transpose in the upper, dinv[k] = 1 / L[k][k].
+// chol_factor in panels, the matrix in shared memory. In FP32 for the factor
+// of the tensor-core Hessian: that matrix carries ~1e-7 relative error
+// already, so an FP32 factor is as good a preconditioner for the
+// FP64-residual refinement as an FP64 one (same direction error after each
+// refinement step), at 1/64 of the FP64 cost per operation on GB300. In FP64
+// for the FP64 Hessian (free sets up to kNewtonF64Max; column by column with
+// a root and a division in every column's chain: 160 us for 60 free shells).
+// Same layout: factor in the lower triangle, its transpose in the upper,
+// dinv[k] = 1 / L[k][k].
 //
 // Right-looking in panels of 8 columns, two block barriers per panel:
 //  (1) warp 0 factors the panel's 8 x 8 diagonal block (lane t holds row t;
@@ -1482,37 +1472,48 @@ constexpr int kNewtonF32Max = 224;
 // the factor does not depend on the thread count.
 constexpr int kCholPanel = 8;
 
+// sqrt(d) and 1 / sqrt(d) of a pivot
+__device__ __forceinline__ void pivot_of(float d, float& piv, float& r) {
+  const float dd = fmaxf(d, 1e-37f);
+  piv = sqrtf(dd);
+  r = piv / dd;  // 1 / sqrt(d)
+}
+__device__ __forceinline__ void pivot_of(double d, double& piv, double& r) {
+  const double dd = fmax(d, 1e-300);
+  r = f64::rsqrt64(dd);
+  piv = dd * r;
+}
+
 // (1): the diagonal block at rows / columns kk.. of L, on warp 0
-__device__ __forceinline__ void chol_diag_f(float* L, int n, int kk, float (*pl)[kCholPanel],
-                                            float* pr, float* dinv, int* bad) {
+template <typename T>
+__device__ __forceinline__ void chol_diag_f(T* L, int n, int kk, T (*pl)[kCholPanel], T* pr, T* dinv,
+                                            int* bad) {
   const int t = threadIdx.x & 31;
   const int nb = min(kCholPanel, n - kk);
-  const float tiny = 1e-37f;
-  float a[kCholPanel], lrow[kCholPanel];
+  T a[kCholPanel], lrow[kCholPanel];
 #pragma unroll
   for (int u = 0; u < kCholPanel; ++u) {
-    a[u] = (t < nb && u <= t) ? L[(size_t)(kk + t) * n + kk + u] : (u == t ? 1.0f : 0.0f);
-    lrow[u] = 0.0f;
+    a[u] = (t < nb && u <= t) ? L[(size_t)(kk + t) * n + kk + u] : (u == t ? (T)1 : (T)0);
+    lrow[u] = (T)0;
   }
   bool neg = false;
-  float mypiv = 1.0f, myr = 1.0f;
+  T mypiv = (T)1, myr = (T)1;
 #pragma unroll
   for (int s = 0; s < kCholPanel; ++s) {
-    const float d = __shfl_sync(0xffffffffu, a[s], s);
-    const float dd = fmaxf(d, tiny);
-    const float piv = sqrtf(dd);
-    const float r = piv / dd;  // 1 / sqrt(d)
-    if (s < nb && !(d > 0.0f)) neg = true;
+    const T d = __shfl_sync(0xffffffffu, a[s], s);
+    T piv, r;
+    pivot_of(d, piv, r);
+    if (s < nb && !(d > (T)0)) neg = true;
     if (t == s) {
       mypiv = piv;
       myr = r;
     }
-    const float lts = t > s ? a[s] * r : 0.0f;
+    const T lts = t > s ? a[s] * r : (T)0;
     lrow[s] = lts;
 #pragma unroll
     for (int u = s + 1; u < kCholPanel; ++u) {
-      const float lus = __shfl_sync(0xffffffffu, lts, u);
-      if (t >= u) a[u] = fmaf(-lts, lus, a[u]);
+      const T lus = __shfl_sync(0xffffffffu, lts, u);
+      if (t >= u) a[u] = fma(-lts, lus, a[u]);
     }
   }
   if (t < nb) {
@@ -1528,9 +1529,10 @@ __device__ __forceinline__ void chol_diag_f(float* L, int n, int kk, float (*pl)
   if (neg && t == 0) *bad = 1;
 }
 
-__device__ void chol_factor_f(float* L, int n, int* bad, float* dinv) {
-  __shared__ float pl[kCholPanel][kCholPanel];
-  __shared__ float pr[kCholPanel];
+template <typename T>
+__device__ void chol_factor_f(T* L, int n, int* bad, T* dinv) {
+  __shared__ T pl[kCholPanel][kCholPanel];
+  __shared__ T pr[kCholPanel];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0 && n > 0) chol_diag_f(L, n, 0, pl, pr, dinv, bad);
   __syncthreads();
@@ -1538,19 +1540,19 @@ __device__ void chol_factor_f(float* L, int n, int* bad, float* dinv) {
     const int k8 = k + kCholPanel;
     // (2) panel entries of the trailing rows
     for (int i = k8 + threadIdx.x; i < n; i += blockDim.x) {
-      const float* row = L + (size_t)i * n + k;
-      float x[kCholPanel];
+      const T* row = L + (size_t)i * n + k;
+      T x[kCholPanel];
 #pragma unroll
       for (int s = 0; s < kCholPanel; ++s) {
-        float v = row[s];
+        T v = row[s];
 #pragma unroll
-        for (int u = 0; u < s; ++u) v = fmaf(-x[u], pl[s][u], v);
+        for (int u = 0; u < s; ++u) v = fma(-x[u], pl[s][u], v);
         x[s] = v * pr[s];
         L[(size_t)(k + s) * n + i] = x[s];
       }
     }
     __syncthreads();
-    const float* P = L + (size_t)k * n;  // panel entry s of row i at P[s n + i]
+    const T* P = L + (size_t)k * n;  // panel entry s of row i at P[s n + i]
     if (warp == 0) {
       // (3) on the next diagonal block (rows / columns k8 .. k8 + 7), then (1)
       const int nb = min(kCholPanel, n - k8);
@@ -1560,9 +1562,9 @@ __device__ void chol_factor_f(float* L, int n, int* bad, float* dinv) {
         const int c = e - a * (a + 1) / 2;
         if (a < nb) {
           const int i = k8 + a, j = k8 + c;
-          float v = L[(size_t)i * n + j];
+          T v = L[(size_t)i * n + j];
 #pragma unroll
-          for (int s = 0; s < kCholPanel; ++s) v = fmaf(-P[(size_t)s * n + i], P[(size_t)s * n + j], v);
+          for (int s = 0; s < kCholPanel; ++s) v = fma(-P[(size_t)s * n + i], P[(size_t)s * n + j], v);
           L[(size_t)i * n + j] = v;
         }
       }
@@ -1571,8 +1573,8 @@ __device__ void chol_factor_f(float* L, int n, int* bad, float* dinv) {
     } else {
       // (3) on the 4 x 4 tiles below the next diagonal block
       const int m = n - k8;
-      const int T = (m + 3) / 4;
-      const int ntile = T * (T + 1) / 2 - 3;  // tile rows 0 and 1 lie in the diagonal block
+      const int nt = (m + 3) / 4;
+      const int ntile = nt * (nt + 1) / 2 - 3;  // tile rows 0 and 1 lie in the diagonal block
       for (int tt = threadIdx.x - 32; tt < ntile; tt += blockDim.x - 32) {
         const int lin = tt + 3;
         int ti = (int)((sqrtf(8.0f * (float)lin + 1.0f) - 1.0f) * 0.5f);
@@ -1580,25 +1582,25 @@ __device__ void chol_factor_f(float* L, int n, int* bad, float* dinv) {
         while ((ti + 1) * (ti + 2) / 2 <= lin) ++ti;
         const int tj = lin - ti * (ti + 1) / 2;
         const int i0 = k8 + 4 * ti, j0 = k8 + 4 * tj;
-        float acc[4][4];
+        T acc[4][4];
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             const int i = i0 + a, j = j0 + c;
-            acc[a][c] = (i < n && j <= i) ? L[(size_t)i * n + j] : 0.0f;
+            acc[a][c] = (i < n && j <= i) ? L[(size_t)i * n + j] : (T)0;
           }
 #pragma unroll
         for (int s = 0; s < kCholPanel; ++s) {
-          float xa[4], yc[4];
+          T xa[4], yc[4];
 #pragma unroll
-          for (int a = 0; a < 4; ++a) xa[a] = i0 + a < n ? P[(size_t)s * n + i0 + a] : 0.0f;
+          for (int a = 0; a < 4; ++a) xa[a] = i0 + a < n ? P[(size_t)s * n + i0 + a] : (T)0;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) yc[c] = j0 + c < n ? P[(size_t)s * n + j0 + c] : 0.0f;
+          for (int c = 0; c < 4; ++c) yc[c] = j0 + c < n ? P[(size_t)s * n + j0 + c] : (T)0;
 #pragma unroll
           for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) acc[a][c] = fmaf(-xa[a], yc[c], acc[a][c]);
+            for (int c = 0; c < 4; ++c) acc[a][c] = fma(-xa[a], yc[c], acc[a][c]);
         }
 #pragma unroll
         for (int a = 0; a < 4; ++a)
@@ -1627,25 +1629,26 @@ __device__ void chol_factor_f(float* L, int n, int* bad, float* dinv) {
 // across rows), backward with its rows. Each element receives its updates in
 // column order, forward ascending and backward descending, as in a plain
 // column-by-column substitution.
-__device__ void chol_solve_f(const float* L, const float* dinv, int n, float* y) {
+template <typename T>
+__device__ void chol_solve_f(const T* L, const T* dinv, int n, T* y) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nb = (n + 31) / 32;
   for (int jb = 0; jb < nb; ++jb) {
     const int j0 = jb * 32, j1 = min(j0 + 32, n);
     if (warp == 0) {
       const int i = j0 + lane;
-      float b = i < n ? y[i] : 0.0f;
+      T b = i < n ? y[i] : (T)0;
       for (int j = j0; j < j1; ++j) {
-        const float zj = __shfl_sync(0xffffffffu, b, j - j0) * dinv[j];
-        if (i > j && i < n) b = fmaf(-L[(size_t)j * n + i], zj, b);
+        const T zj = __shfl_sync(0xffffffffu, b, j - j0) * dinv[j];
+        if (i > j && i < n) b = fma(-L[(size_t)j * n + i], zj, b);
         else if (i == j) b = zj;
       }
       if (i < n) y[i] = b;
     }
     __syncthreads();
     for (int i = j1 + threadIdx.x; i < n; i += blockDim.x) {
-      float b = y[i];
-      for (int j = j0; j < j1; ++j) b = fmaf(-L[(size_t)j * n + i], y[j], b);
+      T b = y[i];
+      for (int j = j0; j < j1; ++j) b = fma(-L[(size_t)j * n + i], y[j], b);
       y[i] = b;
     }
     __syncthreads();
@@ -1654,18 +1657,18 @@ __device__ void chol_solve_f(const float* L, const float* dinv, int n, float* y)
     const int j0 = jb * 32, j1 = min(j0 + 32, n);
     if (warp == 0) {
       const int i = j0 + lane;
-      float b = i < n ? y[i] : 0.0f;
+      T b = i < n ? y[i] : (T)0;
       for (int j = j1 - 1; j >= j0; --j) {
-        const float xj = __shfl_sync(0xffffffffu, b, j - j0) * dinv[j];
-        if (i < j) b = fmaf(-L[(size_t)j * n + i], xj, b);
+        const T xj = __shfl_sync(0xffffffffu, b, j - j0) * dinv[j];
+        if (i < j) b = fma(-L[(size_t)j * n + i], xj, b);
         else if (i == j) b = xj;
       }
       if (i < n) y[i] = b;
     }
     __syncthreads();
     for (int i = threadIdx.x; i < j0; i += blockDim.x) {
-      float b = y[i];
-      for (int j = j1 - 1; j >= j0; --j) b = fmaf(-L[(size_t)j * n + i], y[j], b);
+      T b = y[i];
+      for (int j = j1 - 1; j >= j0; --j) b = fma(-L[(size_t)j * n + i], y[j], b);
       y[i] = b;
     }
     __syncthreads();
@@ -1676,6 +1679,9 @@ __device__ void chol_solve_f(const float* L, const float* dinv, int n, float* y)
 // fit in kNewtonSmemL) and the two column buffers (when |F| <= kNewtonColMax).
 constexpr int kNewtonSmemL = 200 * 1024;
 constexpr int kNewtonColMax = 256;
+// FP64 factor in shared memory in panels: factor, 1 / diagonal, right-hand side
+constexpr int kNewtonF64Max = 158;
+static_assert(8 * (kNewtonF64Max * kNewtonF64Max + 2 * kNewtonF64Max) <= kNewtonSmemL, "FP64 factor");
 // FP32 factor in shared memory (factor, 1 / diagonal and the right-hand side)
 // the step runs on one SM; 16 warps (the panel factor needs no more, and keeps
 // its 4 x 4 update tiles in registers at this size)
@@ -1792,6 +1798,28 @@ __global__ void __launch_bounds__(kNewtonThreads) k_glisa_newton_step(Batch bt, 
   }
   if (J.tc && threadIdx.x == 0) atomicAdd(&J.mail->i[MI_F64_FACTORS], 1);
   if (threadIdx.x == 0) J.freeidx[M + 1] = 0;
+  if (nf <= kNewtonF64Max) {  // in panels, all in shared memory
+    double* Ld = l_smem;
+    double* dv = Ld + nf * nf;
+    double* yv = dv + nf;
+    for (int e = threadIdx.x; e < nf * nf; e += kNewtonThreads) {
+      const int i = e / nf, j = e - i * nf;
+      Ld[e] = j <= i ? J.hess[(size_t)fid[i] * M + fid[j]] : 0.0;
+    }
+    for (int m = threadIdx.x; m < M; m += kNewtonThreads) J.delta[m] = 0.0;
+    for (int i = threadIdx.x; i < nf; i += kNewtonThreads) yv[i] = -(1.0 + J.grad[fid[i]]);
+    __syncthreads();
+    chol_factor_f(Ld, nf, &bad, dv);
+    chol_solve_f(Ld, dv, nf, yv);
+    for (int i = threadIdx.x; i < nf; i += kNewtonThreads) {
+      J.delta[fid[i]] = yv[i];
+      J.ctrial[2 * M + i] = dv[i];  // kept, with the factor, for the refinement
+    }
+    if (J.tc)
+      for (int e = threadIdx.x; e < nf * nf; e += kNewtonThreads) J.chol[e] = Ld[e];
+    if (threadIdx.x == 0 && bad) atomicOr(&J.mail->i[MI_ERR], E_SINGULAR);
+    return;
+  }
   const bool l_in_smem = (size_t)nf * nf * sizeof(double) <= (size_t)kNewtonSmemL;
   double* L = l_in_smem ? l_smem : J.chol;
   for (int e = threadIdx.x; e < nf * nf; e += kNewtonThreads) {
@@ -2446,88 +2474,6 @@ __global__ void k_glisa_eval_sum(Batch bt, int what) {
 // The free-set step is k_glisa_newton_step(projected = 1); the trial points
 // come from k_glisa_trial_set after the optional refinement.
 
-// Trial objective differences: tpart[t][tile] = this tile's part of
-// f(c_t) - f(c), f(c) = sum over healthy points of w rho ln(rho / rho0(c)).
-//   rho0_t = sum_m max(c_m + a_t delta_m, 0) g_m
-//          = rho0 + a_t (G^T delta) + sum_{m clipped at t} -(c_m + a_t delta_m) g_m,
-// one pass over G plus the few clipped shells. Where a point is healthy for
-// both, its term is -w rho log1p((rho0_t - rho0) / rho0): the relative change
-// is formed in FP64 and goes through the FP32 log1pf, which keeps each term
-// (and the difference the Armijo test compares) accurate to ~1e-7 of itself
-// without an FP64 log per trial; the few points whose sick status differs
-// between rho0 and rho0_t take FP64 logs. Sums in float-float per thread.
-__global__ void __launch_bounds__(kThreads) k_glisa_trials(Batch bt) {
-  __shared__ double red[kWarps * 2 * kTrials];
-  __shared__ double out[2 * kTrials];
-  int tile;
-  const JobDev& J = decode_local(bt, tile);
-  if (glisa_idle(J)) return;
-  float ah[kTrials], al[kTrials], an[kTrials];
-#pragma unroll
-  for (int t = 0; t < kTrials; ++t) ah[t] = al[t] = an[t] = 0.0f;
-  const int nclip = J.clip[J.nshell];
-  const double cut = J.density_cutoff;
-  for (int i = 0; i < J.ppt; ++i) {
-    const int p = point_of(J, tile, i);
-    if (p >= J.npoint) continue;
-    double u = 0.0;
-#pragma unroll 8
-    for (int m = 0; m < J.nshell; ++m) u += J.gmat[(size_t)m * J.npoint + p] * J.delta[m];
-    // corr_t = -sum_{m clipped at t} (c_m + 2^-t delta_m) g_m: the clipped
-    // sets shrink as t grows, so walk the list (sorted by t_m, largest first)
-    // once, keeping the running sums of c g and delta g
-    double corr[kTrials];
-    {
-      double sc = 0.0, sd = 0.0;
-      int k = 0;
-#pragma unroll
-      for (int t = kTrials - 1; t >= 0; --t) {
-        for (; k < nclip && J.clip[J.nshell + 1 + k] > t; ++k) {
-          const int m = J.clip[k];
-          const double g = J.gmat[(size_t)m * J.npoint + p];
-          sc += J.propars[m] * g;
-          sd += J.delta[m] * g;
-        }
-        corr[t] = -(sc + ldexp(1.0, -t) * sd);
-      }
-    }
-    const double rho = J.rho[p], w = J.w[p], r0 = J.rho0[p];
-    const bool h0 = !(rho < cut || r0 < cut);
-    const double inv = h0 ? 1.0 / r0 : 0.0;
-    const float wr = (float)(w * rho);
-#pragma unroll
-    for (int t = 0; t < kTrials; ++t) {
-      const double dr = ldexp(1.0, -t) * u + corr[t];
-      const double rt = r0 + dr;
-      const bool ht = !(rho < cut || rt < cut);
-      double big = 0.0;
-      float term = 0.0f;
-      if (h0 && ht) {
-        term = -wr * log1pf((float)(dr * inv));
-        an[t] += fabsf(term);
-      } else if (ht) big = w * rho * log(rho / rt);
-      else if (h0) big = -(w * rho * log(rho / r0));
-      if (big != 0.0) {
-        const float bh = (float)big;
-        term = bh;
-        al[t] += (float)(big - (double)bh);
-      }
-      const float s = ah[t] + term;  // TwoSum into (ah, al)
-      const float bb = s - ah[t];
-      al[t] += (ah[t] - (s - bb)) + (term - bb);
-      ah[t] = s;
-    }
-  }
-  double acc[2 * kTrials];
-#pragma unroll
-  for (int t = 0; t < kTrials; ++t) {
-    acc[t] = (double)ah[t] + (double)al[t];
-    acc[kTrials + t] = (double)an[t];
-  }
-  block_sum<2 * kTrials>(acc, red, out);
-  if (threadIdx.x < 2 * kTrials) J.tpart[(size_t)threadIdx.x * J.ntile + tile] = out[threadIdx.x];
-}
-
 // One warp per job: Armijo choice among the trials, apply the step.
 // One warp per trial (kTrials warps): warp t forms F(c_t) - F(c) and the
 // Armijo bound of trial t; the first trial (in step order) that passes is
@@ -2745,11 +2691,10 @@ void launch_lisa_newton_inner(const HostBatch& hb, cudaStream_t st, int mixed, i
   }
 }
 
-void launch_glisa_pro(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_glisa_pro, K_POINT, kThreads); }
-void launch_glisa_grad(const HostBatch& hb, cudaStream_t st) {
-  HP_LAUNCH(k_glisa_grad, K_POINT, kThreads, 0);
+void launch_glisa_hess(const HostBatch& hb, cudaStream_t st) {
+  launch_glisa_hess64(hb, st, hb.hess64_rows);
+  if (hb.hess_old) HP_LAUNCH(k_glisa_hess, K_HESS, kThreads);
 }
-void launch_glisa_hess(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_glisa_hess, K_HESS, kThreads); }
 void launch_glisa_reduce(const HostBatch& hb, cudaStream_t st) {
   HP_LAUNCH(k_glisa_reduce, K_SQUARE, kReduceThreads);
 }
@@ -2791,7 +2736,7 @@ void launch_glisa_refine(const HostBatch& hb, cudaStream_t st, int gff, int fuse
     if (unfused) launch_glisa_hv_ff(hb, st);
   } else {
     HP_LAUNCH(k_glisa_hv, K_POINT1, kThreads);
-    HP_LAUNCH(k_glisa_grad, K_POINT, kThreads, 1);
+    launch_glisa_grad(hb, st, 1);
   }
   HP_LAUNCH(k_glisa_gsum, K_SQUARE, kThreads);  // K_SQUARE: ceil(M^2 / 256) >= ceil(M / 8) blocks
   if (hb.blocks[K_JOB] > 0) {  // dynamic shared memory: the FP32 factor (set up by launch_glisa_solve)
@@ -2824,7 +2769,7 @@ void launch_glisa_pnewton(const HostBatch& hb, cudaStream_t st, int gff, int fus
   HP_LAUNCH(k_glisa_trial_set, K_JOB, kThreads);
   if (fuse_shells > 0) launch_glisa_trials_fused(hb, st, fuse_shells);
   else if (gff) launch_glisa_trials_ff(hb, st);
-  else HP_LAUNCH(k_glisa_trials, K_POINT, kThreads);
+  else launch_glisa_trials64(hb, st);
   HP_LAUNCH(k_glisa_trial_pick, K_JOB, 32 * kTrials);
 }
 

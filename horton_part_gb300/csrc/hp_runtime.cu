@@ -127,6 +127,8 @@ struct hp_job {
   // oldok), given back when another allocation needs the room (make_room)
   void* keep_mem = nullptr;
   size_t keep_bytes = 0;
+  void* sched_mem = nullptr;  // gLISA FP64: dev.hsched
+  size_t sched_bytes = 0;
   void* pack_mem = nullptr;  // fused gLISA: packed G (dev.gpack, dev.gtile_off)
   size_t pack_bytes = 0;
   std::vector<double> changes;  // outer changes of this run
@@ -281,6 +283,7 @@ int blocks_for(const JobDev& J, int kind) {
     case K_FUSE: return J.fuse ? std::min(J.ntile, kFuseCtas) : 0;
     case K_HESS:
       if (J.scheme != SCHEME_GLISA || J.fuse) return 0;  // fused jobs: in the fused pass
+      if (J.hsched) return J.hbuf;
       return J.tc ? tc_hess_blocks(J) : J.nsplit * J.htiles * (J.htiles + 1) / 2;
     case K_SQUARE: return J.scheme == SCHEME_GLISA ? (J.nshell * J.nshell + kThreads - 1) / kThreads : 0;
   }
@@ -315,7 +318,13 @@ int build_batch(hp_ctx* ctx, const std::vector<hp_job*>& jobs, HostBatch& hb) {
   hb.nact_max = 0;
   hb.solve_tiles = solve_tiles(jobs);
   hb.any_g = hb.any_nog = false;
-  for (const hp_job* j : jobs) (j->dev.gmat ? hb.any_g : hb.any_nog) = true;
+  hb.hess64_rows = 0;
+  hb.hess_old = false;
+  for (const hp_job* j : jobs) {
+    (j->dev.gmat ? hb.any_g : hb.any_nog) = true;
+    if (j->dev.hsched) hb.hess64_rows = std::max(hb.hess64_rows, j->dev.nshell);
+    else hb.hess_old = true;
+  }
   for (int j = 0; j < n; ++j) {
     ctx->batch_host[j] = jobs[j]->dev;
     hb.nact_max = std::max(hb.nact_max, jobs[j]->dev.nact_max);
@@ -507,6 +516,62 @@ int pack_layout(hp_ctx* ctx, const std::vector<hp_job*>& jobs) {
   return HP_OK;
 }
 
+// FP64 gLISA jobs of at most kH64Rows shells: the schedule of k_glisa_hess64
+// from the masks of active shells (k_basis64), once per job. A unit is some
+// points of one tile, about 16 units per block; its work is points times
+// products. A job without room for the schedule keeps k_glisa_hess.
+int hess_layout(hp_ctx* ctx, const std::vector<hp_job*>& jobs) {
+  auto wanted = [](const hp_job* j) {
+    const JobDev& J = j->dev;
+    return J.scheme == SCHEME_GLISA && J.gmat && !J.tc && J.solver != SOLVER_SC && J.nshell <= kH64Rows &&
+           !J.hsched;
+  };
+  bool any = false;
+  for (hp_job* j : jobs) any |= wanted(j);
+  if (!any) return HP_OK;
+  HP_CK(cudaStreamSynchronize(ctx->stream));
+  for (hp_job* j : jobs) {
+    if (!wanted(j)) continue;
+    JobDev& J = j->dev;
+    std::vector<unsigned> mask((size_t)J.natom * J.ntile);
+    HP_CK(cudaMemcpy(mask.data(), J.smask, 4 * mask.size(), cudaMemcpyDeviceToHost));
+    const int64_t tri = (int64_t)J.nshell * (J.nshell + 1) / 2;
+    const int64_t room = (int64_t)J.nsplit * J.nshell * J.nshell / tri;  // packed partials hpart holds
+    int unit = (int)((J.npoint + 16 * kH64Blocks - 1) / (16 * kH64Blocks));
+    unit = std::min(std::max((unit + 15) / 16 * 16, 64), J.tile_points);
+    const int upt = (J.tile_points + unit - 1) / unit;
+    const int nu = J.ntile * upt;
+    std::vector<int64_t> work(nu, 0);
+    for (int t = 0; t < J.ntile; ++t) {
+      int64_t n = 0;
+      for (int a = 0; a < J.natom; ++a) n += __builtin_popcount(mask[(size_t)a * J.ntile + t]);
+      for (int u = 0; u < upt; ++u) {
+        const int64_t q0 = (int64_t)t * J.tile_points + (int64_t)u * unit;
+        const int64_t q1 = std::min<int64_t>({q0 + unit, (int64_t)(t + 1) * J.tile_points, (int64_t)J.npoint});
+        work[(size_t)t * upt + u] = std::max<int64_t>(0, q1 - q0) * (n * (n + 1) / 2 + 8 * n);
+      }
+    }
+    const int nb = (int)std::min<int64_t>({(int64_t)kH64Blocks, room, (int64_t)nu});
+    if (nb < 1) continue;
+    const std::vector<int> sched = tile_schedule(work, nb);
+    const size_t bytes = 4 * ((size_t)nb + 1 + nu);
+    void* mem = nullptr;
+    if (!make_room(ctx, bytes) || job_alloc_retry(ctx, &mem, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
+    HP_CK(cudaMemcpyAsync(mem, sched.data(), bytes, cudaMemcpyHostToDevice, ctx->stream));
+    J.hsched = reinterpret_cast<int*>(mem);
+    J.hbuf = nb;
+    J.hunit = unit;
+    j->sched_mem = mem;
+    j->sched_bytes = bytes;
+    j->bytes += bytes;
+    ctx->used += bytes;
+  }
+  return HP_OK;
+}
+
 int job_init(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatch& hb) {
   launch_nelec(hb, ctx->stream);
   bool any_basis = false, any_basis_ff = false, any_rdist = false, any_rd = false;
@@ -521,7 +586,11 @@ int job_init(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatch& hb)
   if (any_geo) launch_tile_rmin(hb, ctx->stream);
   if (any_rd) launch_rdist64(hb, ctx->stream);
   if (any_rdist) launch_rdist_ff(hb, ctx->stream);
-  if (any_basis) launch_basis64(hb, ctx->stream);
+  if (any_basis) {
+    launch_basis64(hb, ctx->stream);
+    int rc = hess_layout(ctx, jobs);
+    if (rc) return rc;
+  }
   if (any_basis_ff) launch_glisa_basis_ff(hb, ctx->stream);
   int fuse_shells = 0;
   for (hp_job* j : jobs)
@@ -1583,6 +1652,7 @@ int32_t hp_job_destroy(hp_job* job) {
   cudaStreamSynchronize(ctx->stream);
   job_free(ctx, job->mem);  // back to the context's pool, in stream order
   job_free(ctx, job->pack_mem);
+  job_free(ctx, job->sched_mem);
   job_free(ctx, job->keep_mem);
   ctx->used -= job->bytes;
   ctx->kept -= job->keep_bytes;
@@ -1704,6 +1774,8 @@ int eval_ready(hp_job* job, HostBatch& hb) {
     rc = job_init(ctx, one, hb);
     if (rc) return rc;
     HP_CK(cudaStreamSynchronize(ctx->stream));
+    rc = build_batch(ctx, one, hb);  // the descriptor has its schedule now
+    if (rc) return rc;
   }
   return HP_OK;
 }
