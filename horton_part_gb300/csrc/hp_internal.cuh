@@ -212,6 +212,7 @@ struct JobDev {
   double* radrho;         // nrad: spherical average of w_a rho
   // FP64 kernels (hp_fp64.cuh)
   const double* etab;     // 2^(j/512), j < 512
+  const float2* etabf;    // the same as float pairs (hi, lo): MBIS in float-float
   double* rd;             // MBIS: distances [natom][npoint], or null (recomputed)
   double* oldpro;         // MBIS, aLISA sc with G: pro-atoms of the last inner iteration
                           // [natom][npoint], or null; valid where oldok[natom][ntile] is set
@@ -690,13 +691,20 @@ struct DensityArgs {
   const int* info;        // [nshell][5]: l, pure, nprim, first primitive, first function
   const double* amin;     // [nshell] smallest exponent of the shell
   const double* exps;     // [nprim]
+  const float* rcut2;     // [nprim] squared distance from which the primitive is below 2^-70 of the
+                          // shell's most diffuse one
   const double* coefs;    // [nprim] contraction coefficient x primitive normalisation
   const double* mats;     // [nmat][nbasis][nbasis]
+  const double* etab;     // 2^(j/512)
+  const int* groups;      // [ngroup + 1] first shells of the runs of shells with one centre
+  int ngroup;
   double* out;            // [nmat][npoint]
   unsigned long long* stats;  // [3]: shell-tile pairs, function-point pairs, FMA per matrix; or null
 };
-constexpr size_t kDensSmemMax = 200 * 1024;
-size_t density_smem_bytes(int nbasis, int nshell, int tile);
+// the tile of a basis is the largest whose values fit: 200 KB as before the
+// exponential's table (4 KB) joined them
+constexpr size_t kDensSmemMax = 200 * 1024 + 4096;
+size_t density_smem_bytes(int nbasis, int nshell, int tile, int threads);
 int density_tile(int nbasis, int nshell);
 int set_pure_tables(const double* pure2, const double* pure3);
 void launch_density(const DensityArgs& a, cudaStream_t st);

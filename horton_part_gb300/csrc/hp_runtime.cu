@@ -58,7 +58,7 @@ struct hp_ctx {
   std::vector<hp_job*> slots;
   JobDev* batch_dev = nullptr;     // JobDev array of the current batch
   JobDev* batch_host = nullptr;    // pinned staging
-  double* exp_tab = nullptr;       // 2^(j/512), j < 512 (JobDev::etab)
+  double* exp_tab = nullptr;       // 2^(j/512), j < 512 (JobDev::etab), then as float pairs (etabf)
   int* prefix_dev = nullptr;       // [K_NKIND][jobs of the batch + 1]
   int* prefix_host = nullptr;      // pinned staging
   // kernel timing (hp_ctx_profile)
@@ -1150,10 +1150,18 @@ int32_t hp_ctx_create(int32_t device, size_t hbm_budget, void* stream, hp_ctx** 
     return fail(HP_ERR_NO_MEMORY, "context allocation failed");
   }
   {
-    double tab[512];
-    for (int j = 0; j < 512; ++j) tab[j] = (double)exp2l((long double)j / 512.0L);
+    struct {
+      double d[512];
+      float2 f[512];
+    } tab;
+    for (int j = 0; j < 512; ++j) {
+      const long double v = exp2l((long double)j / 512.0L);
+      tab.d[j] = (double)v;
+      const float hi = (float)v;
+      tab.f[j] = make_float2(hi, (float)(v - (long double)hi));
+    }
     if (cudaMalloc(&c->exp_tab, sizeof(tab)) != cudaSuccess ||
-        cudaMemcpy(c->exp_tab, tab, sizeof(tab), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaMemcpy(c->exp_tab, &tab, sizeof(tab), cudaMemcpyHostToDevice) != cudaSuccess) {
       hp_ctx_destroy(c);
       return fail(HP_ERR_NO_MEMORY, "context allocation failed");
     }
@@ -1423,6 +1431,7 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   }
   J.mail = ctx->mail_dev + slot;
   J.etab = ctx->exp_tab;
+  J.etabf = reinterpret_cast<const float2*>(ctx->exp_tab + 512);
   J.natom = A; J.npoint = N; J.ntile = ntile; J.nparam = P; J.nshell = S; J.qa = qa;
   J.scheme = d->scheme; J.solver = solver; J.maxiter = maxiter;
   J.mixed = !mixed ? PH_FP64 : d->precision == HP_PRECISION_FF ? PH_FF : PH_FP32;
@@ -2022,6 +2031,7 @@ struct hp_density_plan {
   int* info = nullptr;
   unsigned long long* stats = nullptr;   // [3]
   size_t bytes = 0;
+  int* groups = nullptr;                 // [ngroup + 1], then rcut2 [nprim] (floats)
   double* scratch = nullptr;             // host-pointer evaluations: points and out
   size_t scratch_points = 0;
 };
@@ -2035,6 +2045,7 @@ int32_t hp_density_plan_create(hp_ctx* ctx, const hp_density_desc* d, hp_density
     return fail(HP_ERR_INVALID, "incomplete density description");
   const int ns = d->nshell, nb = d->nbasis;
   std::vector<double> amin(ns, 0.0);
+  std::vector<float> rcut2(std::max(1, d->nprim), INFINITY);
   int nf = 0;
   bool pure2 = false, pure3 = false;
   for (int s = 0; s < ns; ++s) {
@@ -2047,10 +2058,19 @@ int32_t hp_density_plan_create(hp_ctx* ctx, const hp_density_desc* d, hp_density
     nf += nfs;
     if (pure && l == 2) pure2 = true;
     if (pure && l == 3) pure3 = true;
-    double a = INFINITY;
+    double a = INFINITY, ca = 0.0;
     for (int k = k0; k < k0 + np; ++k) {
       if (!(d->exponents[k] > 0.0)) return fail(HP_ERR_INVALID, "exponents must be positive");
-      if (d->coeffs[k] != 0.0) a = std::min(a, d->exponents[k]);
+      if (d->coeffs[k] != 0.0 && d->exponents[k] < a) {
+        a = d->exponents[k];
+        ca = std::fabs(d->coeffs[k]);
+      }
+    }
+    for (int k = k0; k < k0 + np; ++k) {
+      // |c_k| exp(-a_k r^2) < 2^-70 |c_a| exp(-a r^2), a margin for the rounding of r^2 to FP32
+      const double lead = std::log(std::fabs(d->coeffs[k]) / ca) + 70.0 * std::log(2.0);
+      const double r2 = 1.000001 * std::max(lead, 0.0) / (d->exponents[k] - a);
+      rcut2[k] = d->exponents[k] > a && std::isfinite(r2) && r2 < 1e30 ? (float)r2 : INFINITY;
     }
     amin[s] = std::isfinite(a) ? a : 1e300;  // a shell with no nonzero coefficient is never significant
   }
@@ -2061,12 +2081,21 @@ int32_t hp_density_plan_create(hp_ctx* ctx, const hp_density_desc* d, hp_density
   if (tile == 0) return fail(HP_ERR_UNSUPPORTED, "basis too large for one point tile");
   HP_CK(cudaSetDevice(ctx->device));
   const size_t ndbl = 3 * (size_t)ns + ns + 2 * (size_t)d->nprim + (size_t)d->nmat * nb * nb;
-  const size_t bytes = 8 * ndbl + 4 * 5 * (size_t)ns + 8 * 3;
+  std::vector<int> groups;  // runs of consecutive shells with one centre
+  for (int k = 0; k < ns; ++k)
+    if (k == 0 || memcmp(d->centers + 3 * k, d->centers + 3 * (k - 1), 24) != 0) groups.push_back(k);
+  const int ngroup = (int)groups.size();
+  groups.push_back(ns);
+  const size_t rcut_at = groups.size();
+  groups.resize(rcut_at + rcut2.size());
+  memcpy(groups.data() + rcut_at, rcut2.data(), 4 * rcut2.size());
+  const size_t bytes = 8 * ndbl + 4 * 5 * (size_t)ns + 8 * 3 + 4 * groups.size();
   if (!make_room(ctx, bytes)) return fail(HP_ERR_NO_MEMORY, "HBM budget exceeded");
   hp_density_plan* p = new hp_density_plan();
   p->ctx = ctx;
   if (cudaMalloc(&p->dev, 8 * std::max<size_t>(ndbl, 1)) != cudaSuccess ||
       cudaMalloc(&p->info, 4 * std::max<size_t>(5 * (size_t)ns, 1)) != cudaSuccess ||
+      cudaMalloc(&p->groups, 4 * groups.size()) != cudaSuccess ||
       cudaMalloc(&p->stats, 8 * 3) != cudaSuccess) {
     hp_density_plan_destroy(p);
     return fail(HP_ERR_NO_MEMORY, "device allocation failed");
@@ -2084,6 +2113,7 @@ int32_t hp_density_plan_create(hp_ctx* ctx, const hp_density_desc* d, hp_density
   rc |= cudaMemcpyAsync(co, d->coeffs, 8 * (size_t)d->nprim, cudaMemcpyHostToDevice, st) != cudaSuccess;
   rc |= cudaMemcpyAsync(mats, d->mats, 8 * (size_t)d->nmat * nb * nb, cudaMemcpyHostToDevice, st) != cudaSuccess;
   rc |= cudaMemcpyAsync(p->info, d->shell_info, 4 * 5 * (size_t)ns, cudaMemcpyHostToDevice, st) != cudaSuccess;
+  rc |= cudaMemcpyAsync(p->groups, groups.data(), 4 * groups.size(), cudaMemcpyHostToDevice, st) != cudaSuccess;
   rc |= cudaMemsetAsync(p->stats, 0, 8 * 3, st) != cudaSuccess;
   if (pure2 || pure3) {
     double t2[30] = {0.0}, t3[70] = {0.0};
@@ -2110,6 +2140,10 @@ int32_t hp_density_plan_create(hp_ctx* ctx, const hp_density_desc* d, hp_density
   a.coefs = co;
   a.mats = mats;
   a.stats = p->stats;
+  a.etab = ctx->exp_tab;
+  a.groups = p->groups;
+  a.ngroup = ngroup;
+  a.rcut2 = reinterpret_cast<const float*>(p->groups + rcut_at);
   *out = p;
   return HP_OK;
 }
@@ -2176,6 +2210,7 @@ int32_t hp_density_plan_destroy(hp_density_plan* p) {
   if (p->dev) cudaFree(p->dev);
   if (p->info) cudaFree(p->info);
   if (p->stats) cudaFree(p->stats);
+  if (p->groups) cudaFree(p->groups);
   if (p->scratch) cudaFree(p->scratch);
   delete p;
   return HP_OK;
