@@ -19,20 +19,6 @@
 
 namespace hp {
 
-namespace ffa {
-
-// 2^(i/64), i = 0..63, as (hi, lo) float pairs; copied into shared memory by
-// each block (the index differs between lanes).
-__constant__ float2 c_exp2_table[64];
-
-// Block-local copy of the table (call with all threads, before any exp_ff).
-__device__ __forceinline__ void load_exp_table(float2* tab) {
-  if (threadIdx.x < 64) tab[threadIdx.x] = c_exp2_table[threadIdx.x];
-  __syncthreads();
-}
-
-}  // namespace ffa
-
 namespace {
 
 using ffa::f2;
@@ -352,26 +338,6 @@ __global__ void __launch_bounds__(kThreads) k_final_atweights_ff(Batch bt, int u
 // launchers
 // ---------------------------------------------------------------------------
 
-namespace {
-
-// 2^(i/64) as float pairs, from the host's double-precision exp2; once per device.
-void ensure_exp_table() {
-  static int done_mask = 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 31 && (done_mask >> dev) & 1) return;
-  float2 t[64];
-  for (int i = 0; i < 64; ++i) {
-    const double v = exp2((double)i / 64.0);
-    const float hi = (float)v;
-    t[i] = make_float2(hi, (float)(v - (double)hi));
-  }
-  cudaMemcpyToSymbol(ffa::c_exp2_table, t, sizeof(t));
-  if (dev < 31) done_mask |= 1 << dev;
-}
-
-}  // namespace
-
 // Point-atom distances of a mixed / ff job as float pairs (once per job):
 // every later kernel reads them instead of re-forming the distance.
 __global__ void __launch_bounds__(kThreads) k_rdist_ff(Batch bt) {
@@ -396,11 +362,11 @@ __global__ void __launch_bounds__(kThreads) k_rdist_ff(Batch bt) {
 // classified once per block into shared memory (an FP64 comparison per shell
 // and point would run on the FP64 pipe, 1/64 of the FP32 rate).
 __global__ void __launch_bounds__(kThreads) k_glisa_basis_ff(Batch bt) {
-  __shared__ float2 tab[64];
+  __shared__ float2 tab[512];
   __shared__ int ord[kGffMaxShells];  // 2, 1 (FF paths) or 0 (FP64)
-  ffa::load_exp_table(tab);
   int blk;
   const JobDev& J = decode_local_ff(bt, blk);
+  load_exp512(tab, J.etabf);
   for (int s = threadIdx.x; s < J.nshell; s += kThreads) {
     const double o = J.sh_order[s];
     ord[s] = o == 2.0 ? 2 : o == 1.0 ? 1 : 0;
@@ -425,7 +391,7 @@ __global__ void __launch_bounds__(kThreads) k_glisa_basis_ff(Batch bt) {
       if (order != 0) {
         const float* c = J.fpar + 4 * s;
         const f2 x = ffa::mul(f2{c[2], c[3]}, order == 2 ? d2 : r);
-        g = ffa::mul(f2{c[0], c[1]}, ffa::exp_ff(ffa::neg(x), tab));
+        g = ffa::mul(f2{c[0], c[1]}, ffa::exp_ff512(ffa::neg(x), tab));
       } else {
         const double v = basis_shell<double>(J.sh_order[s], J.sh_alpha[s], J.sh_pref[s],
                                              Dist<double>::r(J, p, a));
@@ -461,7 +427,6 @@ void launch_rdist_ff(const HostBatch& hb, cudaStream_t st) {
 }
 
 void launch_glisa_basis_ff(const HostBatch& hb, cudaStream_t st) {
-  ensure_exp_table();
   HP_LAUNCH_FF(k_glisa_basis_ff, K_POINT1, kThreads);
 }
 

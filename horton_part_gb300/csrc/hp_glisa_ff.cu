@@ -16,7 +16,7 @@
 #include <math.h>
 
 #include "hp_ff.cuh"
-#include "hp_internal.cuh"
+#include "hp_fp64.cuh"
 #include "hp_umma.cuh"
 
 namespace hp {
@@ -1236,73 +1236,113 @@ __global__ void __launch_bounds__(kThreads) k_glisa_wgram(Batch bt) {
 // per atom, as k_promol) and its reciprocal in FP64 for k_glisa_atweights_ff.
 __global__ void __launch_bounds__(kThreads) k_glisa_promol_ff(Batch bt) {
   __shared__ float2 cf[kGffMaxShells];
+  __shared__ int act[kFuseMaxShells];
   int blk;
   const JobDev& J = decode_local_gf(bt, blk);
+  // fused jobs: the tile's active rows from the packed planes (the other rows
+  // add exact zeros), and no FP64 operation for an atom without one
+  const int tile = blk / J.ppt;
+  const int* ga = J.gpack ? J.gact + (size_t)tile * (J.nshell + 1) : nullptr;
+  const int nact = ga ? ga[J.nshell] : 0;
+  for (int i = threadIdx.x; i < nact; i += kThreads) act[i] = ga[i];
   load_pairs(J.propars, J.nshell, cf);
   const int p = blk * kThreads + threadIdx.x;
   if (p >= J.npoint) return;
   const size_t N = J.npoint;
   double promol = 0.0;
-  int m = J.shell_off[0];
-  for (int a = 0; a < J.natom; ++a) {
-    const int m1 = J.shell_off[a + 1];
-    Dot2 d{0.f, 0.f};
-    for (; m < m1; ++m) dot2_add(d, J.gmat32[m * N + p], J.gmat_lo[m * N + p], cf[m].x, cf[m].y);
-    const double pro = dot2_value(d);
+  int a = 0, m1 = J.shell_off[1];
+  Dot2 d{0.f, 0.f};
+  bool any = false;
+  auto flush = [&]() {  // atom a is complete
+    const double pro = any ? dot2_value(d) : 0.0;
     J.rhoa[(size_t)a * N + p] = pro;
-    promol += pro;
-    promol += 1e-100;
+    if (any) promol += pro;
+    // 1e-100 per atom, as k_promol: lost in a sum of 1e-80 or more
+    if ((unsigned)(__double2hiint(promol) - 0x2f600000) >= 0x50900000u) promol += 1e-100;
+    d = Dot2{0.f, 0.f};
+    any = false;
+    ++a;
+    if (a < J.natom) m1 = J.shell_off[a + 1];
+  };
+  if (ga) {
+    const int q = p - tile * J.tile_points;  // a warp's points are one sub-tile
+    const float* hi = J.gpack + J.gtile_off[tile] + (size_t)(q >> 5) * nact * 32 + (q & 31);
+    const float* lo = hi + J.gpack_plane;
+    for (int i = 0; i < nact; i += 4) {
+      float h[4], l[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int k = min(i + u, nact - 1);
+        h[u] = hi[32 * k];
+        l[u] = lo[32 * k];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (i + u >= nact) break;
+        const int k = act[i + u];
+        while (k >= m1) flush();
+        dot2_add(d, h[u], l[u], cf[k].x, cf[k].y);
+        any = true;
+      }
+    }
+  } else {
+    for (int m = 0; m < J.nshell; ++m) {
+      while (m >= m1) flush();
+      dot2_add(d, J.gmat32[m * N + p], J.gmat_lo[m * N + p], cf[m].x, cf[m].y);
+      any = true;
+    }
   }
+  while (a < J.natom) flush();
   J.promol[p] = promol;
   J.invpro[p] = 1.0 / promol;
 }
 
 // at_weights of a float-float gLISA job from the final promolecule, one block
 // per point tile for all atoms (k_atweights takes a block per atom and tile
-// and re-reads the per-point arrays for each atom): per atom
-// rho_a = clip(pro_a / promol, 0, 1) rho, the tile's sum of w rho_a (QA_POP)
-// and largest rho_a, and the tile's entropy sum of w rho ln(rho / promol)
-// over the points above the cutoff. Each thread takes its points in the same
-// order and the block sums are the same as in k_atweights.
+// and re-reads the per-point arrays for each atom): rho_a = clip(pro_a /
+// promol, 0, 1) rho, the tile's sum of w rho_a (QA_POP) and the tile's entropy
+// sum of w rho ln(rho / promol) over the points above the cutoff. Bound by
+// the FP64 pipe: a warp per atom (no block sums), the clip by integer
+// comparisons, and nothing for an atom whose rows are all zero on the tile
+// (its pro-atom is). With k_glisa_promol_ff on the active rows: 470 -> 286 us
+// a job on the 20-atom molecule.
 __global__ void __launch_bounds__(kThreads) k_glisa_atweights_ff(Batch bt) {
   __shared__ double red[kWarps];
   __shared__ double out[1];
-  __shared__ float redm[kWarps];
   int tile;
   const JobDev& J = decode_local_gf(bt, tile);
   const size_t N = J.npoint;
+  const int p0 = tile * J.tile_points, p1 = min(p0 + J.tile_points, J.npoint);
   double acc[1] = {0.0};
-  for (int i = 0; i < J.ppt; ++i) {
-    const int p = point_in_tile(J, tile, i);
-    if (p >= J.npoint) continue;
+  for (int p = p0 + threadIdx.x; p < p1; p += kThreads) {
     const double promol = J.promol[p], rho = J.rho[p];
     const bool sick = (promol < J.density_cutoff) || (rho < J.density_cutoff);
     if (!sick) acc[0] += J.w[p] * rho * log(rho / promol);
   }
   block_sum<1>(acc, red, out);
   if (threadIdx.x == 0) J.jpart[(size_t)QJ_ENTROPY * J.ntile + tile] = out[0];
-  // the largest rho_a per tile only where a per-atom cutoff keeps it (its
-  // comparison and conversion are FP64 operations, like the sums)
-  const bool want_max = J.amax != nullptr;
-  for (int a = 0; a < J.natom; ++a) {
-    double pop[1] = {0.0};
-    float vmax = 0.0f;
-    double* ra = J.rhoa + (size_t)a * N;
+  const int lane = threadIdx.x & 31;
+  const int* act = J.gact ? J.gact + (size_t)tile * (J.nshell + 1) : nullptr;
+  const int nact = act ? act[J.nshell] : 0;
+  const double* __restrict__ inv = J.invpro;
+  const double* __restrict__ rhov = J.rho;
+  const double* __restrict__ wv = J.w;
+  for (int a = threadIdx.x >> 5; a < J.natom; a += kWarps) {
+    double pop = 0.0;
+    bool any = act == nullptr;
+    for (int i = lane; i < nact && !any; i += 32) any = act[i] >= J.shell_off[a] && act[i] < J.shell_off[a + 1];
+    if (__any_sync(0xffffffffu, any)) {
+      double* ra = J.rhoa + (size_t)a * N;
 #pragma unroll 4
-    for (int i = 0; i < J.ppt; ++i) {
-      const int p = point_in_tile(J, tile, i);
-      if (p >= J.npoint) continue;
-      const double v = fmin(fmax(ra[p] * J.invpro[p], 0.0), 1.0) * J.rho[p];
-      ra[p] = v;
-      if (want_max) vmax = fmaxf(vmax, v > 3e38 ? 3e38f : (float)v);
-      pop[0] += J.w[p] * v;
+      for (int p = p0 + lane; p < p1; p += 32) {
+        const double v = f64::clip01(ra[p] * inv[p]) * rhov[p];
+        ra[p] = v;
+        pop = __fma_rn(wv[p], v, pop);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) pop += __shfl_xor_sync(0xffffffffu, pop, o);
     }
-    block_sum<1>(pop, red, out);
-    if (want_max) {
-      const float mx = block_max_f(vmax, redm);
-      if (threadIdx.x == 0) J.amax[(size_t)a * J.ntile + tile] = mx;
-    }
-    if (threadIdx.x == 0) J.apart[((size_t)a * J.qa + QA_POP) * J.ntile + tile] = out[0];
+    if (lane == 0) J.apart[((size_t)a * J.qa + QA_POP) * J.ntile + tile] = pop;
   }
 }
 

@@ -1636,12 +1636,18 @@ __device__ void chol_solve_f(const T* L, const T* dinv, int n, T* y) {
   for (int jb = 0; jb < nb; ++jb) {
     const int j0 = jb * 32, j1 = min(j0 + 32, n);
     if (warp == 0) {
-      const int i = j0 + lane;
+      const int i = j0 + lane, w = j1 - j0;
       T b = i < n ? y[i] : (T)0;
-      for (int j = j0; j < j1; ++j) {
-        const T zj = __shfl_sync(0xffffffffu, b, j - j0) * dinv[j];
-        if (i > j && i < n) b = fma(-L[(size_t)j * n + i], zj, b);
-        else if (i == j) b = zj;
+      T l[32];  // this row's entries, read ahead of the chain
+#pragma unroll
+      for (int u = 0; u < 32; ++u) l[u] = u < lane && i < n ? L[(size_t)(j0 + u) * n + i] : (T)0;
+      const T di = i < n ? dinv[i] : (T)0;
+#pragma unroll
+      for (int u = 0; u < 32; ++u) {
+        if (u >= w) break;
+        if (lane == u) b *= di;
+        const T zj = __shfl_sync(0xffffffffu, b, u);
+        if (lane > u) b = fma(-l[u], zj, b);
       }
       if (i < n) y[i] = b;
     }
@@ -1656,12 +1662,18 @@ __device__ void chol_solve_f(const T* L, const T* dinv, int n, T* y) {
   for (int jb = nb - 1; jb >= 0; --jb) {
     const int j0 = jb * 32, j1 = min(j0 + 32, n);
     if (warp == 0) {
-      const int i = j0 + lane;
+      const int i = j0 + lane, w = j1 - j0;
       T b = i < n ? y[i] : (T)0;
-      for (int j = j1 - 1; j >= j0; --j) {
-        const T xj = __shfl_sync(0xffffffffu, b, j - j0) * dinv[j];
-        if (i < j) b = fma(-L[(size_t)j * n + i], xj, b);
-        else if (i == j) b = xj;
+      T l[32];
+#pragma unroll
+      for (int u = 0; u < 32; ++u) l[u] = u > lane && u < w ? L[(size_t)(j0 + u) * n + i] : (T)0;
+      const T di = i < n ? dinv[i] : (T)0;
+#pragma unroll
+      for (int u = 31; u >= 0; --u) {
+        if (u >= w) continue;
+        if (lane == u) b *= di;
+        const T xj = __shfl_sync(0xffffffffu, b, u);
+        if (lane < u) b = fma(-l[u], xj, b);
       }
       if (i < n) y[i] = b;
     }
