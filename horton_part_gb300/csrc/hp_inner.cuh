@@ -59,26 +59,13 @@ __device__ __forceinline__ bool last_block_of(const JobDev& J, int a) {
 // warp_tile_sum over partials that other blocks of this launch wrote (read
 // from L2), the same order.
 __device__ __forceinline__ double partial_value_cg(const JobDev& J, const double* slot) {
-  if (!J.mixed) return __ldcg(slot);
   const float2 v = __ldcg(reinterpret_cast<const float2*>(slot));
   return (double)v.x + (double)v.y;
 }
 
 __device__ __forceinline__ double warp_tile_sum_cg(const JobDev& J, const double* p, int ntile) {
-  const int lane = threadIdx.x & 31;
-  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-  int t = lane;
-  for (; t + 96 < ntile; t += 128) {
-    s0 += partial_value_cg(J, p + t);
-    s1 += partial_value_cg(J, p + t + 32);
-    s2 += partial_value_cg(J, p + t + 64);
-    s3 += partial_value_cg(J, p + t + 96);
-  }
-  for (; t < ntile; t += 32) s0 += partial_value_cg(J, p + t);
-  double s = (s0 + s1) + (s2 + s3);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  return s;
+  if (!J.mixed) return warp_tile_sum_of(ntile, [&](int t) { return __ldcg(p + t); });
+  return warp_tile_sum_of(ntile, [&](int t) { return partial_value_cg(J, p + t); });
 }
 
 // Mixed precision only: the inner change of FP32-evaluated pro-atoms has a

@@ -413,6 +413,41 @@ __device__ __forceinline__ double partial_value(const JobDev& J, const double* s
   return (double)v.x + (double)v.y;
 }
 
+// Warp sum of load(t) over the tiles t < ntile in a fixed lane order: four
+// chains per lane (tiles t, t + 32, t + 64, t + 96 of every 128), up to eight
+// loads in flight.
+template <typename L>
+__device__ __forceinline__ double warp_tile_sum_of(int ntile, L load) {
+  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+  int t = threadIdx.x & 31;
+  for (; t + 224 < ntile; t += 256) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = load(t + 32 * u);
+    s0 = (s0 + v[0]) + v[4];
+    s1 = (s1 + v[1]) + v[5];
+    s2 = (s2 + v[2]) + v[6];
+    s3 = (s3 + v[3]) + v[7];
+  }
+  for (; t + 96 < ntile; t += 128) {
+    double v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = load(t + 32 * u);
+    s0 += v[0];
+    s1 += v[1];
+    s2 += v[2];
+    s3 += v[3];
+  }
+  double v[3];  // the last up to three
+#pragma unroll
+  for (int u = 0; u < 3; ++u) v[u] = t + 32 * u < ntile ? load(t + 32 * u) : 0.0;
+  s0 = ((s0 + v[0]) + v[1]) + v[2];
+  double s = (s0 + s1) + (s2 + s3);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
 __device__ __forceinline__ void store_partial(const JobDev& J, double* slot, double v) {
   if (!J.mixed) {
     *slot = v;
