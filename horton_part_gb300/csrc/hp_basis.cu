@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_lisa_sc64(Batch bt) {
   const double* __restrict__ wv = J.w;
   double* old = J.oldpro ? J.oldpro + a * N : nullptr;
   const bool stored = old && J.oldok[(size_t)a * nt + tile] != 0;
-  const double cut = J.density_cutoff;
+  const f64::Cutoff cut = f64::cutoff_of(J.density_cutoff);
   const int p1 = min((tile + 1) * J.tile_points, J.npoint);
   with_rows(act.n, [&](auto na) {
     constexpr int NA = decltype(na)::value;
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_lisa_sc64(Batch bt) {
       double op = stored && !first ? old[p] : 0.0;
 #pragma unroll
       for (int j = 0; j < NA; ++j) pro = __fma_rn(c[j], gv[j], pro);
-      const bool sick = (rho < cut) || (pro < cut);
+      const bool sick = f64::below(rho, cut) || f64::below(pro, cut);
       const double wr = sick ? 0.0 : w * f64::div64(rho, sick ? 1.0 : pro);
 #pragma unroll
       for (int j = 0; j < NA; ++j) acc[j] = __fma_rn(gv[j], wr, acc[j]);

@@ -138,6 +138,23 @@ __device__ __forceinline__ double clip01(double x) {
   return b > 0x7ff0000000000000ll ? 0.0 : 1.0;
 }
 
+// x < cut by integer comparisons where cut > 0 (the FP64 pipe bounds the
+// kernels that test each point): the bits of a positive x below those of cut,
+// or the sign bit without a NaN. NaN is not below, as in the comparison.
+struct Cutoff {
+  double cut;
+  unsigned long long bits;
+  bool pos;
+};
+__device__ __forceinline__ Cutoff cutoff_of(double cut) {
+  return {cut, (unsigned long long)__double_as_longlong(cut), cut > 0.0};
+}
+__device__ __forceinline__ bool below(double x, const Cutoff& c) {
+  if (!c.pos) return x < c.cut;
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  return u < c.bits || (u ^ 0x8000000000000000ull) <= 0x7ff0000000000000ull;
+}
+
 // Block sums of nq <= Q per-thread values: the warps' values of a lane are
 // added first (from shared memory, warp q for quantity q), then the lanes,
 // which takes 12 warp-wide additions a quantity instead of 48. put(q, sum)

@@ -97,7 +97,7 @@ __device__ __forceinline__ void mbis_tile(const JobDev& J, int a, int tile, bool
   const double* rd = rd_row(J, a);
   double* old = J.oldpro ? J.oldpro + row : nullptr;
   const bool stored = old && J.oldok[a * J.ntile + tile] != 0;
-  const double cut = J.density_cutoff;
+  const f64::Cutoff cut = f64::cutoff_of(J.density_cutoff);
   const int p0 = tile * J.tile_points + threadIdx.x;
   const int p1 = min((tile + 1) * J.tile_points, J.npoint);
   // the next point's values are loaded while the current one is worked on
@@ -121,7 +121,7 @@ __device__ __forceinline__ void mbis_tile(const JobDev& J, int a, int tile, bool
       e[k] = f64::exp64(S[k] * r, tab);
       pro = __fma_rn(A[k], e[k], pro);
     }
-    const bool sick = (rho < cut) || (pro < cut);
+    const bool sick = f64::below(rho, cut) || f64::below(pro, cut);
     // (no quotient where sick: far from the atom pro underflows, and a zero
     // divisor takes the divide's slow path)
     const double wr = sick ? 0.0 : w * f64::div64(rho, sick ? 1.0 : pro);
@@ -199,7 +199,7 @@ __device__ __forceinline__ double* inner_partials(const JobDev& J, int a, int pa
 // about 30 FP64 instructions a pair at 1.5 shells, against ~150 when the
 // distance, the old pro-atom's exponentials, CUDA's exp and divide and the
 // sums of seven shells were all formed per pair. Two outer iterations of a
-// 22-atom chain of 320k points: 116.7 -> 32.6 ms.
+// 22-atom chain of 320k points: 116.7 -> 29.6 ms (85 % of the FP64 issue).
 __global__ void __launch_bounds__(kThreads, 3) k_mbis_inner64(Batch bt) {
   __shared__ double tab[f64::kExpTab];
   __shared__ double red[kQ * kThreads];
