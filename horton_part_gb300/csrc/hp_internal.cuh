@@ -217,6 +217,10 @@ struct JobDev {
   double* oldpro;         // MBIS, aLISA sc with G: pro-atoms of the last inner iteration
                           // [natom][npoint], or null; valid where oldok[natom][ntile] is set
   int* oldok;
+  // MBIS jobs of few tiles: packets (value, tag) of k_mbis_solve64
+  // [natom][2][spk_nq][ntile], or null
+  ulonglong2* spk;
+  int spk_nq;
   int* hsched;            // gLISA FP64, at most kH64Rows shells: schedule of k_glisa_hess64, or null:
                           // block b's units are entries [hsched[b], hsched[b + 1]) behind hbuf + 1 offsets
   int hbuf, hunit;        // its blocks (packed FP64 partial triangles in hpart), points per unit

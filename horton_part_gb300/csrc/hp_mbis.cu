@@ -12,6 +12,8 @@
 // without them recompute the same bits.
 #include <math.h>
 
+#include <atomic>
+
 #include "hp_inner.cuh"
 
 namespace hp {
@@ -77,11 +79,12 @@ __global__ void __launch_bounds__(kThreads) k_promol64(Batch bt) {
 // e_k (the update multiplies by A_k) and the change sum w (oldpro - pro)^2.
 // Per pair 12 FP64 instructions a shell (9 of the exponential) and 13 more.
 // amp[2 k], cur[2 k + 1], prev[2 k], prev[2 k + 1]: the atom's amplitudes,
-// exponents and previous parameters; out: the tile's partials, stride ntile.
-template <int NSH>
+// exponents and previous parameters; put(slot, v) stores the tile's partials
+// (slots 0 .. 2 NSH - 1 the moments, kQ - 1 the change).
+template <int NSH, typename Put>
 __device__ __forceinline__ void mbis_tile(const JobDev& J, int a, int tile, bool first,
                                           const double* amp, const double* cur, const double* prev,
-                                          const double* tab, double* red, double* out) {
+                                          const double* tab, double* red, Put put) {
   constexpr int NQ = 2 * NSH + 1;
   double A[NSH], S[NSH], acc[NQ];
 #pragma unroll
@@ -144,24 +147,22 @@ __device__ __forceinline__ void mbis_tile(const JobDev& J, int a, int tile, bool
     const double d = op - pro;
     acc[NQ - 1] = __fma_rn(w * d, d, acc[NQ - 1]);
   }
-  const int nt = J.ntile;
-  f64::block_sums<NQ>(acc, NQ, red, [&](int q, double v) {
-    out[(size_t)(q == NQ - 1 ? kQ - 1 : q) * nt] = v;
-  });
+  f64::block_sums<NQ>(acc, NQ, red, [&](int q, double v) { put(q == NQ - 1 ? kQ - 1 : q, v); });
   if (old && threadIdx.x == 0) J.oldok[a * J.ntile + tile] = 1;
 }
 
+template <typename Put>
 __device__ __forceinline__ void mbis_tile_n(int nsh, const JobDev& J, int a, int tile, bool first,
                                             const double* amp, const double* cur, const double* prev,
-                                            const double* tab, double* red, double* out) {
+                                            const double* tab, double* red, Put put) {
   switch (nsh) {
-    case 1: mbis_tile<1>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
-    case 2: mbis_tile<2>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
-    case 3: mbis_tile<3>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
-    case 4: mbis_tile<4>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
-    case 5: mbis_tile<5>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
-    case 6: mbis_tile<6>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
-    default: mbis_tile<7>(J, a, tile, first, amp, cur, prev, tab, red, out); break;
+    case 1: mbis_tile<1>(J, a, tile, first, amp, cur, prev, tab, red, put); break;
+    case 2: mbis_tile<2>(J, a, tile, first, amp, cur, prev, tab, red, put); break;
+    case 3: mbis_tile<3>(J, a, tile, first, amp, cur, prev, tab, red, put); break;
+    case 4: mbis_tile<4>(J, a, tile, first, amp, cur, prev, tab, red, put); break;
+    case 5: mbis_tile<5>(J, a, tile, first, amp, cur, prev, tab, red, put); break;
+    case 6: mbis_tile<6>(J, a, tile, first, amp, cur, prev, tab, red, put); break;
+    default: mbis_tile<7>(J, a, tile, first, amp, cur, prev, tab, red, put); break;
   }
 }
 
@@ -170,9 +171,10 @@ __device__ __forceinline__ void mbis_tile_n(int nsh, const JobDev& J, int a, int
 // tile's partials are zeroed and it is counted. One warp forms the bound: in
 // every thread it costs as much of the FP64 pipe as the tile itself. Uniform
 // over the block; skip_s: one int of shared memory.
+template <typename Put>
 __device__ __forceinline__ bool mbis_skip(const JobDev& J, int a, int tile, int nsh, bool first,
                                           const double* cur, const double* prev, const double* tab,
-                                          double* out, int* skip_s) {
+                                          Put put, int* skip_s) {
   if (!J.tgeo || !(J.amax[(size_t)a * J.ntile + tile] < (float)J.density_cutoff)) return false;
   if (threadIdx.x < 32) {
     const double b = f64::mbis_bound_warp(cur, first ? nullptr : prev, nsh, tile_rmin(J, a, tile), tab);
@@ -182,17 +184,13 @@ __device__ __forceinline__ bool mbis_skip(const JobDev& J, int a, int tile, int 
   const bool skip = *skip_s != 0;
   __syncthreads();
   if (!skip) return false;
-  if (threadIdx.x < 2 * nsh) out[(size_t)threadIdx.x * J.ntile] = 0.0;
+  if (threadIdx.x < 2 * nsh) put((int)threadIdx.x, 0.0);
   if (threadIdx.x == 0) {
-    out[(size_t)(kQ - 1) * J.ntile] = 0.0;
+    put(kQ - 1, 0.0);
     if (J.oldok) J.oldok[a * J.ntile + tile] = 0;
     count_skipped(J, tile, 1.0);
   }
   return true;
-}
-
-__device__ __forceinline__ double* inner_partials(const JobDev& J, int a, int parity) {
-  return J.apart + ((size_t)a * J.qa + QA_INNER + parity * kQ) * J.ntile;
 }
 
 // MBIS inner iteration, one block per (atom, tile). Bound by the FP64 pipe:
@@ -213,79 +211,152 @@ __global__ void __launch_bounds__(kThreads, 3) k_mbis_inner64(Batch bt) {
   const int s0 = J.shell_off[a], nsh = J.shell_off[a + 1] - s0;
   const bool first = J.inner_it[a] == 0;
   const double *amp = J.keep + 2 * s0, *cur = J.cur + 2 * s0, *prev = J.prev + 2 * s0;
-  double* out = inner_partials(J, a, 0) + tile;
-  if (!mbis_skip(J, a, tile, nsh, first, cur, prev, tab, out, &skip_s))
-    mbis_tile_n(nsh, J, a, tile, first, amp, cur, prev, tab, red, out);
+  double* out = J.apart + ((size_t)a * J.qa + QA_INNER) * J.ntile + tile;
+  const int nt = J.ntile;
+  auto put = [&](int slot, double v) { out[(size_t)slot * nt] = v; };
+  if (!mbis_skip(J, a, tile, nsh, first, cur, prev, tab, put, &skip_s))
+    mbis_tile_n(nsh, J, a, tile, first, amp, cur, prev, tab, red, put);
   if (last_block_of(J, a)) mbis_update(J, a);
 }
 
 // The whole inner solve of every atom in one launch, for batches small enough
 // that all blocks are resident (a cooperative launch): atom a's blocks (T
-// consecutive tiles each) go through its iterations together, meeting at a
-// counter per atom; each of them then sums the atom's partials in the order
-// of warp_tile_sum and forms the same new parameters, so nothing is handed
-// back. The partials alternate between two buffers: a block that is one
-// iteration ahead does not write what a slower one still reads. Bits as
-// k_mbis_inner64.
-// Water (3 atoms, 147 blocks) through the class: 21.1 -> 14.1 ms.
-// An iteration costs two L2 round trips beside the tiles' work instead of a
-// launch, cold instruction and data caches and an update at its end.
+// consecutive tiles each) go through its iterations together; each of them
+// sums the atom's partials in the order of warp_tile_sum and forms the same
+// new parameters, so nothing is handed back. Bits as k_mbis_inner64.
+//
+// Latency-bound: the partials travel as 16-byte packets (value, tag), written
+// and read as one access each, and a reader polls the packets themselves: one
+// L2 round trip an iteration instead of the four of a fence, a counter, its
+// poll and the partials, and no acquire that empties the L1 cache the tiles'
+// values are read from. The tag holds the launch's number and the iteration.
+// The packets alternate between two buffers: a block writes iteration i + 2
+// when it has read all packets of i + 1, whose writers had read those of i.
+//
+// FP64 issue is shared by the blocks of an SM, and the atoms with most shells
+// iterate longest: their blocks come last in the grid, where each has an SM
+// with a lighter one (first, the few SMs that are filled first held two of
+// the heaviest blocks, and every iteration waited for them).
+// Water (3 atoms, 291 blocks) through the class: 14.0 -> 11.4 ms
+// (counter and 512-point tiles before; 21.1 with a launch per iteration).
+//
 // The wait is bounded: a block that runs out of polls sets E_TIMEOUT and
 // ends, and so do the others, each by its own bound.
 constexpr int kSolvePolls = 1 << 20;
 
-__global__ void __launch_bounds__(kThreads, 2) k_mbis_solve64(Batch bt, int T) {
+__device__ __forceinline__ void put_packet(ulonglong2* p, double v, unsigned long long tag) {
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+      "l"(__double_as_longlong(v)), "l"(tag)
+      : "memory");
+}
+
+__device__ __forceinline__ double get_packet(const ulonglong2* p, unsigned long long& tag) {
+  long long v;
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+      : "=l"(v), "=l"(tag)
+      : "l"(p)
+      : "memory");
+  return __longlong_as_double(v);
+}
+
+// The warp's sum of ntile packets of this tag, in the order of
+// warp_tile_sum_of; waits for them (*late is set where they do not come).
+__device__ __forceinline__ double packet_sum(const ulonglong2* pk, int ntile, unsigned long long tag,
+                                             int* late) {
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int t = threadIdx.x & 31; t < ntile; t += 256) {
+    double v[8];
+    int polls = 0;
+    bool ok;
+    do {
+      ok = true;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        v[u] = 0.0;
+        if (t + 32 * u < ntile) {
+          unsigned long long g;
+          v[u] = get_packet(pk + t + 32 * u, g);
+          ok &= g == tag;
+        }
+      }
+    } while (!ok && ++polls < kSolvePolls);
+    if (!ok) *late = 1;
+#pragma unroll
+    for (int h = 0; h < 8; h += 4) {
+      if (t + 32 * h + 96 < ntile) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s[u] += v[h + u];
+      } else {  // the last up to three
+        s[0] = ((s[0] + v[h]) + v[h + 1]) + v[h + 2];
+      }
+    }
+  }
+  __syncwarp();
+  double y = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+  return y;
+}
+
+__global__ void __launch_bounds__(kThreads, 2) k_mbis_solve64(Batch bt, int T, unsigned seq) {
   __shared__ double tab[f64::kExpTab];
   __shared__ double red[kQ * kThreads];
   __shared__ double amp[2 * kMbisMaxShell], cur[2 * kMbisMaxShell], prev[2 * kMbisMaxShell];
   __shared__ double m[kQ];
-  __shared__ int skip_s, late_s, state_s;
+  __shared__ int skip_s, late_s, state_s, atom_s;
   int local;
   const JobDev& J = decode_local_mb(bt, local);
   f64::load_exp64(tab, J.etab);
-  const int nb = (J.ntile + T - 1) / T;  // blocks of an atom
-  const int a = local / nb, b = local - a * nb;
+  const int nt = J.ntile, natom = J.natom;
+  const int nb = (nt + T - 1) / T;  // blocks of an atom
+  const int b = local % nb;
+  {  // the (local / nb)-th atom by shell count
+    int* cnt = reinterpret_cast<int*>(red);
+    for (int i = threadIdx.x; i < natom; i += kThreads) cnt[i] = J.shell_off[i + 1] - J.shell_off[i];
+    __syncthreads();
+    for (int i = threadIdx.x; i < natom; i += kThreads) {
+      int rank = 0;
+      for (int k = 0; k < natom; ++k) rank += cnt[k] < cnt[i] || (cnt[k] == cnt[i] && k < i);
+      if (rank == local / nb) atom_s = i;
+    }
+    if (threadIdx.x == 0) late_s = 0;
+    __syncthreads();
+  }
+  const int a = atom_s;
   const int s0 = J.shell_off[a], nsh = J.shell_off[a + 1] - s0;
-  const int t0 = b * T, t1 = min(t0 + T, J.ntile);
+  const int t0 = b * T, t1 = min(t0 + T, nt);
   if (threadIdx.x < 2 * nsh) {
     amp[threadIdx.x] = J.keep[2 * s0 + threadIdx.x];
     cur[threadIdx.x] = prev[threadIdx.x] = J.cur[2 * s0 + threadIdx.x];
   }
-  if (threadIdx.x == 0) late_s = 0;
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int it = 0;; ++it) {
-    double* part = inner_partials(J, a, it & 1);
+    const unsigned long long tag = ((unsigned long long)seq << 32) | (unsigned)(it + 1);
+    ulonglong2* pk = J.spk + (size_t)(2 * a + (it & 1)) * J.spk_nq * nt;
     for (int tile = t0; tile < t1; ++tile) {
-      if (!mbis_skip(J, a, tile, nsh, it == 0, cur, prev, tab, part + tile, &skip_s))
-        mbis_tile_n(nsh, J, a, tile, it == 0, amp, cur, prev, tab, red, part + tile);
-      __syncthreads();  // red, and this block's partials are written
+      auto put = [&](int slot, double v) {
+        put_packet(pk + (size_t)(slot == kQ - 1 ? 2 * nsh : slot) * nt + tile, v, tag);
+      };
+      if (!mbis_skip(J, a, tile, nsh, it == 0, cur, prev, tab, put, &skip_s))
+        mbis_tile_n(nsh, J, a, tile, it == 0, amp, cur, prev, tab, red, put);
+      if (tile + 1 < t1) __syncthreads();  // red
     }
-    if (threadIdx.x == 0) {
-      __threadfence();
-      atomicAdd(&J.arrive[a], 1);
-      const int target = (it + 1) * nb;
-      int polls = 0, seen;
-      do {
-        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(J.arrive + a) : "memory");
-      } while (seen < target && ++polls < kSolvePolls);
-      if (seen < target) late_s = 1;
+    for (int q = warp; q < 2 * nsh + 1; q += kWarps) {
+      const double v = packet_sum(pk + (size_t)q * nt, nt, tag, &late_s);
+      if (lane == 0) m[q] = v;
     }
     __syncthreads();
     if (late_s) {
       if (threadIdx.x == 0) atomicOr(&J.mail->i[MI_ERR], E_TIMEOUT);
       return;
     }
-    for (int q = warp; q < 2 * nsh + 1; q += kWarps) {
-      const double v = warp_tile_sum_cg(J, part + (size_t)(q == 2 * nsh ? kQ - 1 : q) * J.ntile, J.ntile);
-      if (lane == 0) m[q] = v;
-    }
-    __syncthreads();
     // the update (mbis_update): the parameters on warp 0, the test on warp 1
-    double n = 0.0, s = 0.0;
     if (threadIdx.x < nsh) {
-      n = amp[2 * threadIdx.x] * m[2 * threadIdx.x];
-      s = 3.0 * m[2 * threadIdx.x] / m[2 * threadIdx.x + 1];
+      const double n = amp[2 * threadIdx.x] * m[2 * threadIdx.x];
+      const double s = 3.0 * m[2 * threadIdx.x] / m[2 * threadIdx.x + 1];
       prev[2 * threadIdx.x] = cur[2 * threadIdx.x];
       prev[2 * threadIdx.x + 1] = cur[2 * threadIdx.x + 1];
       cur[2 * threadIdx.x] = n;
@@ -418,7 +489,11 @@ int mbis_solve_capacity() {
 void launch_mbis_solve64(const HostBatch& hb, cudaStream_t st) {
   Batch bt = hb.b[K_SOLVE];
   int T = hb.solve_tiles;
-  void* args[] = {&bt, &T};
+  // launches are numbered (packet tags), from 1: the packets start as zeros
+  static std::atomic<unsigned> launches{0};
+  unsigned seq = ++launches;
+  if (seq == 0) seq = ++launches;
+  void* args[] = {&bt, &T, &seq};
   cudaLaunchCooperativeKernel((void*)k_mbis_solve64, dim3((unsigned)hb.blocks[K_SOLVE]), dim3(kThreads), args, 0, st);
   ++g_launch_count;
 }

@@ -147,6 +147,7 @@ void drop_kept(hp_job* j) {
   j->dev.rd = nullptr;
   j->dev.oldpro = nullptr;
   j->dev.oldok = nullptr;
+  j->dev.spk = nullptr;
 }
 
 // Whether the budget has room for `bytes`: jobs give back what they only
@@ -168,6 +169,12 @@ cudaError_t job_alloc_retry(hp_ctx* ctx, void** p, size_t bytes) {
   return job_alloc(ctx, p, bytes);
 }
 
+constexpr int kSolveTiles = 4;  // tiles per block of k_mbis_solve64 at most (solve_tiles)
+
+int solve_blocks(const JobDev& J, int tiles) {
+  return tiles > 0 ? J.natom * ((J.ntile + tiles - 1) / tiles) : 0;
+}
+
 // FP64 jobs: storage for the pair distances (MBIS) and, on the molecular
 // grid, the pro-atoms of the last inner iteration (MBIS, aLISA sc with a
 // stored G), where it takes at most half of what is left of the budget.
@@ -178,7 +185,11 @@ void alloc_kept(hp_ctx* ctx, hp_job* j) {
   if (!mbis && !lisa) return;
   const bool old = !J.local;
   const size_t pair = align_up(8 * (size_t)J.natom * (size_t)J.npoint);
-  const size_t bytes = (mbis ? pair : 0) + (old ? pair + align_up(4 * (size_t)J.natom * J.ntile) : 0);
+  // packets of the one-launch inner solve, for jobs that can take it
+  const bool solve = mbis && old && solve_blocks(J, kSolveTiles) <= mbis_solve_capacity();
+  const size_t packets = solve ? 16 * (size_t)J.natom * 2 * J.spk_nq * J.ntile : 0;
+  const size_t flags = align_up(4 * (size_t)J.natom * J.ntile);
+  const size_t bytes = (mbis ? pair : 0) + (old ? pair + flags : 0) + align_up(packets);
   const size_t room = ctx->budget > ctx->used ? ctx->budget - ctx->used : 0;
   if (bytes > room / 2) return;
   void* mem = nullptr;
@@ -199,6 +210,11 @@ void alloc_kept(hp_ctx* ctx, hp_job* j) {
   if (old) {
     J.oldpro = reinterpret_cast<double*>(at);
     J.oldok = reinterpret_cast<int*>(at + pair);
+    at += pair + flags;
+  }
+  if (solve) {
+    cudaMemsetAsync(at, 0, packets, ctx->stream);
+    J.spk = reinterpret_cast<ulonglong2*>(at);
   }
 }
 
@@ -294,15 +310,11 @@ int blocks_for(const JobDev& J, int kind) {
 // fewest with which a batch's blocks are all resident, at most kSolveTiles
 // (0: one launch per inner iteration). With more tiles a block the launches
 // it saves count for little, and atoms that are done leave their blocks idle.
-constexpr int kSolveTiles = 4;
-
-int solve_blocks(const JobDev& J, int tiles) {
-  return tiles > 0 ? J.natom * ((J.ntile + tiles - 1) / tiles) : 0;
-}
-
 int solve_tiles(const std::vector<hp_job*>& jobs) {
   const JobDev& J0 = jobs[0]->dev;
   if (J0.scheme != SCHEME_MBIS || J0.mixed || J0.local) return 0;
+  for (const hp_job* j : jobs)
+    if (!j->dev.spk) return 0;
   const int cap = mbis_solve_capacity();
   for (int t = 1; t <= kSolveTiles; ++t) {
     int64_t blocks = 0;
@@ -1247,7 +1259,12 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   // tiles: aim for >= 2 * 152 point tiles when the grid is large enough
   // (mixed precision: at least 4 points per thread so the per-block
   // compensated reductions are amortised)
-  const int ppt_min = d->precision != HP_PRECISION_FP64 && !glisa ? 4 : 2;
+  // Small MBIS jobs: one point per thread while all (atom, tile) blocks of
+  // k_mbis_solve64 stay resident, two on an SM: a block of a heavy atom then
+  // shares its SM with a light one (water: 24 -> 18 thousand cycles an
+  // iteration; with 512 points a block has the FP64 work of two).
+  int ppt_min = d->precision != HP_PRECISION_FP64 && !glisa ? 4 : 2;
+  if (mbis && d->precision == HP_PRECISION_FP64 && (int64_t)A * ((N + kThreads - 1) / kThreads) <= 2 * 152) ppt_min = 1;
   // gLISA's passes over G keep one point tile per block: aim for 4 blocks per SM
   const int64_t tiles_target = glisa ? 4 * 152 : 2 * 152;
   int ppt = (int)std::min<int64_t>(
@@ -1255,7 +1272,6 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   const int tile_points = kThreads * ppt;
   const int ntile = (N + tile_points - 1) / tile_points;
   int qa = 2 + std::max(2 * 7 + 1, kMaxShells + 1);
-  if (mbis && d->precision == HP_PRECISION_FP64) qa = 2 + 2 * (2 * kMbisMaxShell + 1);  // k_mbis_solve64
   if (d->scheme == HP_SCHEME_LISA && solver != HP_SOLVER_SC) qa = 2 + kNewtonQ(kmax);
   const int maxiter = d->maxiter;
   // gLISA keeps FP64 evaluation; its mixed mode is the tensor-core Hessian
@@ -1437,6 +1453,7 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   J.mixed = !mixed ? PH_FP64 : d->precision == HP_PRECISION_FF ? PH_FF : PH_FP32;
   J.inner_maxiter = d->inner_maxiter > 0 ? d->inner_maxiter : 2000;
   J.linspace_size = d->linspace_size > 0 ? d->linspace_size : (glisa ? 40 : 20);
+  J.spk_nq = 2 * kmax + 1;
   J.nsplit = nsplit; J.ppt = ppt; J.tile_points = tile_points; J.htiles = htiles;
   J.tc = tc ? 1 : 0;
   J.gff = gff ? 1 : 0;

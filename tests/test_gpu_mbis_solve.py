@@ -1,9 +1,10 @@
-"""The cutoff test of the FP64 inner kernels at the ends of its range."""
+"""The one-launch MBIS inner solve at its tile edges, and the cutoff test of
+the FP64 inner kernels at the ends of its range."""
 
 import numpy as np
 import pytest
 
-from horton_part_gb300 import _lib
+from horton_part_gb300 import _lib, synthetic
 from horton_part_gb300.mbis import get_initial_mbis_propars, get_nshell
 from horton_part_gb300.molgrid import MolecularGrid, becke_molecular_grid
 from oracle import hp_oracle as O
@@ -31,6 +32,27 @@ def _job(ctx, coords, numbers, grid, rho, **kw):
     return _lib.Job(ctx, "mbis", coords, numbers.astype(float), grid.points, grid.weights, rho,
                     np.concatenate([[0], np.cumsum(nsh)]).astype(np.int32),
                     np.concatenate([get_initial_mbis_propars(z) for z in numbers]), **args)
+
+
+# 256-point tiles up to 2 x 152 blocks of two atoms (38912 points), 512-point
+# tiles from there on, two tiles a block and more than 256 tiles at 140000
+@pytest.mark.parametrize("npoint", [1, 257, 38912, 38913, 140000])
+def test_same_bits_as_a_launch_per_iteration(npoint, gpu_context):
+    small = _hydride(8, 240, 302, npoint)
+    mol = synthetic.chain_molecule({6: 14, 1: 18}, 60, 194, seed=9)
+    results = []
+    for others in (False, True):
+        jobs = [_job(gpu_context, *small)]
+        if others:  # more blocks than are resident: a launch per inner iteration
+            jobs.append(_job(gpu_context, mol.coordinates, mol.numbers, mol.grid, mol.density))
+        for _ in range(2):
+            gpu_context.step(jobs)
+        results.append((jobs[0].results(at_weights=True), jobs[0].info().inner_iterations))
+        for j in jobs:
+            j.close()
+    assert results[0][1] == results[1][1]
+    for key in results[0][0]:
+        np.testing.assert_array_equal(results[0][0][key], results[1][0][key])
 
 
 @pytest.mark.parametrize("cutoff", [-1.0, 0.0, 1e-3])
