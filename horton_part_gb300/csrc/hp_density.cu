@@ -4,7 +4,9 @@
 // FP64 on the GPU.
 //
 // One block per tile of T consecutive points (T chosen by the host so that
-// the tile's basis values fit in shared memory, at most kDensTile):
+// the tile's basis values fit in shared memory, at most kDensTile; two blocks
+// a tile where that leaves SMs idle, each with half of the tile's points and
+// all of its significant shells):
 //  1. the tile's bounding box; a shell is skipped for the whole tile when
 //     a_min d_min^2 > kDensExpCut (a_min its smallest exponent, d_min the
 //     distance from its centre to the box), i.e. every primitive is below
@@ -20,12 +22,13 @@
 //  3. rho(p) = sum_a phi_a (D_aa phi_a + 2 sum_{b<a} D_ab phi_b) for every
 //     density matrix (total, spin, ...): the block's threads split as
 //     (point, a-slice), rows a = slice, slice + S, ... in order, and the
-//     slices' sums are added in slice order.
+//     slices' sums are added in a fixed tree.
 // The arithmetic is FP64 throughout; the cost is the FP64 issue rate of
 // phase 3 (n_sig^2 / 2 FMA per point and matrix, near the rate of a cuBLAS
 // FP64 product) and of the exponentials (hp_fp64.cuh: 11 instructions a
 // primitive; CUDA's exp and a distance per shell took 15 % of the time).
-// 604,000 points, 190 functions: 15.0 -> 13.4 ms.
+// 604,000 points, 190 functions: 15.0 -> 12.5 ms (11.9 ms are the contraction's
+// FMAs).
 //
 // A low-rank factor D = L L^T (n_sig x n_occ products instead) was measured
 // at 8.4 ms and not kept: it holds only for matrices formed from orbitals
@@ -108,8 +111,11 @@ __device__ __forceinline__ void shell_out(bool pure, double rad, double x, doubl
 
 // Basis values of one shell at one point (phase 2): x, y, z from its centre,
 // r2 their squared length; zeros for a lane without a point (live false).
-// All lanes of the warp, one shell.
-__device__ __forceinline__ void shell_values(const DensityArgs& a, int s, double x, double y, double z,
+// All lanes of the warp, one shell. Not inlined: one copy of the exponential
+// and of the components instead of one per call site keeps the kernel in the
+// instruction cache (13.6 -> 12.5 ms on 604,000 points; on 4,500 points, where
+// every line is fetched once, phase 2 takes 13 instead of 26 thousand cycles).
+static __device__ __noinline__ void shell_values(const DensityArgs& a, int s, double x, double y, double z,
                                              double r2, float r2f, double* out, int T, const double* tab,
                                              bool live, bool write) {
   const int l = a.info[5 * s];
@@ -138,7 +144,14 @@ __global__ void __launch_bounds__(kDensThreadsMax) k_density(DensityArgs a) {
   extern __shared__ double dsm[];
   __shared__ double box[6];
   __shared__ int wcnt[kDensThreadsMax / 32], wfun[kDensThreadsMax / 32];
-  const int T = a.tile;
+  // the block's points: one of the nsub parts of a tile
+  const int T = a.tile / a.nsub;
+  const int64_t q0 = (int64_t)(blockIdx.x / a.nsub) * a.tile;
+  const int part = blockIdx.x % a.nsub;
+  const int nq = (int)min((int64_t)a.tile, a.npoint - q0);
+  const int64_t p0 = q0 + (int64_t)part * T;
+  const int np = min(T, nq - part * T);
+  if (np <= 0) return;
   const int NT = blockDim.x, NW = NT >> 5;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double* phi = dsm;
@@ -146,15 +159,13 @@ __global__ void __launch_bounds__(kDensThreadsMax) k_density(DensityArgs a) {
   double* tab = slice + NT;
   int* fidx = reinterpret_cast<int*>(tab + f64::kExpTab);
   int* loc = fidx + a.nbasis;
-  const int64_t p0 = (int64_t)blockIdx.x * T;
-  const int np = (int)min((int64_t)T, a.npoint - p0);
   f64::load_exp64(tab, a.etab);
   // 1. bounding box of the tile (a warp per coordinate) and the significant
   // shells (in shell order)
   if (warp < 3) {
     double vmin = INFINITY, vmax = -INFINITY;
-    for (int i = lane; i < np; i += 32) {
-      const double v = a.points[(p0 + i) * 3 + warp];
+    for (int i = lane; i < nq; i += 32) {
+      const double v = a.points[(q0 + i) * 3 + warp];
       vmin = fmin(vmin, v);
       vmax = fmax(vmax, v);
     }
@@ -198,7 +209,8 @@ __global__ void __launch_bounds__(kDensThreadsMax) k_density(DensityArgs a) {
     }
     __syncthreads();
     int fo = nf, st = ns, ft = nf;
-    for (int w = 0; w < NW; ++w) {
+    const int nw = min(NW, (a.nshell - base + 31) / 32);  // the warps with a shell
+    for (int w = 0; w < nw; ++w) {
       if (w < warp) fo += wfun[w];
       st += wcnt[w];
       ft += wfun[w];
@@ -213,19 +225,20 @@ __global__ void __launch_bounds__(kDensThreadsMax) k_density(DensityArgs a) {
     ns = st;
     nf = ft;
   }
-  if (a.stats && threadIdx.x == 0) {
-    const unsigned long long nn = (unsigned long long)np;
+  if (a.stats && threadIdx.x == 0 && part == 0) {
+    const unsigned long long nn = (unsigned long long)nq;
     atomicAdd(&a.stats[0], (unsigned long long)ns);
     atomicAdd(&a.stats[1], (unsigned long long)nf * nn);
     atomicAdd(&a.stats[2], (unsigned long long)nf * (unsigned long long)(nf + 1) / 2ull * nn);
   }
   // 2. basis values of the significant shells (zero past the last point): a
   // warp per (group of shells with one centre, 32 points; fewer for a tile
-  // of 8 or 16)
+  // of 8 or 16); per shell where the groups leave most warps idle
   const int npw = min(T, 32), nchunk = T / npw;
-  for (int e = warp; e < a.ngroup * nchunk; e += NW) {
+  const bool single = 2 * a.ngroup * nchunk <= NW;
+  for (int e = warp; e < (single ? a.nshell : a.ngroup) * nchunk; e += NW) {
     const int g = e / nchunk, i = (e - g * nchunk) * npw + (lane & (npw - 1));
-    const int sa = a.groups[g], sb = a.groups[g + 1];
+    const int sa = single ? g : a.groups[g], sb = single ? g + 1 : a.groups[g + 1];
     const int64_t p = p0 + min(i, np - 1);
     const double x = a.points[p * 3] - a.centers[3 * sa];
     const double y = a.points[p * 3 + 1] - a.centers[3 * sa + 1];
@@ -252,11 +265,11 @@ __global__ void __launch_bounds__(kDensThreadsMax) k_density(DensityArgs a) {
     }
     slice[threadIdx.x] = acc;
     __syncthreads();
-    if (q == 0 && i < np) {
-      double r = 0.0;
-      for (int k = 0; k < S; ++k) r += slice[k * T + i];
-      a.out[(size_t)mat * a.npoint + p0 + i] = r;
+    for (int h = S / 2; h > 0; h /= 2) {  // (S is a power of two)
+      if (q < h) slice[threadIdx.x] += slice[threadIdx.x + h * T];
+      __syncthreads();
     }
+    if (q == 0 && i < np) a.out[(size_t)mat * a.npoint + p0 + i] = slice[i];
     __syncthreads();
   }
 }
@@ -290,10 +303,15 @@ void launch_density(const DensityArgs& a, cudaStream_t st) {
   }
   const int64_t nblk = (a.npoint + a.tile - 1) / a.tile;
   if (nblk <= 0) return;
+  DensityArgs b = a;
+  b.nsub = 2 * nblk <= 152 && a.tile == 64 ? 2 : 1;
   // fewer tiles than SMs: four times the slices, so that a tile's time is not
-  // that of eight warps (water, 4,500 points: 68.5 -> 67.1 us a call from host arrays)
+  // that of eight warps, and half a tile a block while all blocks have an SM
+  // (water, 4,500 points: 35.4 -> 29.1 us by the halves, 23.5 with phase 2 out
+  // of line)
   const int threads = nblk <= 152 ? kDensThreadsMax : kDensThreads;
-  k_density<<<(unsigned)nblk, threads, density_smem_bytes(a.nbasis, a.nshell, a.tile, threads), st>>>(a);
+  const size_t smem = density_smem_bytes(a.nbasis, a.nshell, a.tile / b.nsub, threads);
+  k_density<<<(unsigned)(nblk * b.nsub), threads, smem, st>>>(b);
   ++g_launch_count;
 }
 

@@ -726,6 +726,7 @@ struct DensityArgs {
   const double* points;  // [npoint][3]
   int64_t npoint;
   int nshell, nbasis, nmat, tile;
+  int nsub;  // blocks per tile (launch_density)
   const double* centers;  // [nshell][3]
   const int* info;        // [nshell][5]: l, pure, nprim, first primitive, first function
   const double* amin;     // [nshell] smallest exponent of the shell
