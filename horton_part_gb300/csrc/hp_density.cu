@@ -143,6 +143,7 @@ static __device__ __noinline__ void shell_values(const DensityArgs& a, int s, do
 __global__ void __launch_bounds__(kDensThreadsMax) k_density(DensityArgs a) {
   extern __shared__ double dsm[];
   __shared__ double box[6];
+  __shared__ double pt[3 * kDensTile];  // the tile's points
   __shared__ int wcnt[kDensThreadsMax / 32], wfun[kDensThreadsMax / 32];
   // the block's points: one of the nsub parts of a tile
   const int T = a.tile / a.nsub;
@@ -159,13 +160,15 @@ __global__ void __launch_bounds__(kDensThreadsMax) k_density(DensityArgs a) {
   double* tab = slice + NT;
   int* fidx = reinterpret_cast<int*>(tab + f64::kExpTab);
   int* loc = fidx + a.nbasis;
+  for (int i = threadIdx.x; i < 3 * nq; i += NT) pt[i] = a.points[q0 * 3 + i];
   f64::load_exp64(tab, a.etab);
+  __syncthreads();
   // 1. bounding box of the tile (a warp per coordinate) and the significant
   // shells (in shell order)
   if (warp < 3) {
     double vmin = INFINITY, vmax = -INFINITY;
     for (int i = lane; i < nq; i += 32) {
-      const double v = a.points[(q0 + i) * 3 + warp];
+      const double v = pt[3 * i + warp];
       vmin = fmin(vmin, v);
       vmax = fmax(vmax, v);
     }
@@ -239,10 +242,10 @@ __global__ void __launch_bounds__(kDensThreadsMax) k_density(DensityArgs a) {
   for (int e = warp; e < (single ? a.nshell : a.ngroup) * nchunk; e += NW) {
     const int g = e / nchunk, i = (e - g * nchunk) * npw + (lane & (npw - 1));
     const int sa = single ? g : a.groups[g], sb = single ? g + 1 : a.groups[g + 1];
-    const int64_t p = p0 + min(i, np - 1);
-    const double x = a.points[p * 3] - a.centers[3 * sa];
-    const double y = a.points[p * 3 + 1] - a.centers[3 * sa + 1];
-    const double z = a.points[p * 3 + 2] - a.centers[3 * sa + 2];
+    const double* pp = pt + 3 * (part * T + min(i, np - 1));
+    const double x = pp[0] - a.centers[3 * sa];
+    const double y = pp[1] - a.centers[3 * sa + 1];
+    const double z = pp[2] - a.centers[3 * sa + 2];
     const double r2 = x * x + y * y + z * z;
     const float r2f = (float)r2;
     for (int s = sa; s < sb; ++s)
