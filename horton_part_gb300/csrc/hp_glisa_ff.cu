@@ -1199,7 +1199,7 @@ __global__ void __launch_bounds__(kThreads) k_glisa_wgram(Batch bt) {
   const int M = J.nshell;
   const size_t tri = (size_t)M * (M + 1) / 2;
   const float* hp = reinterpret_cast<const float*>(J.hpart);
-  const int nblk = (M * M + kThreads - 1) / kThreads;  // this job's K_SQUARE blocks
+  const int nblk = square_blocks(M);
   for (int e = local * kWarps + warp; e < J.wgn; e += nblk * kWarps) {
     int lo = 0, hi = J.natom;  // the atom a with wgoff[a] <= e < wgoff[a + 1]
     while (hi - lo > 1) {
@@ -1214,18 +1214,7 @@ __global__ void __launch_bounds__(kThreads) k_glisa_wgram(Batch bt) {
     const int j = q - i * (i + 1) / 2;
     const int gi = J.shell_off[lo] + i, gj = J.shell_off[lo] + j;
     const size_t t = (size_t)gi * (gi + 1) / 2 + gj;
-    double h0 = 0.0, h1 = 0.0, h2 = 0.0, h3 = 0.0;
-    int sp = lane;
-    for (; sp + 96 < J.nsplit; sp += 128) {
-      h0 += hp[(size_t)sp * tri + t];
-      h1 += hp[(size_t)(sp + 32) * tri + t];
-      h2 += hp[(size_t)(sp + 64) * tri + t];
-      h3 += hp[(size_t)(sp + 96) * tri + t];
-    }
-    for (; sp < J.nsplit; sp += 32) h0 += hp[(size_t)sp * tri + t];
-    double h = (h0 + h1) + (h2 + h3);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
+    const double h = warp_tile_sum_of(J.nsplit, [&](int sp) { return (double)hp[(size_t)sp * tri + t]; });
     if (lane == 0) J.wgram[e] = h;
   }
 }

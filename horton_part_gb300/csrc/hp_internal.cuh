@@ -561,6 +561,16 @@ __device__ __forceinline__ double nlis_rn(double n, double r) {
 
 namespace hp {
 
+// Blocks of kind K_SQUARE of a job with M shells: at least one per kThreads
+// elements of an M x M matrix, and for the reductions over many partials a
+// block per SM where that leaves 64 elements a block (141 shells: 78 blocks
+// had half of the SMs).
+__host__ __device__ constexpr int square_blocks(int M) {
+  const int full = (M * M + kThreads - 1) / kThreads, fine = (M * M + 63) / 64;
+  const int chip = fine < 152 ? fine : 152;
+  return full > chip ? full : chip;
+}
+
 // Launch kinds: blocks per job for each kind of work.
 enum Kind {
   K_POINT = 0,      // one block per point tile
@@ -569,7 +579,7 @@ enum Kind {
   K_ATOM = 2,       // one 32-thread block per atom
   K_JOB = 3,        // one block per job
   K_HESS = 4,       // gLISA Hessian: (tile pair, point split)
-  K_SQUARE = 5,     // gLISA reduce: ceil(nshell^2 / kThreads)
+  K_SQUARE = 5,     // gLISA reduce: square_blocks(nshell)
   K_FUSE = 7,       // fused gLISA pass: min(ntile, kFuseCtas) persistent blocks per job
   K_SOLVE = 8,      // whole inner solve: natom * ceil(ntile / solve_tiles), all resident
   K_NKIND = 9

@@ -1210,7 +1210,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_glisa_reduce(Batch bt) {
   const int M = J.nshell;
   const int e = local * kReduceThreads + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nblk = (M * M + kThreads - 1) / kThreads;  // this job's K_SQUARE blocks
+  const int nblk = square_blocks(M);
   if (J.tc && M <= kTcSinglePassShells) {
     // FP32 packed lower triangles of the single-pass tensor-core kernels.
     // The triangle's E elements form chunks of 32 (lane = element); the block
@@ -1322,21 +1322,10 @@ __global__ void __launch_bounds__(kReduceThreads) k_glisa_reduce(Batch bt) {
       J.hess[(size_t)j * M + i] = s;
     }
   }
-  // gradient rows: one warp per row, lanes over tiles (four chains, fixed order)
-  for (int m = local * kReduceWarps + warp; m < M; m += nblk * kReduceWarps) {
+  // gradient rows: one warp per row, neighbouring rows on different SMs
+  for (int m = warp * nblk + local; m < M; m += nblk * kReduceWarps) {
     const double* gp = J.gpart + (size_t)m * J.ntile;
-    double h0 = 0.0, h1 = 0.0, h2 = 0.0, h3 = 0.0;
-    int t = lane;
-    for (; t + 96 < J.ntile; t += 128) {
-      h0 += gp[t];
-      h1 += gp[t + 32];
-      h2 += gp[t + 64];
-      h3 += gp[t + 96];
-    }
-    for (; t < J.ntile; t += 32) h0 += gp[t];
-    double h = (h0 + h1) + (h2 + h3);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
+    const double h = warp_tile_sum_of(J.ntile, [&](int t) { return gp[t]; });
     if (lane == 0) J.grad[m] = -h;  // df_i = -int rho g_i / rho0 (glisa.py:452-455)
   }
 }
@@ -2129,21 +2118,10 @@ __global__ void __launch_bounds__(kThreads) k_glisa_gsum(Batch bt) {
   if (glisa_idle(J)) return;
   if (!glisa_refine_now(J)) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nblk = (J.nshell * J.nshell + kThreads - 1) / kThreads;  // this job's K_SQUARE blocks
-  for (int m = local * kWarps + warp; m < J.nshell; m += nblk * kWarps) {
+  const int nblk = square_blocks(J.nshell);
+  for (int m = warp * nblk + local; m < J.nshell; m += nblk * kWarps) {
     const double* gp = J.gpart + (size_t)m * J.ntile;
-    double h0 = 0.0, h1 = 0.0, h2 = 0.0, h3 = 0.0;
-    int t = lane;
-    for (; t + 96 < J.ntile; t += 128) {
-      h0 += gp[t];
-      h1 += gp[t + 32];
-      h2 += gp[t + 64];
-      h3 += gp[t + 96];
-    }
-    for (; t < J.ntile; t += 32) h0 += gp[t];
-    double h = (h0 + h1) + (h2 + h3);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
+    const double h = warp_tile_sum_of(J.ntile, [&](int t) { return gp[t]; });
     if (lane == 0) J.hsum[m] = h;
   }
 }
@@ -2199,55 +2177,74 @@ __global__ void __launch_bounds__(kThreads) k_glisa_refine(Batch bt) {
 // Projected-Newton trial points c_t = max(c + 2^-t delta, 0), t < kTrials,
 // and the list of shells the projection clips at the full step (the clipped
 // set of every shorter step is a subset of it). A block of NT threads (tms:
-// kTrialSetSmem ints of shared memory, wcount: NT / 32).
+// kTrialSetSmem ints of shared memory, wcount: kTrials kTrialSetSmem / 32).
 constexpr int kTrialSetSmem = 2048;  // shells whose clip steps are sorted in shared memory
+
+// 2^-t
+__device__ __forceinline__ double trial_step(int t) { return __hiloint2double((1023 - t) << 20, 0); }
 
 template <int NT>
 __device__ void trial_set_body(const JobDev& J, int* tms, int* wcount) {
   const int M = J.nshell;
   for (int e = threadIdx.x; e < kTrials * M; e += NT) {
     const int t = e / M, m = e - t * M;
-    const double a = ldexp(1.0, -t);
+    const double a = trial_step(t);
     J.ctrial[e] = fmax(J.propars[m] + a * J.delta[m], 0.0);
   }
   // clipped shells with the number of trials t_m at which they are clipped
   // (c + 2^-t delta < 0 for t < t_m), sorted by t_m, largest first, shells
   // of equal t_m in index order
   int* tm = J.clip + M + 1;
-  if (M <= kTrialSetSmem) {  // all threads: t_m per shell, then one ballot compaction per t
+  if (M <= kTrialSetSmem) {
+    // all threads: t_m per shell; the counts of every (t, warp of shells),
+    // their prefix sums (t descending) on one warp, then the positions
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int m = threadIdx.x; m < M; m += NT) {
+    const int nc = (M + 31) / 32;  // warps of shells
+    for (int m0 = warp * 32; m0 < M; m0 += NT) {
+      const int m = m0 + lane;
       int t = 0;
-      if (J.propars[m] + J.delta[m] < 0.0) {
-        t = 1;
-        while (t < kTrials && J.propars[m] + ldexp(1.0, -t) * J.delta[m] < 0.0) ++t;
+      if (m < M) {
+        const double c = J.propars[m], d = J.delta[m];
+        if (c + d < 0.0) {
+          t = 1;
+          while (t < kTrials && c + trial_step(t) * d < 0.0) ++t;
+        }
+        tms[m] = t;
       }
-      tms[m] = t;
+#pragma unroll
+      for (int k = 1; k <= kTrials; ++k) {
+        const unsigned b = __ballot_sync(0xffffffffu, t == k);
+        if (lane == 0) wcount[(kTrials - k) * nc + (m0 >> 5)] = __popc(b);
+      }
     }
     __syncthreads();
-    int n = 0;
-    for (int t = kTrials; t >= 1; --t) {
-      for (int base = 0; base < M; base += NT) {
-        const int m = base + threadIdx.x;
-        const bool f = m < M && tms[m] == t;
-        const unsigned b = __ballot_sync(0xffffffffu, f);
-        if (lane == 0) wcount[warp] = __popc(b);
-        __syncthreads();
-        int off = n, total = n;
-        for (int w = 0; w < NT / 32; ++w) {
-          if (w < warp) off += wcount[w];
-          total += wcount[w];
+    if (warp == 0) {  // exclusive prefix sums in place
+      int n = 0;
+      for (int e0 = 0; e0 < kTrials * nc; e0 += 32) {
+        const int e = e0 + lane;
+        const int own = e < kTrials * nc ? wcount[e] : 0;
+        int x = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, x, o);
+          if (lane >= o) x += y;
         }
-        if (f) {
-          const int k = off + __popc(b & ((1u << lane) - 1u));
-          J.clip[k] = m;
-          tm[k] = t;
-        }
-        __syncthreads();
-        n = total;
+        if (e < kTrials * nc) wcount[e] = n + x - own;
+        n += __shfl_sync(0xffffffffu, x, 31);
+      }
+      if (lane == 0) J.clip[M] = n;
+    }
+    __syncthreads();
+    for (int m0 = warp * 32; m0 < M; m0 += NT) {
+      const int m = m0 + lane;
+      const int t = m < M ? tms[m] : 0;
+      const unsigned same = __match_any_sync(0xffffffffu, t);
+      if (t > 0) {
+        const int k = wcount[(kTrials - t) * nc + (m0 >> 5)] + __popc(same & ((1u << lane) - 1u));
+        J.clip[k] = m;
+        tm[k] = t;
       }
     }
-    if (threadIdx.x == 0) J.clip[M] = n;
   } else if (threadIdx.x == 0) {
     int n = 0;
     for (int m = 0; m < M; ++m) {
@@ -2282,7 +2279,7 @@ __device__ void trial_set_body(const JobDev& J, int* tms, int* wcount) {
 
 __global__ void __launch_bounds__(kThreads) k_glisa_trial_set(Batch bt) {
   __shared__ int tms[kTrialSetSmem];
-  __shared__ int wcount[kWarps];
+  __shared__ int wcount[kTrials * kTrialSetSmem / 32];
   int local;
   const JobDev& J = decode_local(bt, local);
   if (glisa_idle(J)) return;
@@ -2510,14 +2507,20 @@ __global__ void __launch_bounds__(32 * kTrials) k_glisa_trial_pick(Batch bt) {
   if (glisa_idle(J)) return;
   const int lane = threadIdx.x & 31, t = threadIdx.x >> 5;
   const int M = J.nshell;
+  if (J.fuse)  // the entropy and negativity partials of the pass at the step's start
+    for (int q = threadIdx.x; q < J.ntile; q += blockDim.x) {
+      J.jpart[(size_t)QJ_ENT_PREV * J.ntile + q] = J.jpart[(size_t)QJ_ENTROPY * J.ntile + q];
+      J.jpart[(size_t)QJ_NEG_PREV * J.ntile + q] = J.jpart[(size_t)QJ_NEG * J.ntile + q];
+    }
   // sum (c_t - c) over the step the trial pass evaluated, 2^-t delta_m on
   // the shells the projection keeps and -c_m on those it clips: near the
   // optimum the whole change of F is ~1e-16, below the rounding of either
   // the difference of the two sums (each ~ the electron count) or of c_t
   // itself (c_t - c differs from 2^-t delta by the rounding of c + 2^-t
   // delta, ~1e-16 c per shell, which rho0_t does not contain)
-  const double a = ldexp(1.0, -t);
+  const double a = trial_step(t);
   double ds = 0.0, dec = 0.0;
+#pragma unroll 4
   for (int m = lane; m < M; m += 32) {
     const double c = J.propars[m], x = c + a * J.delta[m];
     const double d = x < 0.0 ? -c : a * J.delta[m];
@@ -2529,16 +2532,10 @@ __global__ void __launch_bounds__(32 * kTrials) k_glisa_trial_pick(Batch bt) {
     ds += __shfl_xor_sync(0xffffffffu, ds, o);
     dec += __shfl_xor_sync(0xffffffffu, dec, o);
   }
-  double df = 0.0, dn = 0.0;  // f(c_t) - f(c), and the magnitude of its FP32 terms
-  for (int q = lane; q < J.ntile; q += 32) {
-    df += J.tpart[(size_t)t * J.ntile + q];
-    dn += J.tpart[(size_t)(kTrials + t) * J.ntile + q];
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    df += __shfl_xor_sync(0xffffffffu, df, o);
-    dn += __shfl_xor_sync(0xffffffffu, dn, o);
-  }
+  // f(c_t) - f(c), and the magnitude of its FP32 terms
+  const double* tp = J.tpart + (size_t)t * J.ntile;
+  const double df = warp_tile_sum_of(J.ntile, [&](int q) { return tp[q]; });
+  const double dn = warp_tile_sum_of(J.ntile, [&](int q) { return tp[(size_t)kTrials * J.ntile + q]; });
   // Armijo on F = f + sum c: F(c_t) <= F(c) + 1e-4 dF.(c_t - c), up to the
   // rounding of the FP32 terms
   if (lane == 0) pass[t] = df + ds <= 1e-4 * dec + kArmijoUlps * 0x1p-24 * dn;
@@ -2559,17 +2556,11 @@ __global__ void __launch_bounds__(32 * kTrials) k_glisa_trial_pick(Batch bt) {
   __syncthreads();
   const int pick = pick_s;
   // the step's start (k_copy_old's work, which projected-Newton steps leave
-  // to this kernel): the parameters, and for fused jobs the entropy and
-  // negativity partials of the pass at them
+  // to this kernel)
   for (int m = threadIdx.x; m < M; m += blockDim.x) {
     J.propars_old[m] = J.propars[m];
     J.propars[m] = J.ctrial[pick * M + m];
   }
-  if (J.fuse)
-    for (int q = threadIdx.x; q < J.ntile; q += blockDim.x) {
-      J.jpart[(size_t)QJ_ENT_PREV * J.ntile + q] = J.jpart[(size_t)QJ_ENTROPY * J.ntile + q];
-      J.jpart[(size_t)QJ_NEG_PREV * J.ntile + q] = J.jpart[(size_t)QJ_NEG * J.ntile + q];
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2742,7 +2733,7 @@ void launch_glisa_refine(const HostBatch& hb, cudaStream_t st, int gff, int fuse
     HP_LAUNCH(k_glisa_hv, K_POINT1, kThreads);
     launch_glisa_grad(hb, st, 1);
   }
-  HP_LAUNCH(k_glisa_gsum, K_SQUARE, kThreads);  // K_SQUARE: ceil(M^2 / 256) >= ceil(M / 8) blocks
+  HP_LAUNCH(k_glisa_gsum, K_SQUARE, kThreads);  // a warp per row
   if (hb.blocks[K_JOB] > 0) {  // dynamic shared memory: the FP32 factor (set up by launch_glisa_solve)
     k_glisa_refine<<<hb.blocks[K_JOB], kThreads, kNewtonSmemL, st>>>(hb.b[K_JOB]);
     ++g_launch_count;

@@ -305,7 +305,7 @@ int blocks_for(const JobDev& J, int kind) {
       if (J.scheme != SCHEME_GLISA || J.fuse) return 0;  // fused jobs: in the fused pass
       if (J.hsched) return J.hbuf;
       return J.tc ? tc_hess_blocks(J) : J.nsplit * J.htiles * (J.htiles + 1) / 2;
-    case K_SQUARE: return J.scheme == SCHEME_GLISA ? (J.nshell * J.nshell + kThreads - 1) / kThreads : 0;
+    case K_SQUARE: return J.scheme == SCHEME_GLISA ? square_blocks(J.nshell) : 0;
   }
   return 0;
 }
