@@ -602,13 +602,12 @@ struct HostBatch {
 
 void launch_nelec(const HostBatch& hb, cudaStream_t st);
 void launch_tile_rmin(const HostBatch& hb, cudaStream_t st);
-void launch_copy_old(const HostBatch& hb, cudaStream_t st);
+void launch_copy_old(const HostBatch& hb, cudaStream_t st, bool inner);
 void launch_promol(const HostBatch& hb, cudaStream_t st, int mixed, int model, bool weights = true);
 void launch_final_atweights(const HostBatch& hb, cudaStream_t st, int mixed, int model, int use_old);
 void launch_change(const HostBatch& hb, cudaStream_t st, int mixed, int model);
 void launch_outer_finish(const HostBatch& hb, cudaStream_t st, int with_charges);
 void launch_charges(const HostBatch& hb, cudaStream_t st);
-void launch_inner_init(const HostBatch& hb, cudaStream_t st);
 void launch_count_active(const HostBatch& hb, cudaStream_t st);
 // one launch per inner iteration, parameter update included (hp_inner.cuh)
 void launch_mbis_inner(const HostBatch& hb, cudaStream_t st, int mixed);

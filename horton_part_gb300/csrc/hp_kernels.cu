@@ -37,6 +37,21 @@ __device__ __forceinline__ const JobDev& decode_local(const Batch& bt, int& loca
   return bt.jobs[j];
 }
 
+// The block's job descriptor in shared memory: in kernels of one short block
+// per job each first read of a line of it was an L2 round trip of its own, in
+// a chain with the array behind it. All threads; synchronises.
+struct JobCopy {
+  unsigned long long raw[(sizeof(JobDev) + 7) / 8];
+};
+__device__ __forceinline__ const JobDev& decode_job(const Batch& bt, JobCopy* copy) {
+  static_assert(sizeof(JobDev) % 8 == 0 && alignof(JobDev) == 8, "copied by 8-byte words");
+  const JobDev& G = bt.jobs[find_job(bt, blockIdx.x)];
+  const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&G);
+  for (int i = threadIdx.x; i < (int)(sizeof(JobDev) / 8); i += blockDim.x) copy->raw[i] = src[i];
+  __syncthreads();
+  return *reinterpret_cast<const JobDev*>(copy->raw);
+}
+
 __device__ __forceinline__ AtomTile decode_atom_tile(const Batch& bt, const JobDev*& Jp) {
   const int b = blockIdx.x;
   const int j = find_job(bt, b);
@@ -213,9 +228,10 @@ __global__ void k_init_params(Batch bt) {
   }
 }
 
-__global__ void k_copy_old(Batch bt) {
-  int local;
-  const JobDev& J = decode_local(bt, local);
+// The parameters a step starts from; inner: and the state of its inner solve.
+__global__ void k_copy_old(Batch bt, int inner) {
+  __shared__ JobCopy jc;
+  const JobDev& J = decode_job(bt, &jc);
   if (glisa_idle(J)) return;
   for (int i = threadIdx.x; i < J.nparam; i += blockDim.x) J.propars_old[i] = J.propars[i];
   if (J.scheme == SCHEME_MBIS && !J.mixed)  // the amplitudes of the step's start (hp_mbis.cu)
@@ -226,6 +242,24 @@ __global__ void k_copy_old(Batch bt) {
       J.jpart[(size_t)QJ_ENT_PREV * J.ntile + t] = J.jpart[(size_t)QJ_ENTROPY * J.ntile + t];
       J.jpart[(size_t)QJ_NEG_PREV * J.ntile + t] = J.jpart[(size_t)QJ_NEG * J.ntile + t];
     }
+  if (!inner) return;
+  for (int i = threadIdx.x; i < J.nparam; i += blockDim.x) {
+    J.cur[i] = J.propars[i];
+    J.prev[i] = J.propars[i];
+  }
+  for (int a = threadIdx.x; a < J.natom; a += blockDim.x) {
+    J.active[a] = 1;
+    J.inner_it[a] = 0;
+    J.arrive[a] = 0;
+    J.atom_out[a * AO_COUNT + AO_INNER_CHANGE] = 1e300;
+  }
+  if (J.mixed)
+    for (int s = threadIdx.x; s < J.nshell; s += blockDim.x) fill_fco(J, s, J.propars, J.propars);
+  if (threadIdx.x == 0) {
+    J.mail->i[MI_NACTIVE] = J.natom;
+    J.mail->i[MI_INNER_MAX] = 0;
+    J.mail->d[MD_INNER_TOTAL] = 0.0;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -383,8 +417,8 @@ __global__ void __launch_bounds__(kFinishThreads) k_outer_finish(Batch bt, int w
   __shared__ double chg[kFinishAtoms];
   __shared__ double ent_s;
   __shared__ double change_s;
-  int local;
-  const JobDev& J = decode_local(bt, local);
+  __shared__ JobCopy jc;
+  const JobDev& J = decode_job(bt, &jc);
   if (glisa_idle(J)) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int it = J.mail->i[MI_ITER];
@@ -456,28 +490,6 @@ __global__ void k_count_active(Batch bt) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
   if (lane == 0) J.mail->i[MI_NACTIVE] = c;
-}
-
-__global__ void k_inner_init(Batch bt) {
-  int local;
-  const JobDev& J = decode_local(bt, local);
-  for (int i = threadIdx.x; i < J.nparam; i += blockDim.x) {
-    J.cur[i] = J.propars[i];
-    J.prev[i] = J.propars[i];
-  }
-  for (int a = threadIdx.x; a < J.natom; a += blockDim.x) {
-    J.active[a] = 1;
-    J.inner_it[a] = 0;
-    J.arrive[a] = 0;
-    J.atom_out[a * AO_COUNT + AO_INNER_CHANGE] = 1e300;
-  }
-  if (J.mixed)
-    for (int s = threadIdx.x; s < J.nshell; s += blockDim.x) fill_fco(J, s, J.propars, J.propars);
-  if (threadIdx.x == 0) {
-    J.mail->i[MI_NACTIVE] = J.natom;
-    J.mail->i[MI_INNER_MAX] = 0;
-    J.mail->d[MD_INNER_TOTAL] = 0.0;
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2280,8 +2292,8 @@ __device__ void trial_set_body(const JobDev& J, int* tms, int* wcount) {
 __global__ void __launch_bounds__(kThreads) k_glisa_trial_set(Batch bt) {
   __shared__ int tms[kTrialSetSmem];
   __shared__ int wcount[kTrials * kTrialSetSmem / 32];
-  int local;
-  const JobDev& J = decode_local(bt, local);
+  __shared__ JobCopy jc;
+  const JobDev& J = decode_job(bt, &jc);
   if (glisa_idle(J)) return;
   trial_set_body<kThreads>(J, tms, wcount);
 }
@@ -2499,68 +2511,92 @@ constexpr double kArmijoUlps = 8.0;
 // converged parameters are those of the direct evaluation.
 constexpr double kR0HandoffChange = 1e4;
 
-__global__ void __launch_bounds__(32 * kTrials) k_glisa_trial_pick(Batch bt) {
+// Latency: everything it reads is loaded before the first sum, and the copies
+// of the step's start (k_copy_old's work, which projected-Newton steps leave
+// to this kernel) are made by warps of their own (16.4 -> 15.1 us; the sums' FP64 issue on one SM is what is left).
+constexpr int kPickThreads = 32 * kTrials + 128;
+__global__ void __launch_bounds__(kPickThreads) k_glisa_trial_pick(Batch bt) {
   __shared__ int pass[kTrials];
-  __shared__ int pick_s;
-  int local;
-  const JobDev& J = decode_local(bt, local);
+  __shared__ JobCopy jc;
+  const JobDev& J = decode_job(bt, &jc);
   if (glisa_idle(J)) return;
   const int lane = threadIdx.x & 31, t = threadIdx.x >> 5;
-  const int M = J.nshell;
-  if (J.fuse)  // the entropy and negativity partials of the pass at the step's start
-    for (int q = threadIdx.x; q < J.ntile; q += blockDim.x) {
-      J.jpart[(size_t)QJ_ENT_PREV * J.ntile + q] = J.jpart[(size_t)QJ_ENTROPY * J.ntile + q];
-      J.jpart[(size_t)QJ_NEG_PREV * J.ntile + q] = J.jpart[(size_t)QJ_NEG * J.ntile + q];
-    }
-  // sum (c_t - c) over the step the trial pass evaluated, 2^-t delta_m on
-  // the shells the projection keeps and -c_m on those it clips: near the
-  // optimum the whole change of F is ~1e-16, below the rounding of either
-  // the difference of the two sums (each ~ the electron count) or of c_t
-  // itself (c_t - c differs from 2^-t delta by the rounding of c + 2^-t
-  // delta, ~1e-16 c per shell, which rho0_t does not contain)
-  const double a = trial_step(t);
-  double ds = 0.0, dec = 0.0;
+  const int M = J.nshell, nt = J.ntile;
+  if (t >= kTrials) {
+    const int i0 = threadIdx.x - 32 * kTrials;
+    for (int m = i0; m < M; m += 128) J.propars_old[m] = J.propars[m];
+    if (J.fuse) {  // the entropy and negativity partials of the pass at the start
+      const double* __restrict__ ent = J.jpart + (size_t)QJ_ENTROPY * nt;
+      const double* __restrict__ neg = J.jpart + (size_t)QJ_NEG * nt;
+      double* __restrict__ ent0 = J.jpart + (size_t)QJ_ENT_PREV * nt;
+      double* __restrict__ neg0 = J.jpart + (size_t)QJ_NEG_PREV * nt;
 #pragma unroll 4
-  for (int m = lane; m < M; m += 32) {
-    const double c = J.propars[m], x = c + a * J.delta[m];
-    const double d = x < 0.0 ? -c : a * J.delta[m];
-    ds += d;
-    dec += (1.0 + J.grad[m]) * d;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    ds += __shfl_xor_sync(0xffffffffu, ds, o);
-    dec += __shfl_xor_sync(0xffffffffu, dec, o);
-  }
-  // f(c_t) - f(c), and the magnitude of its FP32 terms
-  const double* tp = J.tpart + (size_t)t * J.ntile;
-  const double df = warp_tile_sum_of(J.ntile, [&](int q) { return tp[q]; });
-  const double dn = warp_tile_sum_of(J.ntile, [&](int q) { return tp[(size_t)kTrials * J.ntile + q]; });
-  // Armijo on F = f + sum c: F(c_t) <= F(c) + 1e-4 dF.(c_t - c), up to the
-  // rounding of the FP32 terms
-  if (lane == 0) pass[t] = df + ds <= 1e-4 * dec + kArmijoUlps * 0x1p-24 * dn;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int pick = kTrials - 1;
-    for (int k = 0; k < kTrials; ++k)
-      if (pass[k]) {
-        pick = k;
-        break;
+      for (int q = i0; q < nt; q += 128) {
+        ent0[q] = ent[q];
+        neg0[q] = neg[q];
       }
-    pick_s = pick;
-    J.mail->d[MD_LS_X] = ldexp(1.0, -pick);
+    }
+  } else {
+    const double* __restrict__ par = J.propars;
+    const double* __restrict__ dl = J.delta;
+    const double* __restrict__ gr = J.grad;
+    const double* __restrict__ tp = J.tpart + (size_t)t * nt;
+    const double* __restrict__ tn = tp + (size_t)kTrials * nt;
+    // sum (c_t - c) over the step the trial pass evaluated, 2^-t delta_m on
+    // the shells the projection keeps and -c_m on those it clips: near the
+    // optimum the whole change of F is ~1e-16, below the rounding of either
+    // the difference of the two sums (each ~ the electron count) or of c_t
+    // itself (c_t - c differs from 2^-t delta by the rounding of c + 2^-t
+    // delta, ~1e-16 c per shell, which rho0_t does not contain)
+    const double a = trial_step(t);
+    constexpr int kU = 8;
+    double ds = 0.0, dec = 0.0;
+    double f[4] = {0.0, 0.0, 0.0, 0.0}, n[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int k0 = lane; k0 < max(M, nt); k0 += 32 * kU) {
+      double c[kU], d[kU], g[kU], x[kU], y[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const int k = k0 + 32 * u;
+        c[u] = k < M ? par[k] : 0.0;
+        d[u] = k < M ? dl[k] : 0.0;
+        g[u] = k < M ? gr[k] : 0.0;
+        x[u] = k < nt ? tp[k] : 0.0;
+        y[u] = k < nt ? tn[k] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        f[u & 3] += x[u];
+        n[u & 3] += y[u];
+        if (k0 - lane + 32 * u >= M) continue;
+        const double step = c[u] + a * d[u] < 0.0 ? -c[u] : a * d[u];
+        ds += step;
+        dec += (1.0 + g[u]) * step;
+      }
+    }
+    // f(c_t) - f(c), and the magnitude of its FP32 terms
+    double df = (f[0] + f[1]) + (f[2] + f[3]), dn = (n[0] + n[1]) + (n[2] + n[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      ds += __shfl_xor_sync(0xffffffffu, ds, o);
+      dec += __shfl_xor_sync(0xffffffffu, dec, o);
+      df += __shfl_xor_sync(0xffffffffu, df, o);
+      dn += __shfl_xor_sync(0xffffffffu, dn, o);
+    }
+    // Armijo on F = f + sum c: F(c_t) <= F(c) + 1e-4 dF.(c_t - c), up to the
+    // rounding of the FP32 terms
+    if (lane == 0) pass[t] = df + ds <= 1e-4 * dec + kArmijoUlps * 0x1p-24 * dn;
+  }
+  __syncthreads();
+  int pick = kTrials - 1;
+  for (int k = kTrials - 1; k >= 0; --k)
+    if (pass[k]) pick = k;
+  if (threadIdx.x == 0) {
+    J.mail->d[MD_LS_X] = trial_step(pick);
     // fused jobs away from convergence: the next pass takes rho0 of the
     // accepted trial from the trial pass (r0t) instead of forming G^T c
     J.mail->i[MI_R0T] = J.r0t && J.mail->d[MD_CHANGE] >= kR0HandoffChange * J.threshold ? pick + 1 : 0;
   }
-  __syncthreads();
-  const int pick = pick_s;
-  // the step's start (k_copy_old's work, which projected-Newton steps leave
-  // to this kernel)
-  for (int m = threadIdx.x; m < M; m += blockDim.x) {
-    J.propars_old[m] = J.propars[m];
-    J.propars[m] = J.ctrial[pick * M + m];
-  }
+  for (int m = threadIdx.x; m < M; m += kPickThreads) J.propars[m] = J.ctrial[pick * M + m];
 }
 
 // ---------------------------------------------------------------------------
@@ -2584,7 +2620,7 @@ void launch_nelec(const HostBatch& hb, cudaStream_t st) {
 
 void launch_tile_rmin(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_tile_rmin, K_ATOM, kThreads); }
 
-void launch_copy_old(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_copy_old, K_JOB, 128); }
+void launch_copy_old(const HostBatch& hb, cudaStream_t st, bool inner) { HP_LAUNCH(k_copy_old, K_JOB, 128, inner ? 1 : 0); }
 
 // FP32 variants live in hp_mixed.cu, float-float (MBIS) in hp_ff.cu; `mixed`
 // is the job group's evaluation phase (Phase).
@@ -2639,7 +2675,6 @@ void launch_outer_finish(const HostBatch& hb, cudaStream_t st, int with_charges)
 
 void launch_charges(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_charges, K_JOB, kChargesThreads); }
 
-void launch_inner_init(const HostBatch& hb, cudaStream_t st) { HP_LAUNCH(k_inner_init, K_JOB, 128); }
 
 void launch_count_active(const HostBatch& hb, cudaStream_t st) {
   HP_LAUNCH(k_count_active, K_JOB, 32);
@@ -2765,7 +2800,7 @@ void launch_glisa_pnewton(const HostBatch& hb, cudaStream_t st, int gff, int fus
   if (fuse_shells > 0) launch_glisa_trials_fused(hb, st, fuse_shells);
   else if (gff) launch_glisa_trials_ff(hb, st);
   else launch_glisa_trials64(hb, st);
-  HP_LAUNCH(k_glisa_trial_pick, K_JOB, 32 * kTrials);
+  HP_LAUNCH(k_glisa_trial_pick, K_JOB, kPickThreads);
 }
 
 }  // namespace hp

@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kThreads) k_change_mx(Batch bt) {
 
 // ---------------------------------------------------------------------------
 // MBIS inner fixed point (mbis.py:81-163); coefficients of (cur, prev) in fco,
-// written by k_inner_init / mbis_update
+// written by k_copy_old / mbis_update
 // ---------------------------------------------------------------------------
 
 constexpr int kMxMbisQ = 2 * 7 + 1;

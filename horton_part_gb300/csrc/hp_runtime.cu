@@ -409,7 +409,6 @@ const char* err_text(int err) {
 template <typename F>
 int run_inner(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatch& hb, F launch_one,
               int max_launch, bool counted = false) {
-  launch_inner_init(hb, ctx->stream);
   int chunk = 1;
   for (hp_job* j : jobs) chunk = std::max(chunk, j->last_inner);
   int launched = 0;
@@ -642,7 +641,7 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
   const int model = model_of(j0);
   const bool local = j0->dev.local != 0;
   cudaStream_t st = ctx->stream;
-  launch_copy_old(hb, st);
+  launch_copy_old(hb, st, j0->desc.scheme != HP_SCHEME_GISA);
   {
     ProfScope ps(ctx, HP_KERNEL_PROMOL);
     // FP64 on atom grids, and GISA with a stored G: at_weights in their own passes
@@ -654,11 +653,9 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
     case HP_SCHEME_MBIS:
       if (local) {  // atom grids: every inner iteration of every atom in one launch
         ProfScope ps(ctx, HP_KERNEL_INNER);
-        launch_inner_init(hb, st);
         launch_mbis_local(hb, st, mixed);
       } else if (!mixed && hb.solve_tiles > 0) {  // the same in one cooperative launch
         ProfScope ps(ctx, HP_KERNEL_INNER);
-        launch_inner_init(hb, st);
         launch_mbis_solve64(hb, st);
       } else {
         rc = run_inner(ctx, jobs, hb, [&] {
@@ -670,7 +667,6 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
     case HP_SCHEME_NLIS:  // NLIS / GMBIS (FP64)
       if (local) {
         ProfScope ps(ctx, HP_KERNEL_INNER);
-        launch_inner_init(hb, st);
         launch_nlis_local(hb, st);
       } else {
         rc = run_inner(ctx, jobs, hb, [&] {
@@ -692,7 +688,6 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
     case HP_SCHEME_LISA:
       if (local) {  // atom grids: every inner iteration of every atom in one launch
         ProfScope ps(ctx, HP_KERNEL_INNER);
-        launch_inner_init(hb, st);
         launch_lisa_sc_local(hb, st, mixed);
       } else if (j0->dev.solver == SOLVER_SC)
         rc = run_inner(ctx, jobs, hb, [&] {
@@ -818,7 +813,7 @@ int step_glisa(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatch& h
   };
   for (int iter = 0; iter < iters; ++iter) {
   // projected Newton keeps the step's start in k_glisa_trial_pick
-  if (solver != SOLVER_PNEWTON) launch_copy_old(hb, st);
+  if (solver != SOLVER_PNEWTON) launch_copy_old(hb, st, false);
   if (!fused) {
     ProfScope ps(ctx, HP_KERNEL_GLISA_PRO);
     if (gff) launch_glisa_pro_ff(hb, st);
