@@ -630,7 +630,7 @@ void launch_glisa_check(const HostBatch& hb, cudaStream_t st);
 // evaluation service of the host-driven gLISA solvers (FP64 jobs):
 // what 0: objective (entropy) and int rho0 after k_glisa_pro;
 // what 1: sqrt(int (sum_m delta_m g_m)^2), the promolecule change for delta;
-// what 2: sqrt(sum over atoms of the QA_CHANGE partials) after k_glisa_change
+// what 2: sqrt(sum over atoms of the QA_CHANGE partials) after the change pass
 void launch_glisa_eval(const HostBatch& hb, cudaStream_t st, int what);
 // trials + Armijo pick; fuse_shells > 0: the fused trial pass (batch of fused jobs)
 void launch_glisa_pnewton(const HostBatch& hb, cudaStream_t st, int gff, int fuse_shells);
