@@ -472,7 +472,7 @@ void launch_mbis_inner64(const HostBatch& hb, cudaStream_t st) {
 
 // Blocks of k_mbis_solve64 that are resident together on this device.
 int mbis_solve_capacity() {
-  static int dev_of = -1, cap = 0;
+  static thread_local int dev_of = -1, cap = 0;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev_of != dev) {
