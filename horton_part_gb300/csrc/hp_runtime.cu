@@ -156,8 +156,10 @@ void drop_kept(hp_job* j) {
 
 // Whether the budget has room for `bytes`: jobs give back what they only
 // keep to save recomputation (their results do not depend on it) before an
-// allocation is refused.
+// allocation is refused. Nothing is given back where that would not be enough
+// (a server offers the same waiting job again at every step).
 bool make_room(hp_ctx* ctx, size_t bytes) {
+  if (ctx->used - ctx->kept + bytes > ctx->budget) return false;
   for (size_t k = 0; k < ctx->slots.size() && ctx->used + bytes > ctx->budget; ++k)
     if (ctx->slots[k]) drop_kept(ctx->slots[k]);
   return ctx->used + bytes <= ctx->budget;

@@ -1,0 +1,51 @@
+"""The device memory of a context: what FP64 jobs only keep to save recomputation (distances, pro-atoms, packets of the
+inner solve) is given back when it makes room for something else, and stays where it does not."""
+
+import numpy as np
+import pytest
+
+from horton_part_gb300 import _lib
+from horton_part_gb300.mbis import get_initial_mbis_propars
+from oracle import hp_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+NUMBERS = np.array([1, 1])
+
+
+def _job(ctx, npoint, maxiter=3):
+    """Two hydrogens on `npoint` random points: the memory counts here, not the integral's accuracy."""
+    rng = np.random.default_rng(npoint)
+    coords = np.array([[0.0, 0.0, 0.0], [0.0, 0.0, 1.5]])
+    points = rng.uniform(-3.0, 3.0, (npoint, 3))
+    rho = sum(O.mbis_proatom(get_initial_mbis_propars(1), np.linalg.norm(points - c, axis=1)) for c in coords)
+    return _lib.Job(ctx, "mbis", coords, NUMBERS.astype(float), points, np.full(npoint, 216.0 / npoint), rho,
+                    np.arange(3, dtype=np.int32), np.concatenate([get_initial_mbis_propars(1)] * 2), grid_type=3,
+                    threshold=1e-12, inner_threshold=1e-8, inner_maxiter=50, maxiter=maxiter)
+
+
+@pytest.fixture(scope="module")
+def sizes(gpu_context):
+    """(device bytes of the 4000-point job with its kept arrays, without them)"""
+    ctx = _lib.Context(0)
+    job = _job(ctx, 4000)
+    full = job.info().device_bytes
+    ctx.close()
+    ctx = _lib.Context(0, hbm_budget=full)
+    job = _job(ctx, 4000)
+    plain = job.info().device_bytes
+    ctx.close()
+    assert full - plain >= 2 * 8 * 2 * 4000  # the distances and the pro-atoms of every pair
+    return full, plain
+
+
+def test_a_refused_job_takes_nothing_from_a_live_one(sizes):
+    full, plain = sizes
+    budget = 32 * full
+    ctx = _lib.Context(0, hbm_budget=budget)
+    job = _job(ctx, 4000)
+    assert job.info().device_bytes == full
+    with pytest.raises(MemoryError):
+        _job(ctx, 4000 * 64)  # more than the whole budget
+    assert job.info().device_bytes == full
+    ctx.close()
