@@ -2169,10 +2169,12 @@ int32_t hp_density_plan_create(hp_ctx* ctx, const hp_density_desc* d, hp_density
 
 namespace {
 // Host points and densities of up to this many bytes together pass through
-// pinned memory that the kernel reads and writes itself (the points once,
-// into shared memory): two copies on the host instead of two transfers, each
-// of them staged by the driver (water, 4,500 points: 54.1 -> 44.9 us
-// a call). Larger sets are copied to the device.
+// pinned memory that the kernel reads and writes itself (each block reads its
+// tile's points once, into shared memory: twice in all where a tile has two
+// blocks): two copies on the host instead of two transfers, each of them
+// staged by the driver (water, 4,500 points: 54.1 -> 44.9 us a call). They
+// take no device memory, so the budget has no say. Larger sets are copied to
+// the device.
 constexpr size_t kStageBytes = 1 << 20;
 
 bool stage_ready(hp_ctx* ctx) {
@@ -2204,7 +2206,6 @@ int32_t hp_density_plan_eval(hp_density_plan* p, int64_t npoint, const double* p
   if (8 * need <= kStageBytes) {
     std::unique_lock<std::mutex> own(ctx->stage_mu, std::try_to_lock);  // (another thread's call: copies)
     if (own.owns_lock() && stage_ready(ctx)) {
-      if (p->scratch_points < need && !make_room(ctx, 8 * need)) return fail(HP_ERR_NO_MEMORY, "HBM budget exceeded");
       double* pts = reinterpret_cast<double*>(ctx->stage);
       memcpy(pts, points, 8 * 3 * (size_t)npoint);
       a.points = pts;

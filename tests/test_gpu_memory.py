@@ -49,3 +49,40 @@ def test_a_refused_job_takes_nothing_from_a_live_one(sizes):
         _job(ctx, 4000 * 64)  # more than the whole budget
     assert job.info().device_bytes == full
     ctx.close()
+
+
+def _water_plan(ctx):
+    from horton_part_gb300 import synthetic
+    from horton_part_gb300.density import DensityPlan
+
+    mol = synthetic.water(10, 50, seed=1)
+    shells = synthetic.contracted_basis(mol.numbers, mol.coordinates, seed=1)
+    nb = sum(s.nfunc for s in shells)
+    return DensityPlan(shells, synthetic.density_matrix(nb, 5, seed=2), context=ctx), mol.grid.points
+
+
+def test_a_small_host_density_call_needs_no_budget(sizes):
+    full, plain = sizes
+    ctx = _lib.Context(0)
+    plan, points = _water_plan(ctx)
+    plan_bytes = ctx.memory()[0]
+    points = np.repeat(points, 20, axis=0)  # a little below a megabyte with the density
+    want = plan.evaluate(points)
+    plan.close()
+    ctx.close()
+    budget = 32 * full
+    ctx = _lib.Context(0, hbm_budget=budget)
+    plan, _ = _water_plan(ctx)
+    jobs = [_job(ctx, 4000)]
+    while budget - plan_bytes - sum(j.info().device_bytes for j in jobs) >= full:
+        jobs.append(_job(ctx, 4000))
+    held = [j.info().device_bytes for j in jobs]
+    assert held[0] == full and budget - plan_bytes - sum(held) < 8 * 4 * len(points) < 1 << 20
+    np.testing.assert_array_equal(plan.evaluate(points), want)
+    assert [j.info().device_bytes for j in jobs] == held
+    with pytest.raises(MemoryError):  # until nothing fits any more, not even by giving back
+        while True:
+            jobs.append(_job(ctx, 4000))
+    np.testing.assert_array_equal(plan.evaluate(points), want)
+    plan.close()
+    ctx.close()
