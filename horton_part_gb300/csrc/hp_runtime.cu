@@ -1224,7 +1224,7 @@ int32_t hp_ctx_synchronize(hp_ctx* c) {
 
 int32_t hp_ctx_memory(hp_ctx* c, size_t* used, size_t* budget) {
   if (!c) return fail(HP_ERR_INVALID, "null context");
-  if (used) *used = c->used;
+  if (used) *used = c->used - c->kept;
   if (budget) *budget = c->budget;
   return HP_OK;
 }

@@ -86,3 +86,21 @@ def test_a_small_host_density_call_needs_no_budget(sizes):
     np.testing.assert_array_equal(plan.evaluate(points), want)
     plan.close()
     ctx.close()
+
+
+def test_memory_counts_what_only_closing_a_job_frees(sizes):
+    full, plain = sizes
+    ctx = _lib.Context(0, hbm_budget=32 * full)
+    jobs = [_job(ctx, 4000)]
+    assert jobs[0].info().device_bytes == full
+    assert ctx.memory() == (plain, 32 * full)
+    # a job fits as long as used + its bytes stay within the budget, and no longer
+    while ctx.memory()[0] + plain <= ctx.memory()[1]:
+        jobs.append(_job(ctx, 4000))
+        assert ctx.memory()[0] == plain * len(jobs)
+    with pytest.raises(MemoryError):
+        _job(ctx, 4000)
+    for j in jobs:
+        j.close()
+    assert ctx.memory()[0] == 0
+    ctx.close()
