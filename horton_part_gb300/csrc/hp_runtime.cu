@@ -183,7 +183,12 @@ int solve_blocks(const JobDev& J, int tiles) {
 
 // FP64 jobs: storage for the pair distances (MBIS) and, on the molecular
 // grid, the pro-atoms of the last inner iteration (MBIS, aLISA sc with a
-// stored G), where it takes at most half of what is left of the budget.
+// stored G), where it takes at most half of what is left of the budget and
+// all jobs' kept arrays together at most a kKeptShare-th of the budget: other
+// allocators of the process (torch, say) cannot ask for it back, and a job
+// with them holds about three times the memory of one without.
+constexpr size_t kKeptShare = 16;
+
 void alloc_kept(hp_ctx* ctx, hp_job* j) {
   JobDev& J = j->dev;
   const bool mbis = J.scheme == SCHEME_MBIS && !J.mixed;
@@ -197,7 +202,7 @@ void alloc_kept(hp_ctx* ctx, hp_job* j) {
   const size_t flags = align_up(4 * (size_t)J.natom * J.ntile);
   const size_t bytes = (mbis ? pair : 0) + (old ? pair + flags : 0) + align_up(packets);
   const size_t room = ctx->budget > ctx->used ? ctx->budget - ctx->used : 0;
-  if (bytes > room / 2) return;
+  if (bytes > room / 2 || ctx->kept + bytes > ctx->budget / kKeptShare) return;
   void* mem = nullptr;
   if (job_alloc(ctx, &mem, bytes) != cudaSuccess) {
     cudaGetLastError();

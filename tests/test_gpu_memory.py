@@ -104,3 +104,14 @@ def test_memory_counts_what_only_closing_a_job_frees(sizes):
         j.close()
     assert ctx.memory()[0] == 0
     ctx.close()
+
+
+def test_kept_arrays_take_a_16th_of_the_budget_at_most(sizes):
+    full, plain = sizes
+    budget = 40 * full
+    ctx = _lib.Context(0, hbm_budget=budget)
+    jobs = [_job(ctx, 4000) for _ in range(40)]
+    kept = [j.info().device_bytes - plain for j in jobs]
+    assert set(kept) == {0, full - plain}
+    assert kept[0] > 0 and sum(kept) <= budget // 16 < sum(kept) + full - plain
+    ctx.close()
