@@ -128,9 +128,11 @@ struct hp_job {
   double skipped = 0.0;  // point-atom evaluations skipped by the per-atom cutoff
   bool host_driven = false;  // finished by hp_glisa_finish (histories kept by the host)
   // FP64 jobs: the stored distances and pro-atoms (JobDev::rd, oldpro,
-  // oldok), given back when another allocation needs the room (make_room)
+  // oldok), given back when another allocation needs the room (make_room), and
+  // taken again by a later step when there is room once more (regain_kept)
   void* keep_mem = nullptr;
   size_t keep_bytes = 0;
+  bool keep_lost = false;
   void* sched_mem = nullptr;  // gLISA FP64: dev.hsched
   size_t sched_bytes = 0;
   void* pack_mem = nullptr;  // fused gLISA: packed G (dev.gpack, dev.gtile_off)
@@ -148,6 +150,7 @@ void drop_kept(hp_job* j) {
   j->bytes -= j->keep_bytes;
   j->keep_mem = nullptr;
   j->keep_bytes = 0;
+  j->keep_lost = true;
   j->dev.rd = nullptr;
   j->dev.oldpro = nullptr;
   j->dev.oldok = nullptr;
@@ -227,6 +230,22 @@ void alloc_kept(hp_ctx* ctx, hp_job* j) {
     cudaMemsetAsync(at, 0, packets, ctx->stream);
     J.spk = reinterpret_cast<ulonglong2*>(at);
   }
+}
+
+// Before the descriptors of a step are formed: jobs whose arrays were given
+// back take them again by the rule of alloc_kept, so that a job's speed does
+// not depend on what was created and destroyed beside it. True where
+// distances have to be formed again (the pro-atoms are, in every first inner
+// iteration).
+bool regain_kept(hp_ctx* ctx, const std::vector<hp_job*>& jobs) {
+  bool form = false;
+  for (hp_job* j : jobs) {
+    if (!j->keep_lost) continue;
+    alloc_kept(ctx, j);
+    j->keep_lost = j->keep_mem == nullptr;
+    form |= j->dev.rd != nullptr;
+  }
+  return form;
 }
 
 // State of a mixed-precision job after an outer iteration:
@@ -1006,9 +1025,11 @@ int step_group(hp_ctx* ctx, const std::vector<hp_job*>& jobs, int iters) {
     if (rc) return rc;
     HP_CK(cudaStreamSynchronize(ctx->stream));
   }
+  const bool form_rd = regain_kept(ctx, jobs);
   HostBatch hb;
   rc = build_batch(ctx, jobs, hb);
   if (rc) return rc;
+  if (form_rd) launch_rdist64(hb, ctx->stream);
   if (jobs[0]->desc.scheme == HP_SCHEME_GLISA) return step_glisa(ctx, jobs, hb, iters);
   return step_iterstock(ctx, jobs, hb);
 }

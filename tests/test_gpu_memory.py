@@ -115,3 +115,34 @@ def test_kept_arrays_take_a_16th_of_the_budget_at_most(sizes):
     assert set(kept) == {0, full - plain}
     assert kept[0] > 0 and sum(kept) <= budget // 16 < sum(kept) + full - plain
     ctx.close()
+
+
+def test_given_back_arrays_return_when_there_is_room(sizes):
+    """A job that had to give its arrays back has them again, and the one-launch inner solve, once the job that took
+    the room is gone: the same launches and the same bits as a job that never lost them."""
+    full, plain = sizes
+    ctx = _lib.Context(0, hbm_budget=32 * full)
+    runs = []
+    for crowded in (False, True):
+        job = _job(ctx, 4000)
+        ctx.step([job])
+        if crowded:
+            others = []
+            with pytest.raises(MemoryError):
+                while True:
+                    others.append(_job(ctx, 4000))
+            assert job.info().device_bytes == plain
+            ctx.step([job])  # without them, a launch per inner iteration
+            for j in others:
+                j.close()
+        else:
+            ctx.step([job])
+        ctx.profile()
+        ctx.step([job])
+        runs.append((ctx.profile_get("inner")[1], job.info().device_bytes, job.results(at_weights=True)))
+        ctx.profile(False)
+        job.close()
+    assert runs[0][:2] == runs[1][:2] == (1, full)
+    for key in runs[0][2]:
+        np.testing.assert_array_equal(runs[0][2][key], runs[1][2][key])
+    ctx.close()
