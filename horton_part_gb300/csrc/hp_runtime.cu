@@ -178,6 +178,21 @@ cudaError_t job_alloc_retry(hp_ctx* ctx, void** p, size_t bytes) {
   return job_alloc(ctx, p, bytes);
 }
 
+// cudaMalloc for memory outside the pool: freed job memory stays in the pool,
+// so that a failure is retried once after giving back and trimming it.
+cudaError_t device_alloc_retry(hp_ctx* ctx, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaSuccess) return e;
+  cudaGetLastError();
+  for (hp_job* j : ctx->slots)
+    if (j) drop_kept(j);
+  cudaStreamSynchronize(ctx->stream);  // the frees have run
+  cudaMemPoolTrimTo(ctx->pool, 0);
+  e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
 constexpr int kSolveTiles = 4;  // tiles per block of k_mbis_solve64 at most (solve_tiles)
 
 int solve_blocks(const JobDev& J, int tiles) {
@@ -2138,10 +2153,10 @@ int32_t hp_density_plan_create(hp_ctx* ctx, const hp_density_desc* d, hp_density
   if (!make_room(ctx, bytes)) return fail(HP_ERR_NO_MEMORY, "HBM budget exceeded");
   hp_density_plan* p = new hp_density_plan();
   p->ctx = ctx;
-  if (cudaMalloc(&p->dev, 8 * std::max<size_t>(ndbl, 1)) != cudaSuccess ||
-      cudaMalloc(&p->info, 4 * std::max<size_t>(5 * (size_t)ns, 1)) != cudaSuccess ||
-      cudaMalloc(&p->groups, 4 * groups.size()) != cudaSuccess ||
-      cudaMalloc(&p->stats, 8 * 3) != cudaSuccess) {
+  if (device_alloc_retry(ctx, (void**)&p->dev, 8 * std::max<size_t>(ndbl, 1)) != cudaSuccess ||
+      device_alloc_retry(ctx, (void**)&p->info, 4 * std::max<size_t>(5 * (size_t)ns, 1)) != cudaSuccess ||
+      device_alloc_retry(ctx, (void**)&p->groups, 4 * groups.size()) != cudaSuccess ||
+      device_alloc_retry(ctx, (void**)&p->stats, 8 * 3) != cudaSuccess) {
     hp_density_plan_destroy(p);
     return fail(HP_ERR_NO_MEMORY, "device allocation failed");
   }
@@ -2252,7 +2267,8 @@ int32_t hp_density_plan_eval(hp_density_plan* p, int64_t npoint, const double* p
       p->scratch_points = 0;
     }
     if (!make_room(ctx, 8 * need)) return fail(HP_ERR_NO_MEMORY, "HBM budget exceeded");
-    if (cudaMalloc(&p->scratch, 8 * need) != cudaSuccess) return fail(HP_ERR_NO_MEMORY, "device allocation failed");
+    if (device_alloc_retry(ctx, (void**)&p->scratch, 8 * need) != cudaSuccess)
+      return fail(HP_ERR_NO_MEMORY, "device allocation failed");
     p->scratch_points = need;
     ctx->used += 8 * need;
   }

@@ -51,14 +51,15 @@ def test_a_refused_job_takes_nothing_from_a_live_one(sizes):
     ctx.close()
 
 
-def _water_plan(ctx):
+def _water_plan(ctx, nmat=1):
     from horton_part_gb300 import synthetic
     from horton_part_gb300.density import DensityPlan
 
     mol = synthetic.water(10, 50, seed=1)
     shells = synthetic.contracted_basis(mol.numbers, mol.coordinates, seed=1)
     nb = sum(s.nfunc for s in shells)
-    return DensityPlan(shells, synthetic.density_matrix(nb, 5, seed=2), context=ctx), mol.grid.points
+    mats = np.array([synthetic.density_matrix(nb, 5, seed=2)] * nmat)
+    return DensityPlan(shells, mats, context=ctx), mol.grid.points
 
 
 def test_a_small_host_density_call_needs_no_budget(sizes):
@@ -145,4 +146,40 @@ def test_given_back_arrays_return_when_there_is_room(sizes):
     assert runs[0][:2] == runs[1][:2] == (1, full)
     for key in runs[0][2]:
         np.testing.assert_array_equal(runs[0][2][key], runs[1][2][key])
+    ctx.close()
+
+
+@pytest.mark.parametrize("when", ["create", "evaluate"])
+def test_density_plans_take_the_room_that_jobs_give_back(when, sizes):
+    full, plain = sizes
+    ctx = _lib.Context(0)
+    nmat = 40 if when == "create" else 1  # a plan larger than the small jobs below
+    plan, points = _water_plan(ctx, nmat)
+    plan_bytes = ctx.memory()[0]
+    points = np.repeat(points, 30, axis=0)  # past a megabyte: device scratch
+    want, want_few = plan.evaluate(points), plan.evaluate(points[:500])
+    scratch = ctx.memory()[0] - plan_bytes
+    assert scratch == 8 * (3 + nmat) * len(points) > 1 << 20
+    plan.close()
+    ctx.close()
+    need = plan_bytes if when == "create" else scratch
+    budget = 40 * full
+    ctx = _lib.Context(0, hbm_budget=budget)
+    if when == "evaluate":
+        plan, _ = _water_plan(ctx, nmat)
+    held = ctx.memory()[0]
+    job = _job(ctx, 4000)
+    ctx.step([job])
+    jobs = [job]  # small ones until what is left is below what the plan needs with the kept arrays, and not without
+    while budget - held - sum(j.info().device_bytes for j in jobs) >= need:
+        jobs.append(_job(ctx, 2))
+    assert job.info().device_bytes == full and budget - ctx.memory()[0] >= need
+    if when == "create":
+        plan, _ = _water_plan(ctx, nmat)
+        np.testing.assert_array_equal(plan.evaluate(points[:500]), want_few)
+    else:
+        np.testing.assert_array_equal(plan.evaluate(points), want)
+    assert job.info().device_bytes == plain
+    ctx.step([job])  # and the job goes on
+    plan.close()
     ctx.close()
