@@ -90,6 +90,14 @@ __device__ __forceinline__ double dist_of(const JobDev& J, const double* rd, int
 // Amplitude N S^3 / (8 pi) of an MBIS shell.
 __device__ __forceinline__ double mbis_amp(double n, double s) { return n * (s * s * s) * kInv8PiD; }
 
+// New (N, S) of an MBIS shell from the moments of its bare exponential: N = A
+// m0, S = 3 m0 / m1 (mbis.py:150-156). The amplitude cancels in S, but a shell
+// without one has S = 0 / 0 there, and the same here.
+__device__ __forceinline__ void mbis_shell(double amp, double m0, double m1, double& n, double& s) {
+  n = amp * m0;
+  s = amp == 0.0 ? __longlong_as_double(0x7ff8000000000000ll) : 3.0 * m0 / m1;
+}
+
 // Pro-atom of n MBIS shells at distance r from amplitudes and exponents.
 __device__ __forceinline__ double mbis_pro(const double* amp, const double* s, int stride, int n,
                                            double r, const double* tab) {

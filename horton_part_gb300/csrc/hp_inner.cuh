@@ -112,8 +112,12 @@ static __device__ __noinline__ void mbis_update(const JobDev& J, int a) {
   const int k = threadIdx.x;
   double n = 0.0, s = 0.0;
   if (k < nsh) {
-    n = J.mixed ? m[2 * k] : amp[2 * k] * m[2 * k];
-    s = 3.0 * m[2 * k] / m[2 * k + 1];
+    if (J.mixed) {
+      n = m[2 * k];
+      s = 3.0 * m[2 * k] / m[2 * k + 1];
+    } else {
+      f64::mbis_shell(amp[2 * k], m[2 * k], m[2 * k + 1], n, s);
+    }
   }
   const double change = (it == 0) ? 1e100 : sqrt(m[2 * nsh]);
   const bool conv = change < J.inner_threshold || mixed_stalled(J, change);

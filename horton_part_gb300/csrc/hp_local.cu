@@ -185,7 +185,8 @@ __device__ __forceinline__ void mbis_radial(const JobDev& J, int a, const double
     __syncthreads();
     if (threadIdx.x < NSH) {
       const int k = threadIdx.x;
-      const double n = amp[k] * m[2 * k], s = 3.0 * m[2 * k] / m[2 * k + 1];
+      double n, s;
+      f64::mbis_shell(amp[k], m[2 * k], m[2 * k + 1], n, s);
       pa[2 * k] = n;
       pa[2 * k + 1] = s;
       sx[k] = s;

@@ -355,8 +355,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_mbis_solve64(Batch bt, int T, u
     }
     // the update (mbis_update): the parameters on warp 0, the test on warp 1
     if (threadIdx.x < nsh) {
-      const double n = amp[2 * threadIdx.x] * m[2 * threadIdx.x];
-      const double s = 3.0 * m[2 * threadIdx.x] / m[2 * threadIdx.x + 1];
+      double n, s;
+      f64::mbis_shell(amp[2 * threadIdx.x], m[2 * threadIdx.x], m[2 * threadIdx.x + 1], n, s);
       prev[2 * threadIdx.x] = cur[2 * threadIdx.x];
       prev[2 * threadIdx.x + 1] = cur[2 * threadIdx.x + 1];
       cur[2 * threadIdx.x] = n;
