@@ -710,7 +710,9 @@ void launch_rdist64(const HostBatch& hb, cudaStream_t st);  // rd of the batch's
 void launch_promol64(const HostBatch& hb, cudaStream_t st, bool weights);  // weights: k_atweights too
 void launch_mbis_inner64(const HostBatch& hb, cudaStream_t st);
 int mbis_solve_capacity();
-void launch_mbis_solve64(const HostBatch& hb, cudaStream_t st);  // every inner iteration (K_SOLVE)
+constexpr int kSolvePolls = 1 << 20;  // polls after which a wait of k_mbis_solve64 gives up
+// every inner iteration (K_SOLVE); an error means that nothing was launched
+cudaError_t launch_mbis_solve64(const HostBatch& hb, cudaStream_t st, int polls);
 void launch_change64(const HostBatch& hb, cudaStream_t st);
 void launch_final_atweights64(const HostBatch& hb, cudaStream_t st, int use_old);
 

@@ -241,8 +241,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_mbis_inner64(Batch bt) {
 // (counter and 512-point tiles before; 21.1 with a launch per iteration).
 //
 // The wait is bounded: a block that runs out of polls sets E_TIMEOUT and
-// ends, and so do the others, each by its own bound.
-constexpr int kSolvePolls = 1 << 20;
+// ends, and so do the others, each by its own bound (max_polls; kSolvePolls is
+// most of a second).
 
 __device__ __forceinline__ void put_packet(ulonglong2* p, double v, unsigned long long tag) {
   asm volatile(
@@ -264,7 +264,7 @@ __device__ __forceinline__ double get_packet(const ulonglong2* p, unsigned long 
 // The warp's sum of ntile packets of this tag, in the order of
 // warp_tile_sum_of; waits for them (*late is set where they do not come).
 __device__ __forceinline__ double packet_sum(const ulonglong2* pk, int ntile, unsigned long long tag,
-                                             int* late) {
+                                             int max_polls, int* late) {
   double s[4] = {0.0, 0.0, 0.0, 0.0};
   for (int t = threadIdx.x & 31; t < ntile; t += 256) {
     double v[8];
@@ -281,7 +281,7 @@ __device__ __forceinline__ double packet_sum(const ulonglong2* pk, int ntile, un
           ok &= g == tag;
         }
       }
-    } while (!ok && ++polls < kSolvePolls);
+    } while (!ok && ++polls < max_polls);
     if (!ok) *late = 1;
 #pragma unroll
     for (int h = 0; h < 8; h += 4) {
@@ -300,7 +300,7 @@ __device__ __forceinline__ double packet_sum(const ulonglong2* pk, int ntile, un
   return y;
 }
 
-__global__ void __launch_bounds__(kThreads, 2) k_mbis_solve64(Batch bt, int T, unsigned seq) {
+__global__ void __launch_bounds__(kThreads, 2) k_mbis_solve64(Batch bt, int T, unsigned seq, int max_polls) {
   __shared__ double tab[f64::kExpTab];
   __shared__ double red[kQ * kThreads];
   __shared__ double amp[2 * kMbisMaxShell], cur[2 * kMbisMaxShell], prev[2 * kMbisMaxShell];
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_mbis_solve64(Batch bt, int T, u
       if (tile + 1 < t1) __syncthreads();  // red
     }
     for (int q = warp; q < 2 * nsh + 1; q += kWarps) {
-      const double v = packet_sum(pk + (size_t)q * nt, nt, tag, &late_s);
+      const double v = packet_sum(pk + (size_t)q * nt, nt, tag, max_polls, &late_s);
       if (lane == 0) m[q] = v;
     }
     __syncthreads();
@@ -486,16 +486,18 @@ int mbis_solve_capacity() {
   return cap;
 }
 
-void launch_mbis_solve64(const HostBatch& hb, cudaStream_t st) {
+cudaError_t launch_mbis_solve64(const HostBatch& hb, cudaStream_t st, int polls) {
   Batch bt = hb.b[K_SOLVE];
   int T = hb.solve_tiles;
   // launches are numbered (packet tags), from 1: the packets start as zeros
   static std::atomic<unsigned> launches{0};
   unsigned seq = ++launches;
   if (seq == 0) seq = ++launches;
-  void* args[] = {&bt, &T, &seq};
-  cudaLaunchCooperativeKernel((void*)k_mbis_solve64, dim3((unsigned)hb.blocks[K_SOLVE]), dim3(kThreads), args, 0, st);
-  ++g_launch_count;
+  void* args[] = {&bt, &T, &seq, &polls};
+  const cudaError_t e = cudaLaunchCooperativeKernel((void*)k_mbis_solve64, dim3((unsigned)hb.blocks[K_SOLVE]),
+                                                    dim3(kThreads), args, 0, st);
+  if (e == cudaSuccess) ++g_launch_count;
+  return e;
 }
 
 void launch_change64(const HostBatch& hb, cudaStream_t st) {

@@ -53,6 +53,7 @@ struct hp_ctx {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   size_t budget = 0, used = 0;
+  int solve_polls = kSolvePolls;
   size_t kept = 0;  // part of `used` that jobs give back on demand (hp_job::keep_mem)
   Mailbox* mail_dev = nullptr;
   Mailbox* mail_host = nullptr;
@@ -697,7 +698,11 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
         launch_mbis_local(hb, st, mixed);
       } else if (!mixed && hb.solve_tiles > 0) {  // the same in one cooperative launch
         ProfScope ps(ctx, HP_KERNEL_INNER);
-        launch_mbis_solve64(hb, st);
+        const cudaError_t e = launch_mbis_solve64(hb, st, ctx->solve_polls);
+        if (e != cudaSuccess) {
+          cudaGetLastError();
+          rc = fail(HP_ERR_CUDA, std::string("inner solve: ") + cudaGetErrorString(e));
+        }
       } else {
         rc = run_inner(ctx, jobs, hb, [&] {
           ProfScope ps(ctx, HP_KERNEL_INNER);
@@ -1267,6 +1272,14 @@ int32_t hp_ctx_memory(hp_ctx* c, size_t* used, size_t* budget) {
   if (!c) return fail(HP_ERR_INVALID, "null context");
   if (used) *used = c->used - c->kept;
   if (budget) *budget = c->budget;
+  return HP_OK;
+}
+
+// For tests: a limit of the waits of the one-launch MBIS inner solve that runs
+// out (0: the default again). Not part of the ABI.
+int32_t hp_test_solve_polls(hp_ctx* c, int32_t polls) {
+  if (!c) return fail(HP_ERR_INVALID, "null context");
+  c->solve_polls = polls > 0 ? polls : kSolvePolls;
   return HP_OK;
 }
 
