@@ -141,20 +141,26 @@ __device__ __forceinline__ f2 exp_ff(f2 x, const float2* tab) {
 }
 
 // exp(x) for x <= 88 with a table of 512 (2^(i/512) as float pairs): 60 % of
-// the instructions of exp_ff, and as accurate. x = n ln2/512 + f, |f| <=
-// 6.8e-4, so that only f + f^2/2 needs two floats: n (ln2/512)_hi as an exact
-// pair, x.hi minus its high part is exact (Sterbenz, or n = 0), and e^f - 1 =
-// (f.hi + f.hi^2/2) + f.lo (1 + f.hi) + f.hi^3 (1/6 + f.hi/24).
-// Returns 0 below the FP32 normal range, as exp_ff.
+// the instructions of exp_ff. x = n ln2/512 + f, |f| <= 6.8e-4, so that only f
+// + f^2/2 needs two floats, and e^f - 1 = (f.hi + f.hi^2/2) + f.lo (1 + f.hi)
+// + f.hi^3 (1/6 + f.hi/24). ln2/512 = C1 + C2 + C3: n C1 is a pair p, x.hi -
+// p.hi is exact (Sterbenz, or n = 0), and C2 = -2^-38 so that p.lo + n C2 is
+// exact too (multiples of 2^-38 below 2^-18; a C2 of 24 bits loses 7e-15 at
+// x = -60 there). n C3 is below 5e-9, its rounding below 2e-16.
+// Relative error: three roundings of about 2^-24 in the low part, 1.1e-14 at
+// most; the root mean square is 1.2e-15 to 1.3e-15 over -87 <= x <= -1e-2,
+// that of exp_ff 1.9e-15 to 2.1e-15. Below x of about -70 the low part leaves
+// the FP32 range (an absolute error of 2^-149). Returns 0 below the FP32
+// normal range, x < -87, as exp_ff.
 __device__ __forceinline__ f2 exp_ff512(f2 x, const float2* tab) {
   if (x.hi < -87.0f) return {0.0f, 0.0f};
-  const float kC1 = 0x1.62e43p-10f, kC2 = -0x1.05c61p-38f, kC3 = -0x1.950d88p-63f;  // ln2 / 512
+  const float kC1 = 0x1.62e43p-10f, kC2 = -0x1p-38f, kC3 = -0x1.718432p-44f;  // ln2 / 512
   const float nf = rintf(x.hi * 738.6598609f);
   const int n = (int)nf;
   const f2 p = two_prod(nf, kC1);
-  const f2 a = two_sum(x.lo, -p.lo);
+  const f2 a = two_sum(x.lo, -fmaf(nf, kC2, p.lo));
   f2 f = two_sum(x.hi - p.hi, a.hi);
-  f = fast_two_sum(f.hi, f.lo + fmaf(-nf, kC2, fmaf(-nf, kC3, a.lo)));
+  f = fast_two_sum(f.hi, f.lo + fmaf(-nf, kC3, a.lo));
   const f2 sq = two_prod(f.hi, f.hi);
   const f2 h = fast_two_sum(f.hi, 0.5f * sq.hi);
   // the rest of e^f - 1

@@ -20,6 +20,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
 namespace hp {
@@ -569,6 +570,17 @@ __host__ __device__ constexpr int square_blocks(int M) {
   const int full = (M * M + kThreads - 1) / kThreads, fine = (M * M + 63) / 64;
   const int chip = fine < 152 ? fine : 152;
   return full > chip ? full : chip;
+}
+
+// 2^(j/512), j < 512, in FP64 and as float pairs (hi, lo): JobDev::etab, etabf.
+constexpr int kExpEntries = 512;
+inline void fill_exp_tables(double* d, float2* f) {
+  for (int j = 0; j < kExpEntries; ++j) {
+    const long double v = exp2l((long double)j / kExpEntries);
+    d[j] = (double)v;
+    const float hi = (float)v;
+    f[j] = make_float2(hi, (float)(v - (long double)hi));
+  }
 }
 
 // Launch kinds: blocks per job for each kind of work.

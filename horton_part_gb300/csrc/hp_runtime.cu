@@ -1210,15 +1210,10 @@ int32_t hp_ctx_create(int32_t device, size_t hbm_budget, void* stream, hp_ctx** 
   }
   {
     struct {
-      double d[512];
-      float2 f[512];
+      double d[kExpEntries];
+      float2 f[kExpEntries];
     } tab;
-    for (int j = 0; j < 512; ++j) {
-      const long double v = exp2l((long double)j / 512.0L);
-      tab.d[j] = (double)v;
-      const float hi = (float)v;
-      tab.f[j] = make_float2(hi, (float)(v - (long double)hi));
-    }
+    fill_exp_tables(tab.d, tab.f);
     if (cudaMalloc(&c->exp_tab, sizeof(tab)) != cudaSuccess ||
         cudaMemcpy(c->exp_tab, &tab, sizeof(tab), cudaMemcpyHostToDevice) != cudaSuccess) {
       hp_ctx_destroy(c);
@@ -1503,7 +1498,7 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   }
   J.mail = ctx->mail_dev + slot;
   J.etab = ctx->exp_tab;
-  J.etabf = reinterpret_cast<const float2*>(ctx->exp_tab + 512);
+  J.etabf = reinterpret_cast<const float2*>(ctx->exp_tab + kExpEntries);
   J.natom = A; J.npoint = N; J.ntile = ntile; J.nparam = P; J.nshell = S; J.qa = qa;
   J.scheme = d->scheme; J.solver = solver; J.maxiter = maxiter;
   J.mixed = !mixed ? PH_FP64 : d->precision == HP_PRECISION_FF ? PH_FF : PH_FP32;
