@@ -111,6 +111,7 @@ struct hp_job {
   JobDev dev{};
   void* mem = nullptr;
   size_t bytes = 0;
+  size_t uncounted = 0;  // part of `bytes` that does not go against the budget
   // host-side state
   bool initialized = false;
   bool done = false;
@@ -135,7 +136,6 @@ struct hp_job {
   size_t keep_bytes = 0;
   bool keep_lost = false;
   void* sched_mem = nullptr;  // gLISA FP64: dev.hsched
-  size_t sched_bytes = 0;
   void* pack_mem = nullptr;  // fused gLISA: packed G (dev.gpack, dev.gtile_off)
   size_t pack_bytes = 0;
   std::vector<double> changes;  // outer changes of this run
@@ -613,7 +613,7 @@ int hess_layout(hp_ctx* ctx, const std::vector<hp_job*>& jobs) {
     const std::vector<int> sched = tile_schedule(work, nb);
     const size_t bytes = 4 * ((size_t)nb + 1 + nu);
     void* mem = nullptr;
-    if (!make_room(ctx, bytes) || job_alloc_retry(ctx, &mem, bytes) != cudaSuccess) {
+    if (job_alloc_retry(ctx, &mem, bytes) != cudaSuccess) {
       cudaGetLastError();
       continue;
     }
@@ -622,9 +622,8 @@ int hess_layout(hp_ctx* ctx, const std::vector<hp_job*>& jobs) {
     J.hbuf = nb;
     J.hunit = unit;
     j->sched_mem = mem;
-    j->sched_bytes = bytes;
     j->bytes += bytes;
-    ctx->used += bytes;
+    j->uncounted += bytes;
   }
   return HP_OK;
 }
@@ -1350,11 +1349,19 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   const bool fuse_job = tc && solver != HP_SOLVER_M_NEWTON && S <= kGffMaxShells && S <= kFuseMaxShells;
   if (fuse_job) nsplit = std::min(ntile, kFuseCtas);
 
-  // carve one allocation
-  struct Part { void** dst; size_t bytes; };
+  // carve one allocation; `counted` bytes of a part go against the budget: not
+  // the kernels' bookkeeping of a few bytes per (atom, tile), and partial
+  // sums as for tiles of two points a thread, so that which budgets hold a job
+  // does not depend on how its passes are cut
+  struct Part { void** dst; size_t bytes, counted; };
   std::vector<Part> parts;
   JobDev J{};
-  auto add = [&](void* dst, size_t bytes) { parts.push_back({(void**)dst, bytes}); };
+  auto add = [&](void* dst, size_t bytes) { parts.push_back({(void**)dst, bytes, bytes}); };
+  auto add_uncounted = [&](void* dst, size_t bytes) { parts.push_back({(void**)dst, bytes, 0}); };
+  const int ntile_counted = ppt_min == 1 ? std::min(ntile, (N + 2 * kThreads - 1) / (2 * kThreads)) : ntile;
+  auto add_tiles = [&](void* dst, size_t bytes) {
+    parts.push_back({(void**)dst, bytes * ntile, bytes * ntile_counted});
+  };
   add(&J.px, 8 * (size_t)N); add(&J.py, 8 * (size_t)N); add(&J.pz, 8 * (size_t)N);
   add(&J.w, 8 * (size_t)N); add(&J.rho, 8 * (size_t)N);
   if (hilo) {
@@ -1398,12 +1405,12 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   add(&J.promol, 8 * (size_t)N);
   add(&J.invpro, 8 * (size_t)N);
   add(&J.rhoa, 8 * (size_t)A * N);
-  add(&J.apart, 8 * (size_t)A * qa * ntile);
-  add(&J.jpart, 8 * (size_t)QJ_COUNT * ntile);
+  add_tiles(&J.apart, 8 * (size_t)A * qa);
+  add_tiles(&J.jpart, 8 * (size_t)QJ_COUNT);
   add(&J.atom_out, 8 * (size_t)A * AO_COUNT);
   add(&J.active, 4 * (size_t)A); add(&J.inner_it, 4 * (size_t)A);
-  add(&J.arrive, 4 * (size_t)A);
-  add(&J.ls_fail, 8 * (size_t)A * ntile);
+  add_uncounted(&J.arrive, 4 * (size_t)A);
+  add_tiles(&J.ls_fail, 8 * (size_t)A);
   // GISA / aLISA in FP64 keep the (fixed) unit-population shells on the device
   // when the matrix takes at most half of the remaining budget: every pass
   // then reads G instead of recomputing exponentials (gLISA always does).
@@ -1412,7 +1419,7 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   const size_t room = ctx->budget > firm ? ctx->budget - firm : 0;
   const bool gstore = !glisa && !mbis && !nlis && !mixed && gbytes <= room / 2;
   if (gstore) add(&J.gmat, gbytes);
-  if (gstore || (glisa && !gff)) add(&J.smask, 4 * (size_t)A * ntile);
+  if (gstore || (glisa && !gff)) add_uncounted(&J.smask, 4 * (size_t)A * ntile);
   if (glisa) {
     if (!gff) add(&J.gmat, 8 * (size_t)S * N);
     add(&J.gpart, 8 * (size_t)S * ntile);
@@ -1474,18 +1481,21 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   const bool cutoff = (mbis || (d->scheme == HP_SCHEME_LISA && solver == HP_SOLVER_SC)) &&
                       d->grid_type != 1;
   if (cutoff) {
-    add(&J.tgeo, 8 * 5 * (size_t)ntile);
-    add(&J.amax, 4 * (size_t)A * ntile);
-    add(&J.rmin, 8 * (size_t)A * ntile);
+    add_tiles(&J.tgeo, 8 * 5);
+    add_tiles(&J.amax, 4 * (size_t)A);
+    add_uncounted(&J.rmin, 8 * (size_t)A * ntile);
   }
   add(&J.hist_propars, 8 * (size_t)maxiter * P);
   add(&J.hist_charges, 8 * (size_t)maxiter * A);
   add(&J.hist_ent, 8 * (size_t)maxiter); add(&J.hist_chg, 8 * (size_t)maxiter);
   add(&J.charges, 8 * (size_t)A);
-  size_t total = 0;
-  for (auto& p : parts) total += align_up(p.bytes);
-  if (!make_room(ctx, total))
-    return fail(HP_ERR_NO_MEMORY, "job needs " + std::to_string(total) + " bytes; HBM budget exceeded");
+  size_t total = 0, counted = 0;
+  for (auto& p : parts) {
+    total += align_up(p.bytes);
+    counted += align_up(p.counted);
+  }
+  if (!make_room(ctx, counted))
+    return fail(HP_ERR_NO_MEMORY, "job needs " + std::to_string(counted) + " bytes; HBM budget exceeded");
   void* mem = nullptr;
   if (job_alloc_retry(ctx, &mem, total) != cudaSuccess) {
     cudaGetLastError();
@@ -1524,6 +1534,7 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   job->desc.solver = solver;
   job->mem = mem;
   job->bytes = total;
+  job->uncounted = total - counted;
   job->dev = J;
 
   // host staging: SoA grid, float hi/lo, atoms, shells
@@ -1716,7 +1727,7 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
   memset(&ctx->mail_host[slot], 0, sizeof(Mailbox));
   ctx->slots[slot] = job;
   ctx->slots_hi = std::max(ctx->slots_hi, slot + 1);
-  ctx->used += total;
+  ctx->used += counted;
   alloc_kept(ctx, job);
   *out = job;
   return HP_OK;
@@ -1731,7 +1742,7 @@ int32_t hp_job_destroy(hp_job* job) {
   job_free(ctx, job->pack_mem);
   job_free(ctx, job->sched_mem);
   job_free(ctx, job->keep_mem);
-  ctx->used -= job->bytes;
+  ctx->used -= job->bytes - job->uncounted;
   ctx->kept -= job->keep_bytes;
   ctx->slots[job->slot] = nullptr;
   delete job;
@@ -2157,7 +2168,7 @@ int32_t hp_density_plan_create(hp_ctx* ctx, const hp_density_desc* d, hp_density
   const size_t rcut_at = groups.size();
   groups.resize(rcut_at + rcut2.size());
   memcpy(groups.data() + rcut_at, rcut2.data(), 4 * rcut2.size());
-  const size_t bytes = 8 * ndbl + 4 * 5 * (size_t)ns + 8 * 3 + 4 * groups.size();
+  const size_t bytes = 8 * ndbl + 4 * 5 * (size_t)ns + 8 * 3;  // (without groups, the kernel's bookkeeping)
   if (!make_room(ctx, bytes)) return fail(HP_ERR_NO_MEMORY, "HBM budget exceeded");
   hp_density_plan* p = new hp_density_plan();
   p->ctx = ctx;

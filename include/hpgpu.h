@@ -182,8 +182,8 @@ typedef struct {
   int32_t status;       /* hp_status of the job (HP_OK unless it failed) */
   uint32_t warnings;    /* HP_WARN_* bits */
   int32_t converged;    /* 1 when the change fell below the threshold */
-  int64_t device_bytes; /* device memory held by the job, with what it would give
-                           back to make room (hp_ctx_memory) */
+  int64_t device_bytes; /* device memory held by the job, with what hp_ctx_memory
+                           does not count */
   double point_atom_evals; /* pro-atom evaluations done so far (sum over passes) */
   int32_t polish_iterations; /* mixed precision: FP64 outer iterations after a stall */
   int32_t f64_factors; /* gLISA with the tensor-core Hessian: Newton steps whose
@@ -223,7 +223,7 @@ int32_t hp_ctx_synchronize(hp_ctx* ctx);
 /* Bytes reserved by live jobs and density plans, and the budget. What FP64
  * MBIS and aLISA jobs keep to save recomputation (distances and pro-atoms of
  * all pairs) is not counted: it is given back when something else needs the
- * room. */
+ * room. Nor is the bookkeeping of a few bytes per (atom, tile of points). */
 int32_t hp_ctx_memory(hp_ctx* ctx, size_t* used, size_t* budget);
 
 /* Jobs */
