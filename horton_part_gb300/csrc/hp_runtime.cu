@@ -586,12 +586,14 @@ int hess_layout(hp_ctx* ctx, const std::vector<hp_job*>& jobs) {
   bool any = false;
   for (hp_job* j : jobs) any |= wanted(j);
   if (!any) return HP_OK;
-  HP_CK(cudaStreamSynchronize(ctx->stream));
   for (hp_job* j : jobs) {
     if (!wanted(j)) continue;
     JobDev& J = j->dev;
     std::vector<unsigned> mask((size_t)J.natom * J.ntile);
-    HP_CK(cudaMemcpy(mask.data(), J.smask, 4 * mask.size(), cudaMemcpyDeviceToHost));
+    // on the context stream (the legacy one takes no copy while a stream that
+    // waits for it is captured)
+    HP_CK(cudaMemcpyAsync(mask.data(), J.smask, 4 * mask.size(), cudaMemcpyDeviceToHost, ctx->stream));
+    HP_CK(cudaStreamSynchronize(ctx->stream));
     const int64_t tri = (int64_t)J.nshell * (J.nshell + 1) / 2;
     const int64_t room = (int64_t)J.nsplit * J.nshell * J.nshell / tri;  // packed partials hpart holds
     int unit = (int)((J.npoint + 16 * kH64Blocks - 1) / (16 * kH64Blocks));
@@ -1214,7 +1216,8 @@ int32_t hp_ctx_create(int32_t device, size_t hbm_budget, void* stream, hp_ctx** 
     } tab;
     fill_exp_tables(tab.d, tab.f);
     if (cudaMalloc(&c->exp_tab, sizeof(tab)) != cudaSuccess ||
-        cudaMemcpy(c->exp_tab, &tab, sizeof(tab), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaMemcpyAsync(c->exp_tab, &tab, sizeof(tab), cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
+        cudaStreamSynchronize(c->stream) != cudaSuccess) {
       hp_ctx_destroy(c);
       return fail(HP_ERR_NO_MEMORY, "context allocation failed");
     }

@@ -71,4 +71,19 @@ int dc_eval(int what, int n, const double* x, const double* y, double* out, doub
   return cudaGetLastError() != cudaSuccess;
 }
 
+// Another stream of the process in capture, one that waits for the legacy stream.
+static cudaStream_t capturing = nullptr;
+int dc_capture_begin() {
+  if (cudaStreamCreate(&capturing) != cudaSuccess) return 1;
+  return cudaStreamBeginCapture(capturing, cudaStreamCaptureModeRelaxed) != cudaSuccess;
+}
+int dc_capture_end() {
+  cudaGraph_t g = nullptr;
+  const cudaError_t e = cudaStreamEndCapture(capturing, &g);
+  if (g) cudaGraphDestroy(g);
+  cudaStreamDestroy(capturing);
+  cudaGetLastError();
+  return e != cudaSuccess;
+}
+
 }  // extern "C"
