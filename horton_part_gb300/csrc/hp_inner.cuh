@@ -106,6 +106,7 @@ static __device__ __noinline__ void mbis_update(const JobDev& J, int a) {
   inner_sums(J, a, 2 * nsh + 1, 2 * kMbisMaxShell, m);
   if (threadIdx.x >= 32) return;  // one warp
   const int it = J.inner_it[a];
+  __syncwarp();  // every lane has it before lane 0 writes the next one
   double* pc = J.cur + J.par_off[a];
   double* pp = J.prev + J.par_off[a];
   double* amp = J.keep + J.par_off[a];
