@@ -102,6 +102,9 @@ __global__ void __launch_bounds__(kThreads) k_basis64(Batch bt) {
         if (__double_as_longlong(g) != 0) mask |= 1u << k;
       }
     }
+    // without a cutoff a zero row takes part: 0 times the quotient rho / 0 of a
+    // point where every shell underflows
+    if (!(J.density_cutoff > 0.0)) mask = (1u << nsh) - 1u;
     mask = __reduce_or_sync(0xffffffffu, mask);
     if ((threadIdx.x & 31) == 0 && mask) atomicOr(&J.smask[(size_t)a * J.ntile + tile], mask);
   }
