@@ -24,6 +24,18 @@ def _job(ctx, npoint, maxiter=3):
                     threshold=1e-12, inner_threshold=1e-8, inner_maxiter=50, maxiter=maxiter)
 
 
+def _plain_job(ctx, scheme, natom, npoint, per, precision="fp64", solver="default"):
+    rng = np.random.default_rng(1)
+    coords = np.stack([np.zeros(natom), np.zeros(natom), 2.0 * np.arange(natom)], axis=1)
+    points, n = rng.uniform(-3, 3, (npoint, 3)), per * natom
+    extra = {} if scheme == "mbis" else dict(shell_orders=np.full(n, 2.0),
+                                             shell_exponents=np.tile(np.geomspace(0.1, 10, per), natom))
+    return _lib.Job(ctx, scheme, coords, np.ones(natom), points, np.full(npoint, 1.0 / npoint),
+                    np.exp(-np.linalg.norm(points, axis=1)), np.arange(natom + 1, dtype=np.int32) * per,
+                    np.tile([1.0, 2.0], n) if scheme == "mbis" else np.full(n, 1.0 / per), solver=solver,
+                    precision=precision, grid_type=3, maxiter=3, threshold=1e-8, **extra)
+
+
 @pytest.fixture(scope="module")
 def sizes(gpu_context):
     """(device bytes of the 4000-point job with its kept arrays, without them)"""
@@ -168,12 +180,11 @@ def test_density_plans_take_the_room_that_jobs_give_back(when, sizes):
     ctx = _lib.Context(0, hbm_budget=budget)
     if when == "evaluate":
         plan, _ = _water_plan(ctx, nmat)
-    held = ctx.memory()[0]
     job = _job(ctx, 4000)
     ctx.step([job])
-    jobs = [job]  # small ones until what is left is below what the plan needs with the kept arrays, and not without
-    while budget - held - sum(j.info().device_bytes for j in jobs) >= need:
-        jobs.append(_job(ctx, 2))
+    jobs = []  # jobs that keep nothing, until what is left is below what the plan needs with the kept arrays, not without
+    while budget - ctx.memory()[0] - (full - plain) >= need:
+        jobs.append(_plain_job(ctx, "lisa", 1, 64, 2, "fp64", "newton"))
     assert job.info().device_bytes == full and budget - ctx.memory()[0] >= need
     if when == "create":
         plan, _ = _water_plan(ctx, nmat)
@@ -184,18 +195,6 @@ def test_density_plans_take_the_room_that_jobs_give_back(when, sizes):
     ctx.step([job])  # and the job goes on
     plan.close()
     ctx.close()
-
-
-def _plain_job(ctx, scheme, natom, npoint, per, precision="fp64", solver="default"):
-    rng = np.random.default_rng(1)
-    coords = np.stack([np.zeros(natom), np.zeros(natom), 2.0 * np.arange(natom)], axis=1)
-    points, n = rng.uniform(-3, 3, (npoint, 3)), per * natom
-    extra = {} if scheme == "mbis" else dict(shell_orders=np.full(n, 2.0),
-                                             shell_exponents=np.tile(np.geomspace(0.1, 10, per), natom))
-    return _lib.Job(ctx, scheme, coords, np.ones(natom), points, np.full(npoint, 1.0 / npoint),
-                    np.exp(-np.linalg.norm(points, axis=1)), np.arange(natom + 1, dtype=np.int32) * per,
-                    np.tile([1.0, 2.0], n) if scheme == "mbis" else np.full(n, 1.0 / per), solver=solver,
-                    precision=precision, grid_type=3, maxiter=3, threshold=1e-8, **extra)
 
 
 # the bytes of the arrays that hold a job's inputs, parameters, pairs and partial sums (512-point tiles)
