@@ -154,7 +154,9 @@ __global__ void __launch_bounds__(kThreads) k_promol_g64(Batch bt) {
 
 // GISA moments (gisa.py:257-279): at_weights, population sum w rho_a and
 // q-vector sums sum w g_k rho_a of one (atom, tile), from the pro-atoms of
-// k_promol_g64 (rhoa is not written back: GISA reads it nowhere else).
+// k_promol_g64 (rhoa is not written back: GISA reads it nowhere else). Three
+// blocks an SM; 16 rows spill (168 bytes). 10 atoms, 145,500 points, five
+// outer iterations: 2.30 -> 1.04 ms at 6 shells, 4.66 -> 2.32 at 16.
 __global__ void __launch_bounds__(kThreads, 3) k_gisa_moments64(Batch bt) {
   __shared__ double red[(kMaxShells + 1) * kThreads];
   int a, tile;
@@ -196,6 +198,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_gisa_moments64(Batch bt) {
 
 // aLISA self-consistent iteration (alisa.py:193-291), one (atom, tile): the
 // moments sum w c_k g_k rho_a / pro and the change sum w (oldpro - pro)^2.
+// Three blocks an SM; the forms of many active rows spill (552 bytes at 16).
+// 10 atoms, 145,500 points, 40 iterations: 20.9 -> 3.7 ms at 6 shells,
+// 38.6 -> 6.1 at 16.
 __global__ void __launch_bounds__(kThreads, 3) k_lisa_sc64(Batch bt) {
   constexpr int Q = kMaxShells + 1;
   __shared__ double red[Q * kThreads];

@@ -27,8 +27,9 @@
 // phase 3 (n_sig^2 / 2 FMA per point and matrix, near the rate of a cuBLAS
 // FP64 product) and of the exponentials (hp_fp64.cuh: 11 instructions a
 // primitive; CUDA's exp and a distance per shell took 15 % of the time).
-// 604,000 points, 190 functions: 15.0 -> 12.5 ms (11.9 ms are the contraction's
-// FMAs).
+// 604,000 points, 190 functions: 15.0 -> 12.5 ms on a molecule of 6.2e9
+// significant FMAs (9.8 ms of them); 1.22 to 1.30 times the FMAs' time on
+// others (10.7 to 17.0 ms for 5.2e9 to 8.7e9).
 //
 // A low-rank factor D = L L^T (n_sig x n_occ products instead) was measured
 // at 8.4 ms and not kept: it holds only for matrices formed from orbitals
@@ -113,7 +114,7 @@ __device__ __forceinline__ void shell_out(bool pure, double rad, double x, doubl
 // r2 their squared length; zeros for a lane without a point (live false).
 // All lanes of the warp, one shell. Not inlined: one copy of the exponential
 // and of the components instead of one per call site keeps the kernel in the
-// instruction cache (13.6 -> 12.5 ms on 604,000 points; on 4,500 points, where
+// instruction cache (13.6 -> 12.5 ms on the 604,000 points above; on 4,500 points, where
 // every line is fetched once, phase 2 takes 13 instead of 26 thousand cycles).
 static __device__ __noinline__ void shell_values(const DensityArgs& a, int s, double x, double y, double z,
                                              double r2, float r2f, double* out, int T, const double* tab,

@@ -265,6 +265,11 @@ __device__ __forceinline__ void mbis_tile_ff(const JobDev& J, int a, int tile, b
   if (threadIdx.x == 0) put_partial_ff(J, a, QA_INNER + kFfMbisQ - 1, tile, out[NQ - 1]);
 }
 
+// Four blocks an SM: best at one to four shells (the chain above, alone: 31.5
+// ms, 32.8 with three blocks and 40.6 with two). From five on the registers
+// spill (1280 bytes at seven), which takes what the template gave: 10 atoms,
+// 145,500 points, 40 iterations, 4.46 -> 2.93 ms at 4 shells, 5.42 -> 4.76 at
+// 6, 5.93 -> 5.82 at 7 (with two blocks 3.10, 3.85 and 4.58).
 __global__ void __launch_bounds__(kThreads, 4) k_mbis_inner_ff(Batch bt) {
   __shared__ float2 tab[512];
   __shared__ float2 red[kWarps * kFfMbisQ];

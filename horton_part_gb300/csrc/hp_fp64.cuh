@@ -110,7 +110,8 @@ __device__ __forceinline__ double mbis_amp(double n, double s) { return n * (s *
 // without one has S = 0 / 0 there, and the same here.
 __device__ __forceinline__ void mbis_shell(double amp, double m0, double m1, double& n, double& s) {
   n = amp * m0;
-  s = amp == 0.0 ? __longlong_as_double(0x7ff8000000000000ll) : 3.0 * m0 / m1;
+  const bool none = (__double_as_longlong(amp) << 1) == 0;  // +-0, by integers
+  s = none ? __longlong_as_double(0x7ff8000000000000ll) : 3.0 * m0 / m1;
 }
 
 // Pro-atom of n MBIS shells at distance r from amplitudes and exponents.

@@ -462,13 +462,6 @@ __device__ __forceinline__ void store_partial(const JobDev& J, double* slot, dou
   *reinterpret_cast<float2*>(slot) = make_float2(hi, (float)(v - (double)hi));
 }
 
-// Fixed-order sum of n values with stride (one thread).
-__device__ __forceinline__ double serial_sum(const double* p, int n) {
-  double s = 0.0;
-  for (int i = 0; i < n; ++i) s += p[i];
-  return s;
-}
-
 constexpr double kInv8PiD = 0.039788735772973836;  // 1 / (8 pi)
 
 // FP32 coefficients of shell s for a (new, old) parameter pair, formed in

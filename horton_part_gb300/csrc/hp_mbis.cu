@@ -198,6 +198,10 @@ __device__ __forceinline__ bool mbis_skip(const JobDev& J, int a, int tile, int 
 // distance, the old pro-atom's exponentials, CUDA's exp and divide and the
 // sums of seven shells were all formed per pair. Two outer iterations of a
 // 22-atom chain of 320k points: 116.7 -> 29.6 ms (85 % of the FP64 issue).
+// Three blocks an SM: best at one and two shells; from four on the registers
+// spill (516 bytes at seven), and it is still 3.9 times as fast as the kernel
+// before (10 atoms, 145,500 points, 40 iterations: 34.3 -> 8.6 ms at 4
+// shells, 49.6 -> 12.7 at 7).
 __global__ void __launch_bounds__(kThreads, 3) k_mbis_inner64(Batch bt) {
   __shared__ double tab[f64::kExpTab];
   __shared__ double red[kQ * kThreads];

@@ -51,7 +51,9 @@ __global__ void k_na_init(const double* __restrict__ propars, int nshell, double
   }
 }
 
-// Same arithmetic as the job kernel k_mbis_inner64, pair by pair without stored values (one atom).
+// The iteration of the job kernel k_mbis_inner64 for one atom in plain FP64
+// arithmetic (CUDA's exp and divide, the amplitude in each shell's value):
+// equal to it up to rounding.
 __global__ void __launch_bounds__(kNaThreads)
     k_na_mbis_inner(const double* __restrict__ rho, const double* __restrict__ w,
                     const double* __restrict__ r, int npoint, int nshell, double density_cutoff,

@@ -1560,7 +1560,6 @@ int32_t hp_job_create(hp_ctx* ctx, const hp_job_desc* d, hp_job** out) {
       plane(J.gmat32, 4 * (size_t)S * N);
       plane(J.gmat_lo, 4 * (size_t)S * N);
     }
-
     std::sort(skip.begin(), skip.end());
     char* at = (char*)mem;
     for (const auto& r : skip) {
