@@ -693,24 +693,34 @@ int step_iterstock(hp_ctx* ctx, const std::vector<hp_job*>& jobs, const HostBatc
   }
   int rc = HP_OK;
   switch (j0->desc.scheme) {
-    case HP_SCHEME_MBIS:
+    case HP_SCHEME_MBIS: {
       if (local) {  // atom grids: every inner iteration of every atom in one launch
         ProfScope ps(ctx, HP_KERNEL_INNER);
         launch_mbis_local(hb, st, mixed);
-      } else if (!mixed && hb.solve_tiles > 0) {  // the same in one cooperative launch
+        break;
+      }
+      bool whole = !mixed && hb.solve_tiles > 0;  // the same in one cooperative launch
+      if (whole) {
         ProfScope ps(ctx, HP_KERNEL_INNER);
         const cudaError_t e = launch_mbis_solve64(hb, st, ctx->solve_polls);
-        if (e != cudaSuccess) {
+        if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+          // fewer blocks fit than the device's attributes say (a shared GPU
+          // with a part of the SMs): a launch per iteration, the same bits
           cudaGetLastError();
-          rc = fail(HP_ERR_CUDA, std::string("inner solve: ") + cudaGetErrorString(e));
+          whole = false;
+        } else if (e != cudaSuccess) {
+          cudaGetLastError();
+          return fail(HP_ERR_CUDA, std::string("inner solve: ") + cudaGetErrorString(e));
         }
-      } else {
+      }
+      if (!whole) {
         rc = run_inner(ctx, jobs, hb, [&] {
           ProfScope ps(ctx, HP_KERNEL_INNER);
           launch_mbis_inner(hb, st, mixed);
         }, j0->dev.inner_maxiter + 1);
       }
       break;
+    }
     case HP_SCHEME_NLIS:  // NLIS / GMBIS (FP64)
       if (local) {
         ProfScope ps(ctx, HP_KERNEL_INNER);

@@ -7,6 +7,7 @@
 typedef struct { unsigned x, y, z; } fake_dim3;
 
 int fail_cudaMalloc = 0, fail_cudaLaunchCooperativeKernel = 0; /* how many of the next calls fail */
+int code_cudaLaunchCooperativeKernel = 0;                      /* with this error */
 
 static void* real(const char* name) {
   static void* lib;
@@ -25,7 +26,7 @@ int cudaMalloc(void** p, size_t n) {
 int cudaLaunchCooperativeKernel(const void* f, fake_dim3 grid, fake_dim3 block, void** args, size_t smem, void* st) {
   if (fail_cudaLaunchCooperativeKernel > 0) {
     --fail_cudaLaunchCooperativeKernel;
-    return 720; /* cudaErrorCooperativeLaunchTooLarge */
+    return code_cudaLaunchCooperativeKernel;
   }
   return ((int (*)(const void*, fake_dim3, fake_dim3, void**, size_t, void*))real("cudaLaunchCooperativeKernel"))(
       f, grid, block, args, smem, st);

@@ -18,8 +18,10 @@ SETUP = """
     from horton_part_gb300 import _lib, synthetic
     from horton_part_gb300.density import DensityPlan
     from test_gpu_memory import _job
-    def fail(call, n):
+    def fail(call, n, code=None):
         ctypes.c_int.in_dll(ctypes.CDLL(None), "fail_" + call).value = n
+        if code is not None:
+            ctypes.c_int.in_dll(ctypes.CDLL(None), "code_" + call).value = code
     ctx = _lib.Context(0)
 """
 
@@ -41,7 +43,7 @@ def test_inner_solve_that_is_not_launched(tmp_path, gpu_context):
         job = _job(ctx, 4000, maxiter=2)
         ctx.step([job])
         before = job.results()
-        fail("cudaLaunchCooperativeKernel", 1)
+        fail("cudaLaunchCooperativeKernel", 1, 701)  # cudaErrorLaunchOutOfResources
         try:
             ctx.step([job])
         except _lib.HPError as e:
@@ -88,4 +90,23 @@ def test_density_plan_whose_first_allocation_fails(tmp_path, gpu_context):
         np.testing.assert_array_equal(plan.evaluate(points), want)
         plan.close()
         ctx.step([job])
+    """)
+
+
+@pytest.mark.parametrize("code", [720, 801])  # cudaErrorCooperativeLaunchTooLarge, cudaErrorNotSupported
+def test_inner_solve_that_does_not_fit(code, tmp_path, gpu_context):
+    """A launch per iteration instead, with the same bits."""
+    _run(tmp_path, f"""
+        results, launches = [], []
+        for k in (0, 1):
+            job = _job(ctx, 4000, maxiter=1)
+            fail("cudaLaunchCooperativeKernel", k, {code})
+            ctx.profile()
+            ctx.step([job])
+            launches.append(ctx.profile_get("inner")[1])
+            results.append((job.results(at_weights=True), job.info().inner_iterations))
+        assert launches[0] == 1 and launches[1] > 2, launches
+        assert results[0][1] == results[1][1]
+        for key in results[0][0]:
+            np.testing.assert_array_equal(results[0][0][key], results[1][0][key])
     """)
